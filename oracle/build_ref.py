@@ -57,14 +57,14 @@ def _copy(src, dst):
 
 
 def have_sources():
-    return os.path.isfile(os.path.join(SRC, "simfru_local.c")) or os.path.isdir(REF_DIR)
+    return any(os.path.isfile(os.path.join(d, "simfru_local.c")) for d in (SRC, REF_DIR))
 
 
 def sync_sources():
     """Copy the reference sources (unmodified) into oracle/_ref/src once."""
     if os.path.isfile(os.path.join(SRC, "simfru_local.c")):
         return SRC
-    if not os.path.isdir(REF_DIR):
+    if not have_sources():
         raise FileNotFoundError("reference sources not found (neither %s nor %s)" % (SRC, REF_DIR))
     os.makedirs(SRC, exist_ok=True)
     for fn in os.listdir(REF_DIR):
