@@ -145,6 +145,7 @@ def bind(path):
         "gw_probe_fp64_issue": ([_dp], C.c_int),
         "gw_probe_fcn_warp": ([P(C.c_double)], C.c_int),
         "gw_probe_fcn_compare": ([_dp, C.c_int, C.c_double, C.c_int, _dp, _dp, _dp, _dp], C.c_int),
+        "gw_probe_fp64_math": ([C.c_ulonglong, C.c_longlong, P(C.c_ulonglong)], C.c_int),
         "gw_probe_div": ([C.c_ulonglong, C.c_longlong, P(C.c_ulonglong)], C.c_int),
     }
     for name, (args, res) in sig.items():
@@ -385,6 +386,16 @@ def div_mismatches(n, seed=1, lib=None):
     m = C.c_ulonglong(0)
     _check(L.gw_probe_div(int(seed), int(n), C.byref(m)), "gw_probe_div", L)
     return m.value
+
+
+def fp64_math_mismatches(n, seed=1, lib=None):
+    """(quotients, reciprocals, quotients by constants) of the FRU kernels'
+    FP64 arithmetic whose bits differ from the hardware division's, of n each
+    (gw_probe_fp64_math)."""
+    L = lib if lib is not None else load()
+    m = (C.c_ulonglong * 3)()
+    _check(L.gw_probe_fp64_math(int(seed), int(n), m), "gw_probe_fp64_math", L)
+    return tuple(m)
 
 
 def fcn_warp_us(lib=None):

@@ -19,7 +19,7 @@ EXE = os.path.join(OUT, "gw_caf")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_COMMON = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
-                      "-I" + CSRC, "-I" + INC]
+                      "-I" + CSRC, "-I" + INC, "-I" + OUT]
 CUDA_UNITS = {
     # source: extra flags
     "gw_fru_stage.cu": ["-fmad=false"],
@@ -35,6 +35,23 @@ CUDA_UNITS = {
     "gw_persist.cu": ["-fmad=false"],
 }
 C_UNITS = ["gw_dp.c", "gw_dropin.c"]
+
+
+def write_exp2_table(path):
+    """2^(j/4096) as a rounded double and the remainder, for gw_fp64_math.cuh."""
+    import decimal
+    with decimal.localcontext() as c:
+        c.prec = 60
+        ln2 = decimal.Decimal(2).ln()
+        rows = []
+        for j in range(4096):
+            v = (ln2 * j / 4096).exp()
+            hi = float(v)
+            rows.append("{%s, %s}," % (hi.hex(), float(v - decimal.Decimal(hi)).hex()))
+    text = "\n".join(rows) + "\n"
+    if not os.path.isfile(path) or open(path).read() != text:
+        with open(path, "w") as f:
+            f.write(text)
 
 
 def _nvcc():
@@ -60,6 +77,7 @@ def build(force=False, verbose=False):
     if not force and up_to_date():
         return LIB
     os.makedirs(OUT, exist_ok=True)
+    write_exp2_table(os.path.join(OUT, "gw_exp2_table.h"))
     nvcc = _nvcc()
     jobs = []
     objs = []

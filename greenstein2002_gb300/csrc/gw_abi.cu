@@ -583,6 +583,12 @@ extern "C" int gw_probe_div(unsigned long long seed, long long n, unsigned long 
   return GW_OK;
 }
 
+extern "C" int gw_probe_fp64_math(unsigned long long seed, long long n, unsigned long long* mismatches) {
+  if (!mismatches || n <= 0) return set_err(GW_EINVAL, "gw_probe_fp64_math: bad argument");
+  CK(gw::probe_fp64_math(seed, n, mismatches));
+  return GW_OK;
+}
+
 extern "C" int gw_probe_fcn_warp(double* us) {
   if (!us) return set_err(GW_EINVAL, "gw_probe_fcn_warp: null argument");
   CK(gw::probe_fcn_warp(us));

@@ -23,9 +23,9 @@ int gw_probe_fcn_warp(double *us);
  * Fs/Fw[n][37] and currents Cs/Cw[n][24] of both. */
 int gw_probe_fcn_compare(const double *states, int n, double time, int clamp, double *Fs, double *Fw, double *Cs,
                          double *Cw);
-/* exp() of n arguments as the device evaluates it and with the host libm:
- * exp is the FRU path's only transcendental, and the two may round
- * differently in the last place. */
+/* exp of n arguments as the FRU path evaluates it on the device (fexp of
+ * gw_fp64_math.cuh) and with the host libm: exp is the path's only
+ * transcendental, and the two may round differently in the last place. */
 int gw_probe_exp(const double *x, double *device_y, double *host_y, int n);
 /* FP64 issue cost on one SM, cycles per operation of warp 0 (clock64 over
  * chains of 4096 operations), in this order:
@@ -38,11 +38,16 @@ int gw_probe_exp(const double *x, double *device_y, double *host_y, int n);
  *   [15]     dependent FFMA (FP32), 1 warp */
 #define GW_PROBE_ISSUE_N 16
 int gw_probe_fp64_issue(double cycles[GW_PROBE_ISSUE_N]);
-/* The FRU kernels' FP64 division on the integer pipe (gw_intdiv.h) against
+/* The FP64 division on the integer pipe (gw_intdiv.h) against
  * the hardware division, on n operand pairs the device draws from `seed`
  * (half arbitrary bit patterns, half normal operands of magnitude
  * 1e-8 .. 1e4); *mismatches counts quotients whose bits differ. */
 int gw_probe_div(unsigned long long seed, long long n, unsigned long long *mismatches);
+/* The FRU kernels' quotients, reciprocals and quotients by constants
+ * (gw_fp64_math.cuh) against the hardware division, n of each on operands
+ * of magnitude 1e-8 .. 1e4 the device draws from `seed`; mismatches[0..2]
+ * count results whose bits differ. */
+int gw_probe_fp64_math(unsigned long long seed, long long n, unsigned long long mismatches[3]);
 /* The persistent kernel's wait limit, exercised without a fault: one cell
  * (its current FRU state, globals at rest) runs its first operation, after
  * which a flag that nothing sets keeps its next operation from being posted;

@@ -7,19 +7,21 @@
 // lasts as long as the FP64 instruction chain of its slowest FRU.  Spreading an
 // FRU over its clefts divides that chain by about four at the same total work.
 //
-// R = double: the plain FP64 method.  Every operation is the reference's, and
-// the arithmetic is arranged to issue few FP64 instructions while staying
-// bit-identical to it:
-//   - divisions by constants use Markstein's correction (q = x*r;
-//     q += fma(-q, d, x)*r), which returns the correctly rounded quotient;
-//   - max/min of non-negative doubles compare their bit patterns as integers;
-//   - channel exit totals come from per-state coefficient tables instead of
-//     divergent switches;
-//   - uniforms are compared with thresholds in the integer domain
-//     (u = y/2^32 > P  <=>  y > floor(P*2^32));
-//   - the four voltage exponentials of a substep are computed one per lane,
-//     and exp(2VF/RT) at the end of a substep is reused at the start of the
-//     next.
+// R = double: the plain FP64 method.  Every operation is the reference's,
+// rounded as the reference rounds it, arranged to issue few FP64
+// instructions (what bounds the kernels, see gw_fp64_math.cuh):
+//   - quotients, reciprocals and exponentials from gw_fp64_math.cuh;
+//   - max/min/compares of non-negative doubles on their bit patterns;
+//   - the products of an LCC's exit row are kept and reused when it leaves;
+//     the RyR rates are formed per state present in the cleft, not per RyR;
+//   - a draw is first compared in FP32 with an upper bound of dt*rate; only
+//     channels that may leave form 1 - dt*rate, which is compared with the
+//     draw in the integer domain (u = y/2^32 > P  <=>  y > floor(P*2^32));
+//   - products with 0/1 flags are selections, halvings are folded into FMAs
+//     (both exact), the three interpolated voltages/concentrations and the
+//     four voltage exponentials are computed one per lane, and
+//     exp(2VF/RT) at the end of a substep is reused at the start of the
+//     next (and at the stage start computed once per lane, not per FRU).
 // R = float: the mixed-precision method.  Transition rates, the local Ca ODE
 // and the FRU clock are evaluated in FP32, the Ca states and the clock
 // accumulated as compensated FP32 pairs; FP64 is kept for the FRU arrays in
@@ -38,6 +40,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gw_fp64_math.cuh"
 #include "gw_fru_core.cuh"
 #include "gw_fru_model.cuh"
 #include "gw_kernels.h"
@@ -63,33 +66,17 @@ __device__ __forceinline__ bool abs_lt(double v, double c) {
 }
 __device__ __forceinline__ bool abs_lt(float v, float c) { return (__float_as_int(v) & 0x7fffffff) < __float_as_int(c); }
 
-// x / d for a compile-time constant d with r = 1/d: correctly rounded in FP64
-__device__ __forceinline__ double divc(double x, double d, double r) {
-  const double q = x * r;
-  return fma(fma(-q, d, x), r, q);
-}
+// FP32 (the mixed-precision method): division by a constant as a product,
+// rdiv the fast approximate quotient, qdiv the correctly rounded one.
 __device__ __forceinline__ float divc(float x, float d, float r) { return x * r; }
-// Divisions by variable divisors.  FP64: the hardware's correctly rounded
-// quotient.  (The integer-pipe division of gw_intdiv.h gives the same bits
-// with ~6 fewer FP64-pipe slots, but its longer dependent chain made the
-// latency-bound stage kernels 25-30% slower on GB300, so it is not used
-// here.)  FP32: rdiv is the fast approximate quotient, qdiv the correctly
-// rounded one.
-__device__ __forceinline__ double rdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ float rdiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double qdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ float qdiv(float a, float b) { return a / b; }
-__device__ __forceinline__ double rexp(double x) { return exp(x); }
 __device__ __forceinline__ float rexp(float x) { return expf(x); }
-// e = exp(x) and the GHK denominator e - 1.  FP64: the reference's e - 1.
-// FP32: expm1f, because expf(x) - 1 keeps almost no relative precision for
-// the |x| < 1e-5 of membrane potentials within a few tenths of a mV of zero,
-// and is exactly 0 for potentials of a few uV (just above the 1e-6 mV of the
-// reference's V = 0 branch), which made the GHK factor infinite.
-__device__ __forceinline__ void exp_em1(double x, double& e, double& em1) {
-  e = exp(x);
-  em1 = e - 1.0;
-}
+// e = exp(x) and the GHK denominator e - 1 by expm1f, because expf(x) - 1
+// keeps almost no relative precision for the |x| < 1e-5 of membrane
+// potentials within a few tenths of a mV of zero, and is exactly 0 for
+// potentials of a few uV (just above the 1e-6 mV of the reference's V = 0
+// branch), which made the GHK factor infinite.
 __device__ __forceinline__ void exp_em1(float x, float& e, float& em1) {
   em1 = expm1f(x);
   e = 1.0f + em1;
@@ -109,19 +96,16 @@ __device__ __forceinline__ void thresh(double P, uint64_t& fl, bool& exact) {
     exact = (M & ((1ull << sh) - 1ull)) == 0ull;
   }
 }
-// leaves its state when u > 1 - dt*R (LCC, RyR) ...
 __device__ __forceinline__ bool nonpos(double P) { return __double_as_longlong(P) <= 0LL; }  // P <= 0 (not NaN)
-__device__ __forceinline__ bool leave_gt(uint32_t y, double dt, double R) {
-  const double P = 1.0 - dt * R;
+// y/2^32 > P (LCC, RyR) and y/2^32 >= P (VDI gate, Cl channel)
+__device__ __forceinline__ bool u_above(uint32_t y, double P) {
   if (nonpos(P)) return true;  // never on valid input (dt*rate <= 0.1)
   uint64_t fl;
   bool ex;
   thresh(P, fl, ex);
   return (uint64_t)y > fl;
 }
-// ... or when u >= 1 - dt*R (VDI gate, Cl channel)
-__device__ __forceinline__ bool leave_ge(uint32_t y, double dt, double R) {
-  const double P = 1.0 - dt * R;
+__device__ __forceinline__ bool u_reaches(uint32_t y, double P) {
   if (nonpos(P)) return true;
   uint64_t fl;
   bool ex;
@@ -140,13 +124,9 @@ __device__ __forceinline__ bool leave_ge(uint32_t y, float dt, float R) {
   return comp_u32(y) <= dt * R * 4294967296.0f;
 }
 
-// Destination of a channel that leaves its state (simfru_local.c:215-253):
-// FP64 walks the reference's cumulative probabilities with u = y/2^32; FP32
-// walks the remaining exit mass against 1 - u = (2^32 - y)/2^32, which keeps
-// full resolution near u = 1 where the walk happens.
-__device__ __forceinline__ int choose_dest(const double r[4], const int d[4], int len, double dt, uint32_t y) {
-  return pick_dest(r, d, len, dt, (double)y / 4294967296.0);
-}
+// Destination of a channel that leaves its state (simfru_local.c:215-253) in
+// FP32: walks the remaining exit mass against 1 - u = (2^32 - y)/2^32, which
+// keeps full resolution near u = 1 where the walk happens.
 __device__ __forceinline__ int choose_dest(const float r[4], const int d[4], int len, float dt, uint32_t y) {
   const float c = comp_u32(y) * 2.3283064365386963e-10f;
   float rem = dt * r[0] - dt * r[1];
@@ -171,20 +151,20 @@ __device__ __forceinline__ bool u_below(uint32_t y, float p) { return (float)y *
 
 // LCC exit total = (cX*bX + cY*bY) + cZ*bZ with bases {1, alpha, beta,
 // gamma, alpha', beta'}: the sums of fru_rates_local.c:176-340 in their order.
-__constant__ double c_lcc_coef[13][3] = {
-    {0.0, 0.0, 0.0},
-    {4.0, 1.0, 0.0},                     // 1: 4a + g
-    {1.0, 3.0, aL},                      // 2: b + 3a + aL g
-    {2.0, 2.0, aL * aL},                 // 3
-    {3.0, 1.0, aL * aL * aL},            // 4
-    {4.0, fL, aL * aL * aL * aL},        // 5
-    {gL, 0.0, 0.0},                      // 6
-    {4.0, CCa0_to_C0, 0.0},              // 7: 4a' + omega
-    {1.0, 3.0, CCa1_to_C1},              // 8: b' + 3a' + omega/bL
-    {2.0, 2.0, CCa2_to_C2},              // 9
-    {3.0, 1.0, CCa3_to_C3},              // 10
-    {4.0, CCa4_to_C4, fLprime},          // 11
-    {gLprime, 0.0, 0.0},                 // 12
+__constant__ float c_lcc_coef[13][3] = {
+    {0.0f, 0.0f, 0.0f},
+    {4.0f, 1.0f, 0.0f},                     // 1: 4a + g
+    {1.0f, 3.0f, (float)(aL)},                      // 2: b + 3a + aL g
+    {2.0f, 2.0f, (float)(aL * aL)},                 // 3
+    {3.0f, 1.0f, (float)(aL * aL * aL)},            // 4
+    {4.0f, (float)(fL), (float)(aL * aL * aL * aL)},        // 5
+    {(float)(gL), 0.0f, 0.0f},                      // 6
+    {4.0f, (float)(CCa0_to_C0), 0.0f},              // 7: 4a' + omega
+    {1.0f, 3.0f, (float)(CCa1_to_C1)},              // 8: b' + 3a' + omega/bL
+    {2.0f, 2.0f, (float)(CCa2_to_C2)},              // 9
+    {3.0f, 1.0f, (float)(CCa3_to_C3)},              // 10
+    {4.0f, (float)(CCa4_to_C4), (float)(fLprime)},          // 11
+    {(float)(gLprime), 0.0f, 0.0f},                 // 12
 };
 // basis index of each term, packed 3 x 4 bits per state:
 // 0 = 1, 1 = alpha, 2 = beta, 3 = gamma, 4 = alpha', 5 = beta'
@@ -396,17 +376,6 @@ __device__ __forceinline__ void ghk_terms(R V, R pca_scale, R& e2, R& a2j, bool&
   else a2j = rdiv(R(PCa * 4.0) * pca_scale * VFsqRT, em1) * R(JDHconstant);
 }
 
-// (t - t0) / interval with r = 1/interval rounded once per stage: Markstein's
-// correction of q = x*r returns the correctly rounded quotient
-__device__ __forceinline__ double frac_of(double t, double t0, double interval, double r) {
-  const double x = t - t0;
-  const double q = x * r;
-  return fma(fma(-q, interval, x), r, q);
-}
-__device__ __forceinline__ float frac_of(double t, double t0, double, float rinterval) {
-  return (float)(t - t0) * rinterval;
-}
-
 // The constants of one lane for a stage (the same for every FRU of it).
 template <typename R>
 struct LaneStage {
@@ -441,6 +410,55 @@ __device__ __forceinline__ void lane_stage(const StageParams& p, const Group& g,
   L.cCF = L.isdiv ? R(0.0) : (g.c == 0 ? R(alphacf) : R(betacf));
   L.cK = L.isdiv ? (g.c == 2 ? R(0.4) : R(340.0)) : R(1.0);
   L.cM = L.isdiv ? (g.c == 2 ? R(1.0 - 0.4) : R(60.0)) : R(0.0);
+}
+
+// FP64: exp(2VF/RT) and the GHK factor a2 of fcn_fru.c:78-101 for voltage V
+// (any V and scale: beyond +-500 mV or a scale near the ends of the exponent
+// range the hardware's division).
+__device__ __forceinline__ void ghk_terms(double V, double pca4, double& e2, double& a2j, bool& small) {
+  constexpr double JDHconstant = 1.0 / (2.0 * VSS * Faraday * 1000.0);
+  const double VFRT = const_div(V, kDivRTF);
+  const double VFsqRT = (1000.0 * Faraday) * VFRT;
+  e2 = fexp(2.0 * VFRT);
+  small = abs_lt(V, 1.e-6);
+  a2j = 0.0;
+  if (!small) {
+    const double num = pca4 * VFsqRT, em1 = e2 - 1.0;
+    a2j = (abs_lt(V, 500.0) && fits(pca4) ? fast_div(num, em1) : num / em1) * JDHconstant;
+  }
+}
+
+template <>
+struct LaneStage<double> {
+  double dep0[3], myspan, mydep0;  // V, Cai, CaNSR at t0; the one this lane interpolates (cleft % 3)
+  double pca4, pca2;               // LCC permeability factors of the GHK and the V = 0 form
+  double t0, tf, interval, rhi, rlo;  // rhi + rlo = 1/interval to about 105 bits
+  double e2, a2j;                  // ghk_terms at t0
+  bool small, isdiv, tpos;         // tpos: times are >= 0 (and tf is not NaN)
+  double cA, cCF, cK, cM;          // per-lane voltage exponential (see LaneStage<R>)
+  ConstDiv cR;                     // as a factor (rhi; lanes 0, 1) or a divisor (lanes 2, 3)
+};
+__device__ __forceinline__ void lane_stage(const StageParams& p, const Group& g, LaneStage<double>& L) {
+#pragma unroll
+  for (int i = 0; i < 3; i++) L.dep0[i] = p.dep0[i];
+  L.mydep0 = g.c == 1 ? p.dep0[1] : g.c == 2 ? p.dep0[2] : p.dep0[0];
+  L.myspan = g.c == 1 ? p.span[1] : g.c == 2 ? p.span[2] : p.span[0];
+  L.pca4 = (PCa * 4.0) * p.pca_scale;
+  L.pca2 = (-PCa * 2.0 * 1000.0 * Faraday) * p.pca_scale;
+  L.t0 = p.t0;
+  L.tf = p.tf;
+  L.tpos = ord(p.t0) >= 0 && p.tf >= 0.0;
+  L.interval = p.tf - p.t0;
+  L.rhi = 1.0 / L.interval;
+  L.rlo = fma(-L.interval, L.rhi, 1.0) * L.rhi;
+  ghk_terms(L.dep0[0], L.pca4, L.e2, L.a2j, L.small);
+  L.isdiv = g.c >= 2;
+  L.cA = L.isdiv ? (g.c == 2 ? 12.5 : 30.0) : -35.0;
+  L.cR.rhi = L.isdiv ? (g.c == 2 ? kDiv5.rhi : kDiv12.rhi) : (g.c == 0 ? 0.012 : -0.05);
+  L.cR.rlo = L.isdiv ? (g.c == 2 ? kDiv5.rlo : kDiv12.rlo) : 0.0;
+  L.cCF = g.c == 0 ? alphacf : betacf;
+  L.cK = g.c == 2 ? 0.4 : 340.0;
+  L.cM = g.c == 2 ? 1.0 - 0.4 : 60.0;
 }
 
 // Accumulator of an FRU Ca concentration over the substeps.  FP64: a double,
@@ -487,14 +505,20 @@ template <>
 struct FruClock<double> {
   double t;
   __device__ __forceinline__ void begin(const LaneStage<double>& L) { t = L.t0; }
-  __device__ __forceinline__ bool running(const LaneStage<double>& L) const { return t < L.tf; }
+  // t < tf; for times >= 0 on their bit patterns
+  __device__ __forceinline__ bool running(const LaneStage<double>& L) const {
+    return L.tpos ? ilt(t, L.tf) : t < L.tf;
+  }
   __device__ __forceinline__ double advance(double dtr, const LaneStage<double>& L) {
     const double dt64 = imin(dtr, L.tf - t);
     t = t + dt64;
     return dt64;
   }
+  // (t - t0) / interval, by the two-instruction division with the stage's own
+  // reciprocal: the quotient is known to 2^-105 before its last rounding
   __device__ __forceinline__ double frac(const LaneStage<double>& L) const {
-    return frac_of(t, L.t0, L.interval, L.rinterval);
+    const double x = t - L.t0;
+    return fma(x, L.rhi, x * L.rlo);
   }
 };
 template <>
@@ -593,9 +617,9 @@ __device__ __forceinline__ void substep_a(Fru4<R>& F, Sub4<R>& S, const LaneStag
   {
     const int s = lcc_of(w);
     const uint16_t bi = c_lcc_basis[s];
-    const R X = R(c_lcc_coef[s][0]) * pick_basis(bi & 15, alpha, beta, gam, ap, bp);
-    const R Y = R(c_lcc_coef[s][1]) * pick_basis((bi >> 4) & 15, alpha, beta, gam, ap, bp);
-    const R Z = R(c_lcc_coef[s][2]) * pick_basis((bi >> 8) & 15, alpha, beta, gam, ap, bp);
+    const R X = c_lcc_coef[s][0] * pick_basis(bi & 15, alpha, beta, gam, ap, bp);
+    const R Y = c_lcc_coef[s][1] * pick_basis((bi >> 4) & 15, alpha, beta, gam, ap, bp);
+    const R Z = c_lcc_coef[s][2] * pick_basis((bi >> 8) & 15, alpha, beta, gam, ap, bp);
     R0[0] = X + Y + Z;
   }
   {
@@ -786,6 +810,407 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
   F.nsub++;
 }
 
+// ---- the FP64 substep -----------------------------------------------------------
+template <>
+struct Fru4<double> {
+  FruClock<double> clk;
+  CaAcc<double> jsr, ss;
+  uint32_t w, nsub;
+  int mti;
+  bool lopen, small;
+  double jcoef;  // JRyRmax x open RyRs of the cleft
+  double dep[3], e2, a2j;
+};
+template <>
+struct Sub4<double> {
+  double cajsr, cass, X, Y, Z, Rl, Rv, k12, sat;  // LCC exit products and total, VDI rate, RyR k12 and saturation
+  int regime, ne, pre, etot;
+  uint32_t exmask;  // RyRs that draw an extra uniform (bit 0 of their nibbles)
+  uint32_t exw[kRyR], bw[8];
+};
+template <typename R>
+__device__ __forceinline__ void sub_begin(Sub4<R>& S) {
+  S.etot = 0;
+#pragma unroll
+  for (int i = 0; i < kRyR; i++) S.exw[i] = 0u;
+  S.p34 = R(0);
+}
+__device__ __forceinline__ void sub_begin(Sub4<double>& S) {
+  S.etot = 0;
+#pragma unroll
+  for (int i = 0; i < kRyR; i++) S.exw[i] = 0u;
+}
+
+// The five RyR states of a channel word as masks over their nibbles (bit 0 of
+// nibble i set when RyR i is in the state).
+struct RyrMasks {
+  uint32_t s1, s2, s3, s4, s5, s6, s7, s8;
+};
+__device__ __forceinline__ RyrMasks ryr_masks(uint32_t w) {
+  const uint32_t r = w >> 8;
+  const uint32_t b0 = r & 0x11111u, b1 = (r >> 1) & 0x11111u, b2 = (r >> 2) & 0x11111u;
+  RyrMasks m;
+  m.s1 = b0 & ~b1 & ~b2;
+  m.s2 = ~b0 & b1 & ~b2;
+  m.s3 = b0 & b1 & ~b2;
+  m.s4 = ~b0 & ~b1 & b2;
+  m.s5 = b0 & ~b1 & b2;
+  m.s6 = ~b0 & b1 & b2;
+  m.s7 = b0 & b1 & b2;
+  m.s8 = (r >> 3) & 0x11111u;
+  return m;
+}
+__device__ __forceinline__ double jryr_open(uint32_t w) {
+  const RyrMasks m = ryr_masks(w);
+  const int n = __popc(m.s3 | m.s4 | m.s7);
+  double v = 0.0;
+  v = (n == 1) ? JRyRmax * 1.0 : v;
+  v = (n == 2) ? JRyRmax * 2.0 : v;
+  v = (n == 3) ? JRyRmax * 3.0 : v;
+  v = (n == 4) ? JRyRmax * 4.0 : v;
+  v = (n == 5) ? JRyRmax * 5.0 : v;
+  return v;
+}
+
+__device__ __forceinline__ void fru_begin(Fru4<double>& F, const LaneStage<double>& L) {
+#pragma unroll
+  for (int i = 0; i < 3; i++) F.dep[i] = L.dep0[i];
+  F.lopen = lcc_open(F.w);
+  F.jcoef = jryr_open(F.w);
+  F.clk.begin(L);
+  F.e2 = L.e2;
+  F.a2j = L.a2j;
+  F.small = L.small;
+}
+
+// LCC exit row of each state for the FP64 path: coefficients of the products
+// X, Y, Z with bases (4 bits each from bit 0: 0 = 1, 1 = alpha, 2 = beta,
+// 3 = gamma, 5 = beta'; alpha' = 2 alpha is in the coefficient, exactly), the
+// total X + Y + Z in the reference's order (fru_rates_local.c:176-340), and
+// from bit 12 the row's length and its destinations d1, d2, d3; bit 28 / 29:
+// the row is (Y, X) / (X, Z, Y) instead of (X, Y, Z).
+struct LccRow64 {
+  double x, y, z;
+  uint32_t code, pad;
+};
+constexpr uint32_t lcc_code(uint32_t basis, uint32_t len, uint32_t d1, uint32_t d2, uint32_t d3, uint32_t perm) {
+  return basis | (len << 12) | (d1 << 16) | (d2 << 20) | (d3 << 24) | (perm << 28);
+}
+static __device__ const LccRow64 g_lcc_row64[13] = {
+    {0.0, 0.0, 0.0, lcc_code(0x000, 1, 0, 0, 0, 0), 0},
+    {4.0, 1.0, 0.0, lcc_code(0x031, 3, 2, 7, 0, 0), 0},                           // 1: 4a, g
+    {1.0, 3.0, aL, lcc_code(0x312, 4, 1, 3, 8, 0), 0},                            // 2: b, 3a, aL g
+    {2.0, 2.0, aL * aL, lcc_code(0x312, 4, 2, 4, 9, 0), 0},                       // 3
+    {3.0, 1.0, aL * aL * aL, lcc_code(0x312, 4, 3, 5, 10, 0), 0},                 // 4
+    {4.0, fL, aL * aL * aL * aL, lcc_code(0x302, 4, 4, 6, 11, 0), 0},             // 5
+    {gL, 0.0, 0.0, lcc_code(0x000, 2, 5, 0, 0, 0), 0},                            // 6
+    {4.0 * aL, CCa0_to_C0, 0.0, lcc_code(0x001, 3, 1, 8, 0, 1), 0},               // 7: 4a', omega
+    {1.0, 3.0 * aL, CCa1_to_C1, lcc_code(0x015, 4, 7, 2, 9, 2), 0},               // 8: b', 3a', omega/bL
+    {2.0, 2.0 * aL, CCa2_to_C2, lcc_code(0x015, 4, 8, 3, 10, 2), 0},              // 9
+    {3.0, aL, CCa3_to_C3, lcc_code(0x015, 4, 9, 4, 11, 2), 0},                    // 10
+    {4.0, CCa4_to_C4, fLprime, lcc_code(0x005, 4, 10, 5, 12, 0), 0},              // 11
+    {gLprime, 0.0, 0.0, lcc_code(0x000, 2, 11, 0, 0, 0), 0},                      // 12
+};
+
+// Destination of a channel that leaves its state (simfru_local.c:215-253):
+// the cumulative walk from P = 1 - dt*total over the row r1, r2, (r3), the
+// draw compared with each sum in the integer domain.  d holds d1, d2, d3 in
+// its nibbles, len = 1 + destinations.
+__device__ __forceinline__ uint32_t walk(uint32_t y, double P, double dt, double r1, double r2, int len, uint32_t d) {
+  if (len > 2) {
+    const double acc1 = P + dt * r1;
+    if (u_above(y, acc1)) {
+      d >>= 4;
+      if (len > 3 && u_above(y, acc1 + dt * r2)) d >>= 4;
+    }
+  }
+  return d & 15u;
+}
+
+// a value's leading 20 mantissa bits as FP32, for the upper bounds below
+__device__ __forceinline__ float head32(double x) {
+  return __uint_as_float((uint32_t)__double2hiint(x) * 8u + 0x40000000u);
+}
+
+// First half of one FP64 substep (simfru_local.c:83-146 up to the draws):
+// the layout of the extra draws and the words that precede word 624 first
+// (their loads overlap the rest), then the voltage terms and exit totals.
+__device__ __forceinline__ void substep_a(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const Group& g,
+                                          const StageCtx& sc) {
+  const uint32_t w = F.w;
+  const double cass = F.ss.v;
+  S.cajsr = F.jsr.v;
+  S.cass = cass;
+  {
+    const double cc = imin(cass, threshMAXCa);
+    S.regime = ilt(cc, threshCa56to8) ? 0 : (ilt(cc, threshCa34to7) ? 1 : 2);
+  }
+  {
+    // extra draws: regime 0 resolves 7 and 8, regime 1 resolves 7 (in cleft,
+    // then RyR order); the four counts travel as the bytes of one word
+    const RyrMasks m = ryr_masks(w);
+    S.exmask = (S.regime == 0) ? (m.s7 | m.s8) : (S.regime == 1) ? m.s7 : 0u;
+    S.ne = __popc(S.exmask);
+    uint32_t n = (uint32_t)S.ne << (8 * g.c);
+    n |= __shfl_xor_sync(g.mask, n, 1);
+    n |= __shfl_xor_sync(g.mask, n, 2);
+    S.etot = (int)((n * 0x01010101u) >> 24);
+    S.pre = (int)(((n & ((1u << (8 * g.c)) - 1u)) * 0x01010101u) >> 24);
+  }
+  fetch_old(sc, g, F.mti, S.pre, S.ne, S.etot, S.exw, S.bw);
+  // ---- voltage terms at the substep start, one exponential per lane ----
+  const double V = F.dep[0];
+  const double x = V + L.cA;
+  const double ev = fexp(L.isdiv ? const_div(x, L.cR) : x * L.cR.rhi);
+  double vterm;
+  if (L.isdiv) {
+    const double den = 1.0 + ev;
+    vterm = (abs_lt(V, 500.0) ? fast_div(L.cK, den) : L.cK / den) + L.cM;
+  } else {
+    vterm = L.cCF * ev;
+  }
+  const double alpha = from(g, vterm, 0), beta = from(g, vterm, 1);
+  const double yinf = from(g, vterm, 2), tau = from(g, vterm, 3);
+  const double bp = const_div(beta, kDivBL);  // / (bL * kappa)
+  const double gam = gammacf * cass;
+  {
+    const LccRow64* row = &g_lcc_row64[lcc_of(w)];
+    const double2 xy = __ldg(reinterpret_cast<const double2*>(row));
+    const double z = __ldg(&row->z);
+    const uint32_t code = __ldg(&row->code);
+    const int bx = code & 15u, by = (code >> 4) & 15u, bz = (code >> 8) & 15u;
+    double v = (bx == 1) ? alpha : 1.0;
+    v = (bx == 2) ? beta : v;
+    v = (bx == 5) ? bp : v;
+    S.X = xy.x * v;
+    v = (by == 1) ? alpha : 1.0;
+    v = (by == 3) ? gam : v;
+    S.Y = xy.y * v;
+    v = (bz == 3) ? gam : 1.0;
+    S.Z = z * v;
+    S.Rl = S.X + S.Y + S.Z;
+  }
+  {
+    const double num = (vdi_of(w) == 2) ? (1.0 - yinf) : yinf;
+    S.Rv = abs_lt(V, 500.0) ? fast_div(num, tau) : num / tau;
+  }
+  const double c2 = cass * cass;
+  S.sat = imin(threshMAX, const_div(c2, kDivKrate));
+  S.k12 = k12cf * imin(threshMAX, const_div(c2, kDivKrate2));
+}
+
+// Buffer factors of the local ODE: 1/(1 + a1 + a2) of the subspace and
+// 1/(1 + a1) of the JSR (fcn_fru.c:103-131).  Concentrations of [0, 16) mM
+// keep every divisor in the fast forms' range.
+__device__ __forceinline__ bool conc_ok(double c) { return (uint32_t)__double2hiint(c) < 0x40300000u; }
+__device__ __forceinline__ void buffer_factors(double cajsr, double cass, double& bSS, double& bJSR) {
+  const double xr = cass + KBSR, xl = cass + KBSL, xj = cajsr + KmCSQN;
+  const double dr = xr * xr, dl = xl * xl, dj = xj * xj;
+  if (conc_ok(cass) && conc_ok(cajsr)) {
+    const double a1 = fast_div(BSRtot * KBSR, dr), a2 = fast_div(BSLtot * KBSL, dl);
+    const double aj = fast_div(CSQNtot * KmCSQN, dj);
+    bSS = fast_rcp(1.0 + a1 + a2);
+    bJSR = fast_rcp(1.0 + aj);
+  } else {
+    const double a1 = BSRtot * KBSR / dr, a2 = BSLtot * KBSL / dl;
+    const double aj = CSQNtot * KmCSQN / dj;
+    bSS = 1.0 / (1.0 + a1 + a2);
+    bJSR = 1.0 / (1.0 + aj);
+  }
+}
+
+// Local Ca ODE of one cleft (fcn_fru.c:23-137), FP64; see fcn_fru4 above.
+__device__ __forceinline__ void fcn_fru4(const Group& g, double cajsr, double cass, const double dep[3], double e2,
+                                         double a2j, bool small, bool lopen, double jcoef, double pca2, double& dJSR,
+                                         double& dSS) {
+  constexpr double JDHconstant = 1.0 / (2.0 * VSS * Faraday * 1000.0);
+  const double Cai = dep[1], CaNSR = dep[2];
+  double bSS, bJSR;
+  buffer_factors(cajsr, cass, bSS, bJSR);
+  const double JRyR = jcoef * (cajsr - cass);
+  const double j0 = from(g, JRyR, 0), j1 = from(g, JRyR, 1), j2 = from(g, JRyR, 2), j3 = from(g, JRyR, 3);
+  const double JRyRtot = j0 + j1 + j2 + j3;
+  const double cnext = from(g, cass, (g.c + 1) & 3);
+  const double Jss = const_div(cass - cnext, kDivTauss2ss);
+  const double Jss_prev = from(g, Jss, (g.c + 3) & 3);
+  const double Jxfer = const_div(cass - Cai, kDivTauxfer);
+  double JDH = -(cass * e2 - Cao * 0.341) * a2j;
+  if (small) JDH = pca2 * (cass - Cao * 0.341) * JDHconstant;
+  JDH = lopen ? JDH : 0.0;
+  dSS = bSS * (JDH + JRyR - Jxfer - Jss + Jss_prev);
+  const double Jtr = const_div(CaNSR - cajsr, kDivTautr);
+  dJSR = bJSR * (Jtr - (VSS / VJSR) * JRyRtot);
+}
+
+// Second half: the remaining words, the RyR pseudo-states, the substep size,
+// the Heun step of the local Ca ODE and the transitions (:135-277).
+__device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const Group& g,
+                                          StageCtx& sc) {
+  uint32_t w = F.w;
+  const double cajsr = S.cajsr, cass = S.cass, sat = S.sat;
+  const int regime = S.regime;
+  uint32_t* bw = S.bw;
+  fetch_new(sc, g, F.mti, S.pre, S.ne, S.etot, S.exw, bw);
+  const double k34 = k34cf * sat, k56 = k56cf * sat;
+  RyrMasks m = ryr_masks(w);
+  // k34/(k34+k43): for the draws of regimes 0/1 or for the merged state 7 of
+  // regime 2 (never both)
+  double p34 = 0.0;
+  if (m.s7 | (regime == 2 ? m.s3 | m.s4 : 0u)) p34 = fast_div(k34, k34 + k43);
+  if (S.ne) {
+    uint32_t ex = S.exmask;
+    while (ex) {
+      const int b = __ffs(ex) - 1;  // the RyR's nibble
+      ex &= ex - 1u;
+      const uint32_t y = S.exw[0];  // in RyR order, from a shifting window
+      S.exw[0] = S.exw[1];
+      S.exw[1] = S.exw[2];
+      S.exw[2] = S.exw[3];
+      S.exw[3] = S.exw[4];
+      uint32_t s;
+      if (((w >> (8 + b)) & 15u) == 7u) s = u_below(y, p34) ? 4u : 3u;
+      else s = u_below(y, fast_div(k56, k56 + k65)) ? 6u : 5u;
+      w = set_field(w, 8 + b, (int)s);
+    }
+    m = ryr_masks(w);
+  }
+  // merged states: 3, 4 -> 7 in regime 2; 5, 6 -> 8 in regimes 1 and 2
+  if (regime == 2) {
+    const uint32_t c = (m.s3 | m.s4) << 8;
+    w = (w & ~(c * 15u)) | (c * 7u);
+  }
+  if (regime != 0) {
+    const uint32_t c = (m.s5 | m.s6) << 8;
+    w = (w & ~(c * 15u)) | (c << 3);
+  }
+  m = ryr_masks(w);
+  // ---- exit totals of the RyR states present, and their maximum ----
+  double mx = imax(S.Rl, S.Rv);
+  const double Rc = (cl_of(w) == 1) ? kfIto2 * cass : kbIto2;
+  mx = imax(mx, Rc);
+  double k23 = 0.0, k25 = 0.0, k54 = 0.0, T2 = 0.0, T5 = 0.0, t7a = 0.0, t7b = 0.0, T7 = 0.0, t8a = 0.0, t8b = 0.0,
+         T8 = 0.0;
+  mx = m.s1 ? imax(mx, S.k12) : mx;
+  if (m.s2) {
+    k23 = k23cf * sat;
+    k25 = k25cf * sat;
+    T2 = k21 + k23 + k25;
+    mx = imax(mx, T2);
+  }
+  const double T3 = k32 + k34;
+  mx = m.s3 ? imax(mx, T3) : mx;
+  mx = m.s4 ? imax(mx, k43 + k45) : mx;
+  if (m.s5 | m.s8) k54 = k54cf * sat;
+  if (m.s5) {
+    T5 = k52 + k54 + k56;
+    mx = imax(mx, T5);
+  }
+  mx = m.s6 ? imax(mx, k65) : mx;
+  if (m.s7) {
+    t7a = (1.0 - p34) * k32;  // p34 = k34 / (k43 + k34)
+    t7b = p34 * k45;
+    T7 = t7a + t7b;
+    mx = imax(mx, T7);
+  }
+  if (m.s8) {
+    const double a1 = fast_div(k65, k56 + k65);
+    t8a = a1 * k52;
+    t8b = a1 * k54;
+    T8 = t8a + t8b;
+    mx = imax(mx, T8);
+  }
+  mx = gmax(g, mx);
+  // ---- substep size (simfru_local.c:135-146) ----
+  double dtr = imin(fits(mx) ? fast_div(0.1, mx) : 0.1 / mx, 10.001e-3);
+  if (__any_sync(g.mask, ilt(1.5e-3, cass))) dtr = imin(dtr, 5.001e-3);
+  const double dt = F.clk.advance(dtr, L);
+  // ---- Heun step (simfru_local.c:149-173) ----
+  const bool in_range = conc_ok(cass) && abs_lt(F.dep[0], 500.0);
+  double dJ, dS;
+  fcn_fru4(g, cajsr, cass, F.dep, F.e2, F.a2j, F.small, F.lopen, F.jcoef, L.pca2, dJ, dS);
+  const double k1J = dt * dJ, k1S = dt * dS;
+  const double y1J = cajsr + k1J, y1S = cass + k1S;
+  {
+    const double mine = L.mydep0 + F.clk.frac(L) * L.myspan;
+    F.dep[0] = from(g, mine, 0);
+    F.dep[1] = from(g, mine, 1);
+    F.dep[2] = from(g, mine, 2);
+  }
+  ghk_terms(F.dep[0], L.pca4, F.e2, F.a2j, F.small);
+  fcn_fru4(g, y1J, y1S, F.dep, F.e2, F.a2j, F.small, F.lopen, F.jcoef, L.pca2, dJ, dS);
+  F.jsr.v = fma(k1J + dt * dJ, 0.5, cajsr);
+  F.ss.v = fma(k1S + dt * dS, 0.5, cass);
+  // ---- transitions of this cleft's 8 channels (:215-276) ----
+  // A channel leaves when c = 2^32 - y is below about dt*R*2^32.  First an
+  // upper bound of that in FP32 (dt and R by their heads, raised by 2^-16,
+  // and 2^-22 for the dropped bits of c); the few channels within it form
+  // 1 - dt*R.  The RyRs that may leave take one pass each: the lanes of a
+  // warp share the pass.  Each RyR's row depends only on its own state and
+  // its cleft's constants, so the order of the passes does not matter.
+  const float dth = __fmul_rn(head32(dt), 1.0f + 0x1p-16f);
+  auto near_leaving = [&](uint32_t y, float R) {
+    return __uint_as_float((~y >> 9) | 0x3f800000u) <= __fmaf_rn(R, dth, 1.0f + 0x1p-22f);
+  };
+  uint32_t cand = 0u;
+  {
+    const float f1 = head32(S.k12), f2 = head32(T2), f3 = head32(T3), f4 = head32(k43 + k45), f5 = head32(T5),
+                f6 = head32(k65), f7 = head32(T7), f8 = head32(T8);
+#pragma unroll
+    for (int i = 0; i < kRyR; i++) {
+      const bool b0 = (w >> (8 + 4 * i)) & 1u, b1 = (w >> (9 + 4 * i)) & 1u, b2 = (w >> (10 + 4 * i)) & 1u;
+      const float lo = b1 ? (b0 ? f3 : f2) : (b0 ? f1 : f8), hi = b1 ? (b0 ? f7 : f6) : (b0 ? f5 : f4);
+      cand |= near_leaving(bw[2 + i], b2 ? hi : lo) ? (1u << i) : 0u;
+    }
+  }
+  bool lcc = near_leaving(bw[0], head32(S.Rl));
+  bool vdi = near_leaving(bw[1], head32(S.Rv)), cl = near_leaving(bw[7], head32(Rc));
+  if (!in_range) {
+    cand = 31u;
+    lcc = vdi = cl = true;
+  }
+  const uint32_t w0 = w;
+  if (lcc) {
+    const double P = 1.0 - dt * S.Rl;
+    if (u_above(bw[0], P)) {
+      const uint32_t code = __ldg(&g_lcc_row64[lcc_of(w)].code);
+      const uint32_t perm = code >> 28;
+      const double r1 = (perm == 1) ? S.Y : S.X, r2 = (perm == 2) ? S.Z : (perm == 1) ? S.X : S.Y;
+      w = set_field(w, 0, (int)walk(bw[0], P, dt, r1, r2, (int)((code >> 12) & 15u), code >> 16));
+    }
+  }
+  if (vdi && u_reaches(bw[1], 1.0 - dt * S.Rv)) w = set_field(w, 4, 3 - vdi_of(w));
+  while (cand) {
+    const int i = __ffs(cand) - 1;
+    cand &= cand - 1u;
+    uint32_t y = bw[2];  // the RyR's uniform, by selection (no dynamic register indexing)
+    y = (i == 1) ? bw[3] : y;
+    y = (i == 2) ? bw[4] : y;
+    y = (i == 3) ? bw[5] : y;
+    y = (i == 4) ? bw[6] : y;
+    const int s = ryr_of(w, i);
+    // exit total, first two rates, row length and destinations of the state
+    // (fru_rates_local.c:374-736)
+    const uint32_t to5 = (regime == 0) ? 5u : 8u, to7 = (regime == 2) ? 7u : 3u;
+    double T = S.k12, r1 = 0.0, r2 = 0.0;
+    int len = 2;
+    uint32_t d = 2u;  // 1 -> 2
+    if (s == 2) { T = T2; r1 = k21; r2 = k23; len = 4; d = 1u | (to7 << 4) | (to5 << 8); }
+    if (s == 3) { T = T3; r1 = k32; len = 3; d = 0x42u; }
+    if (s == 4) { T = k43 + k45; r1 = k43; len = 3; d = 3u | (to5 << 4); }
+    if (s == 5) { T = T5; r1 = k52; r2 = k54; len = 4; d = 0x642u; }
+    if (s == 6) { T = k65; d = 5u; }
+    if (s == 7) { T = T7; r1 = t7a; len = 3; d = 0x82u; }
+    if (s == 8) { T = T8; r1 = t8a; len = 3; d = (regime == 2) ? 0x72u : 0x42u; }
+    const double P = 1.0 - dt * T;
+    if (u_above(y, P)) w = set_field(w, 8 + 4 * i, (int)walk(y, P, dt, r1, r2, len, d));
+  }
+  if (cl && u_reaches(bw[7], 1.0 - dt * Rc)) w = set_field(w, 28, 3 - cl_of(w));
+  F.lopen = lcc_open(w);
+  if (w != w0) F.jcoef = jryr_open(w);
+  F.w = w;
+  F.nsub++;
+}
+
 // Regenerate, with the whole warp, the MT rows whose draws in this substep
 // run past word 624 (`go`: this lane's FRU takes a substep now).
 template <typename R>
@@ -824,10 +1249,7 @@ __device__ __forceinline__ void advance4(StageCtx& sc, const Group& g, bool live
     }
     if (!__any_sync(0xffffffffu, go)) break;
     Sub4<R> S;
-    S.etot = 0;
-#pragma unroll
-    for (int i = 0; i < kRyR; i++) S.exw[i] = 0u;
-    S.p34 = R(0);
+    sub_begin(S);
     if (go) substep_a(F, S, L, g, sc);
     regen_step(sc, lane, g, go, F, S);
     if (go) substep_b(F, S, L, g, sc);
@@ -1182,10 +1604,7 @@ __device__ __forceinline__ void stage_body_packed(const DevState& s, const Stage
     }
     if (!__any_sync(0xffffffffu, has)) break;
     Sub4<R> S;
-    S.etot = 0;
-#pragma unroll
-    for (int i = 0; i < kRyR; i++) S.exw[i] = 0u;
-    S.p34 = R(0);
+    sub_begin(S);
     if (go) substep_a(F, S, LS, g, sc);
     regen_step(sc, lane, g, go, F, S);
     if (go) substep_b(F, S, LS, g, sc);

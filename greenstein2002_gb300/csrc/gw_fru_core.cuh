@@ -134,8 +134,8 @@ __device__ __forceinline__ void advance_fru(const StageParams& p, double y[5], u
     // ---- exit rates at the substep start (fru_rates_local.c:126-777) ----
     const LccBasis lb = lcc_basis(dep[0]);
     const double nu = 1.0;
-    const double yinf = nu * (0.4 / (1.0 + exp((dep[0] + 12.5) / 5.0)) + (1.0 - 0.4));
-    const double tau = 60.0 + 340.0 / (1.0 + exp((dep[0] + 30.0) / 12.0));
+    const double yinf = nu * (0.4 / (1.0 + fexp((dep[0] + 12.5) / 5.0)) + (1.0 - 0.4));
+    const double tau = 60.0 + 340.0 / (1.0 + fexp((dep[0] + 30.0) / 12.0));
     const double vdi_open_rate = (1.0 - yinf) / tau, vdi_closed_rate = yinf / tau;
     double cass0[kClefts];
 #pragma unroll

@@ -10,6 +10,8 @@
 #pragma once
 #include <stdint.h>
 
+#include "gw_fp64_math.cuh"
+
 namespace gw {
 
 constexpr int kClefts = 4;          // parameters.h:30
@@ -148,8 +150,8 @@ using LccBasis = LccBasisT<double>;
 
 __device__ __forceinline__ LccBasis lcc_basis(double V) {
   LccBasis b;
-  b.alpha = alphacf * exp(0.012 * (V - 35.0));
-  b.beta = betacf * exp(-0.05 * (V - 35.0));
+  b.alpha = alphacf * fexp(0.012 * (V - 35.0));
+  b.beta = betacf * fexp(-0.05 * (V - 35.0));
   b.bp = b.beta / (bL * kappa);
   return b;
 }
@@ -275,7 +277,7 @@ __device__ __forceinline__ void fcn_fru(const double y[5], const double dep[3], 
   for (int c = 0; c < kClefts; c++) Jss[c] = (y[c + 1] - y[(c + 1) % kClefts + 1]) / tauss2ss;
   const double VFRT = V / RT_over_F;
   const double VFsqRT = (1000.0 * Faraday) * VFRT;
-  const double e2 = exp(2.0 * VFRT);
+  const double e2 = fexp(2.0 * VFRT);
   const bool small = fabs(V) < 1.e-6;
   const double a2j = small ? 0.0 : PCa * 4.0 * VFsqRT / (e2 - 1.0) * JDHconstant;
   {

@@ -123,6 +123,8 @@ cudaError_t probe_exp(const double* x, double* device_y, double* host_y, int n);
 cudaError_t probe_fp64_issue(double* cycles);
 // gw_div_rn against the hardware division on n device-drawn operand pairs.
 cudaError_t probe_div(unsigned long long seed, long long n, unsigned long long* mismatches);
+// fast_div, fast_rcp, const_div against the hardware division (mismatches[3]).
+cudaError_t probe_fp64_math(unsigned long long seed, long long n, unsigned long long* mismatches);
 // fcn on one thread against fcn on a warp, for n states; and the warp's cost
 cudaError_t probe_fcn_compare(const double* states, int n, double time, int clamp, double* Fs, double* Fw,
                               double* Cs, double* Cw);

@@ -314,10 +314,7 @@ __device__ __forceinline__ void run_batch(const Args& a, int ci, int grp0, int n
       }
       if (!__any_sync(kFull, has)) break;
       Sub4<R> S;
-      S.etot = 0;
-#pragma unroll
-      for (int i = 0; i < kRyR; i++) S.exw[i] = 0u;
-      S.p34 = R(0);
+      sub_begin(S);
       if (go) substep_a(F, S, LS, g, sc);
       regen_step(sc, lane, g, go, F, S);
       if (go) substep_b(F, S, LS, g, sc);

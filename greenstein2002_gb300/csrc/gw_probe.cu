@@ -7,6 +7,7 @@
 
 #include "gw_cell_model.h"
 #include "gw_dp_device.cuh"
+#include "gw_fp64_math.cuh"
 #include "gw_intdiv.h"
 #include "gw_kernels.h"
 
@@ -112,14 +113,14 @@ cudaError_t probe_fcn(double* device_us, double* host_us) {
   return e;
 }
 
-// exp() as the FRU kernels evaluate it (CUDA's double exp), element-wise,
+// exp as the FRU substep evaluates it (fexp), element-wise,
 // next to the host libm's: the FRU path's only transcendental (rates
 // fru_rates_local.c:131-132, :346-348; GHK fcn_fru.c:80; currents
 // mpi_master.c:406), so the only arithmetic the device cannot share with
 // the reference's host build bit for bit.
 __global__ void exp_map(const double* x, double* y, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = exp(x[i]);
+  if (i < n) y[i] = fexp(x[i]);
 }
 
 cudaError_t probe_exp(const double* x, double* device_y, double* host_y, int n) {
@@ -289,6 +290,46 @@ cudaError_t probe_div(unsigned long long seed, long long n, unsigned long long* 
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpy(mismatches, d, sizeof *d, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e;
+}
+
+// The FRU substep's quotients, reciprocals and quotients by its constants
+// (gw_fp64_math.cuh) against the hardware division: operands of magnitude
+// 1e-8 .. 1e4 drawn as above; bad[0..2] count results whose bits differ.
+__global__ void fp64_math_probe_kernel(uint64_t seed, long long per_thread, unsigned long long* bad) {
+  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  uint64_t st = seed ^ (tid * 0xd1342543de82ef95ull);
+  const ConstDiv k[9] = {kDiv5, kDiv12, kDivBL, kDivKrate, kDivKrate2, kDivTauss2ss, kDivTauxfer, kDivTautr, kDivRTF};
+  const double d[9] = {5.0, 12.0, 1.9356 * 1.0, 0.00127215, 3.4188, 10.0 * 0.005, 0.005, 3.0, 8.314 * 310.0 / 96.5};
+  unsigned nq = 0, nr = 0, nc = 0;
+  for (long long i = 0; i < per_thread; i++) {
+    uint64_t a = div_probe_next(st), b = div_probe_next(st);
+    const uint64_t ea = 1023 - 27 + div_probe_next(st) % 41, eb = 1023 - 27 + div_probe_next(st) % 41;
+    a = (a & 0x800fffffffffffffull) | (ea << 52);
+    b = (b & 0x800fffffffffffffull) | (eb << 52);
+    const double x = __longlong_as_double((long long)a), y = __longlong_as_double((long long)b);
+    nq += __double_as_longlong(x / y) != __double_as_longlong(fast_div(x, y));
+    nr += __double_as_longlong(1.0 / y) != __double_as_longlong(fast_rcp(y));
+    const int c = (int)(i % 9);
+    nc += __double_as_longlong(x / d[c]) != __double_as_longlong(const_div(x, k[c]));
+  }
+  if (nq) atomicAdd(bad, (unsigned long long)nq);
+  if (nr) atomicAdd(bad + 1, (unsigned long long)nr);
+  if (nc) atomicAdd(bad + 2, (unsigned long long)nc);
+}
+
+cudaError_t probe_fp64_math(unsigned long long seed, long long n, unsigned long long* mismatches) {
+  const int threads = 256, blocks = 152 * 8;
+  const long long per = (n + (long long)threads * blocks - 1) / ((long long)threads * blocks);
+  unsigned long long* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, 3 * sizeof *d);
+  if (e == cudaSuccess) e = cudaMemset(d, 0, 3 * sizeof *d);
+  if (e == cudaSuccess) {
+    fp64_math_probe_kernel<<<blocks, threads>>>(seed, per, d);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(mismatches, d, 3 * sizeof *d, cudaMemcpyDeviceToHost);
   cudaFree(d);
   return e;
 }
