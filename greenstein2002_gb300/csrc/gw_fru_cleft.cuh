@@ -237,6 +237,52 @@ __device__ __forceinline__ void copy_row16(uint32_t* dst, const uint32_t* src, c
   __syncwarp(g.mask);
 }
 
+// The five RyR states of a channel word as masks over their nibbles (bit 0 of
+// nibble i set when RyR i is in the state).
+struct RyrMasks {
+  uint32_t s1, s2, s3, s4, s5, s6, s7, s8;
+};
+__device__ __forceinline__ RyrMasks ryr_masks(uint32_t w) {
+  const uint32_t r = w >> 8;
+  const uint32_t b0 = r & 0x11111u, b1 = (r >> 1) & 0x11111u, b2 = (r >> 2) & 0x11111u;
+  RyrMasks m;
+  m.s1 = b0 & ~b1 & ~b2;
+  m.s2 = ~b0 & b1 & ~b2;
+  m.s3 = b0 & b1 & ~b2;
+  m.s4 = ~b0 & ~b1 & b2;
+  m.s5 = b0 & ~b1 & b2;
+  m.s6 = ~b0 & b1 & b2;
+  m.s7 = b0 & b1 & b2;
+  m.s8 = (r >> 3) & 0x11111u;
+  return m;
+}
+// The extra draws of a substep: regime 0 resolves RyR states 7 and 8,
+// regime 1 resolves 7 (in cleft, then RyR order).  exmask: this lane's RyRs
+// that draw (bit 0 of their nibbles), ne their number, pre the draws of the
+// clefts before, etot the FRU's; the four counts travel as the bytes of one
+// word.
+__device__ __forceinline__ void draw_layout(const Group& g, uint32_t w, int regime, uint32_t& exmask, int& ne, int& pre,
+                                            int& etot) {
+  const RyrMasks m = ryr_masks(w);
+  exmask = (regime == 0) ? (m.s7 | m.s8) : (regime == 1) ? m.s7 : 0u;
+  ne = __popc(exmask);
+  uint32_t n = (uint32_t)ne << (8 * g.c);
+  n |= __shfl_xor_sync(g.mask, n, 1);
+  n |= __shfl_xor_sync(g.mask, n, 2);
+  etot = (int)((n * 0x01010101u) >> 24);
+  pre = (int)(((n & ((1u << (8 * g.c)) - 1u)) * 0x01010101u) >> 24);
+}
+// merged RyR states: 3, 4 -> 7 in regime 2; 5, 6 -> 8 in regimes 1 and 2
+__device__ __forceinline__ uint32_t merge_ryr(uint32_t w, int regime) {
+  const RyrMasks m = ryr_masks(w);
+  const uint32_t c7 = (regime == 2) ? (m.s3 | m.s4) << 8 : 0u, c8 = (regime != 0) ? (m.s5 | m.s6) << 8 : 0u;
+  return (w & ~((c7 | c8) * 15u)) | (c7 * 7u) | (c8 << 3);
+}
+__device__ __forceinline__ int ryr_open_masked(uint32_t w) {
+  const RyrMasks m = ryr_masks(w);
+  return __popc(m.s3 | m.s4 | m.s7);
+}
+
 // The launch's view of one warp's 8 FRUs: each lane's FRU row (in place,
 // global memory) and the copy-on-twist rows of the cell.
 struct StageCtx {
@@ -264,15 +310,21 @@ __device__ __forceinline__ void use_row(StageCtx& sc, uint32_t* row, const uint3
 // from the new generation, tempers, and advances mti.
 __device__ __forceinline__ void fetch_old(const StageCtx& sc, const Group& g, int mti, int pre, int ne, int etot,
                                           uint32_t ex[kRyR], uint32_t bw[8]) {
+  if (ne) {
 #pragma unroll
-  for (int i = 0; i < kRyR; i++) {
-    const int pos = mti + pre + i;
-    if (i < ne && pos < kMtN) ex[i] = sc.m[pos];
+    for (int i = 0; i < kRyR; i++) {
+      const int pos = mti + pre + i;
+      if (i < ne && pos < kMtN) ex[i] = sc.m[pos];
+    }
   }
+  const uint32_t* m = sc.m + (mti + etot + 8 * g.c);
+  if (mti + etot + 32 <= kMtN) {
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const int pos = mti + etot + 8 * g.c + k;
-    if (pos < kMtN) bw[k] = sc.m[pos];
+    for (int k = 0; k < 8; k++) bw[k] = m[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (mti + etot + 8 * g.c + k < kMtN) bw[k] = m[k];
   }
 }
 
@@ -313,8 +365,10 @@ __device__ __forceinline__ void fetch_new(const StageCtx& sc, const Group& g, in
   } else {
     mti = mti + W;
   }
+  if (ne) {
 #pragma unroll
-  for (int i = 0; i < kRyR; i++) ex[i] = mt_temper(ex[i]);
+    for (int i = 0; i < kRyR; i++) ex[i] = mt_temper(ex[i]);
+  }
 #pragma unroll
   for (int k = 0; k < 8; k++) bw[k] = mt_temper(bw[k]);
 }
@@ -579,12 +633,13 @@ template <typename R>
 struct Sub4 {
   R cajsr, cass, alpha, beta, bp, gam, k12, k23, k34, k54, k25, k56, p34, R0[8];
   int regime, ne, pre, etot;
+  uint32_t exmask;  // RyRs that draw an extra uniform (bit 0 of their nibbles)
   uint32_t exw[kRyR], bw[8];
 };
 
 // First half of one substep of the FRU (simfru_local.c:83-146 up to the
-// draws): voltage terms, exit totals, the RyR constants, the layout of the
-// extra draws and the words that precede word 624.
+// draws): the layout of the extra draws and the words that precede word 624,
+// then voltage terms, exit totals and the RyR constants.
 template <typename R>
 __device__ __forceinline__ void substep_a(Fru4<R>& F, Sub4<R>& S, const LaneStage<R>& L, const Group& g,
                                           const StageCtx& sc) {
@@ -599,6 +654,14 @@ __device__ __forceinline__ void substep_a(Fru4<R>& F, Sub4<R>& S, const LaneStag
   const R cA = L.cA, cR = L.cR, cD = L.cD, cCF = L.cCF, cK = L.cK, cM = L.cM;
   cajsr = F.jsr.r();
   cass = F.ss.r();
+  // the layout of the extra draws and the words that precede word 624 first:
+  // their loads overlap the rest
+  {
+    const R cc = imin(cass, R(threshMAXCa));
+    regime = ilt(cc, R(threshCa56to8)) ? 0 : (ilt(cc, R(threshCa34to7)) ? 1 : 2);
+  }
+  draw_layout(g, w, regime, S.exmask, ne, pre, etot);
+  fetch_old(sc, g, mti, pre, ne, etot, S.exw, S.bw);
   // ---- voltage terms at the substep start, one exponential per lane ----
   const R x = dep[0] + cA;
   R q = x * cR;
@@ -636,21 +699,6 @@ __device__ __forceinline__ void substep_a(Fru4<R>& F, Sub4<R>& S, const LaneStag
   k54 = R(k54cf) * sat;
   k25 = R(k25cf) * sat;
   k56 = R(k56cf) * sat;
-  {
-    const R cc = imin(cass, R(threshMAXCa));
-    regime = ilt(cc, R(threshCa56to8)) ? 0 : (ilt(cc, R(threshCa34to7)) ? 1 : 2);
-  }
-  // extra draws: regime 0 resolves 7 and 8, regime 1 resolves 7 (in cleft, then RyR order)
-  ne = 0;
-  #pragma unroll
-  for (int i = 0; i < kRyR; i++) {
-    const int s = ryr_of(w, i);
-    ne += (regime == 0 && (s == 7 || s == 8)) || (regime == 1 && s == 7);
-  }
-  const int n0 = from(g, ne, 0), n1 = from(g, ne, 1), n2 = from(g, ne, 2), n3 = from(g, ne, 3);
-  pre = (g.c > 0 ? n0 : 0) + (g.c > 1 ? n1 : 0) + (g.c > 2 ? n2 : 0);
-  etot = n0 + n1 + n2 + n3;
-  fetch_old(sc, g, mti, pre, ne, etot, S.exw, S.bw);
 }
 
 // Second half: the remaining words, the RyR pseudo-states, the substep size,
@@ -674,55 +722,29 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
   const R pca_scale = L.pca_scale;
   fetch_new(sc, g, mti, pre, ne, etot, exw, bw);
   {
-    // the draws are taken in order from a shifting window (static
-    // register indices); k34/(k34+k43) is formed once, for the draws of
-    // regimes 0/1 or for the merged state 7 of regime 2 (never both)
-    bool has7 = false, has34 = false;
-  #pragma unroll
-    for (int i = 0; i < kRyR; i++) {
-      const int s = ryr_of(w, i);
-      has7 |= (s == 7);
-      has34 |= (s == 3 || s == 4);
+    // k34/(k34+k43) is formed once, for the draws of regimes 0/1 or for the
+    // merged state 7 of regime 2 (never both)
+    const RyrMasks m = ryr_masks(w);
+    if (m.s7 | (regime == 2 ? m.s3 | m.s4 : 0u)) p34 = qdiv(k34, k34 + R(k43));
+    uint32_t ex = S.exmask;
+    while (ex) {
+      const int b = __ffs(ex) - 1;  // the RyR's nibble
+      ex &= ex - 1u;
+      const uint32_t y = exw[0];  // in RyR order, from a shifting window (static register indices)
+      exw[0] = exw[1];
+      exw[1] = exw[2];
+      exw[2] = exw[3];
+      exw[3] = exw[4];
+      int s;
+      if (((w >> (8 + b)) & 15u) == 7u) s = u_below(y, p34) ? 4 : 3;
+      else s = u_below(y, qdiv(k56, k56 + R(k65))) ? 6 : 5;
+      w = set_field(w, 8 + b, s);
     }
-    if ((regime <= 1 && has7) || (regime == 2 && (has7 || has34))) p34 = qdiv(k34, k34 + R(k43));
-  #pragma unroll
-    for (int i = 0; i < kRyR; i++) {
-      int s = ryr_of(w, i);
-      if (regime == 0) {
-        if (s == 7 || s == 8) {
-          const uint32_t y = exw[0];
-          exw[0] = exw[1];
-          exw[1] = exw[2];
-          exw[2] = exw[3];
-          exw[3] = exw[4];
-          if (s == 7) s = u_below(y, p34) ? 4 : 3;
-          else s = u_below(y, qdiv(k56, k56 + R(k65))) ? 6 : 5;
-        }
-      } else if (regime == 1) {
-        if (s == 7) {
-          const uint32_t y = exw[0];
-          exw[0] = exw[1];
-          exw[1] = exw[2];
-          exw[2] = exw[3];
-          exw[3] = exw[4];
-          s = u_below(y, p34) ? 4 : 3;
-        }
-        if (s == 5 || s == 6) s = 8;
-      } else {
-        if (s == 3 || s == 4) s = 7;
-        else if (s == 5 || s == 6) s = 8;
-      }
-      w = set_field(w, 8 + 4 * i, s);
-    }
+    w = merge_ryr(w, regime);
   }
   {
-    bool need7 = false, need8 = false;
-  #pragma unroll
-    for (int i = 0; i < kRyR; i++) {
-      const int s = ryr_of(w, i);
-      need7 |= (s == 7);
-      need8 |= (s == 8);
-    }
+    const RyrMasks m = ryr_masks(w);
+    const bool need7 = m.s7 != 0u, need8 = m.s8 != 0u;
     const R T2 = R(k21) + k23 + k25, T3 = R(k32) + k34, T5 = R(k52) + k54 + k56;
     const R T4 = R(k43 + k45);
     R T7 = R(0), T8 = R(0);
@@ -736,15 +758,10 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
     }
   #pragma unroll
     for (int i = 0; i < kRyR; i++) {
-      const int s = ryr_of(w, i);
-      R r = k12;
-      r = (s == 2) ? T2 : r;
-      r = (s == 3) ? T3 : r;
-      r = (s == 4) ? T4 : r;
-      r = (s == 5) ? T5 : r;
-      r = (s == 6) ? R(k65) : r;
-      r = (s == 7) ? T7 : r;
-      r = (s == 8) ? T8 : r;
+      // by the bits of the state, 1 .. 8
+      const bool b0 = (w >> (8 + 4 * i)) & 1u, b1 = (w >> (9 + 4 * i)) & 1u, b2 = (w >> (10 + 4 * i)) & 1u;
+      const R lo = b1 ? (b0 ? T3 : T2) : (b0 ? k12 : T8), hi = b1 ? (b0 ? T7 : R(k65)) : (b0 ? T5 : T4);
+      const R r = b2 ? hi : lo;
       R0[2 + i] = r;
     }
   }
@@ -806,7 +823,7 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
   }
   if (leave_ge(bw[7], dt, R0[7])) w = set_field(w, 28, 3 - cl_of(w));
   lopen = lcc_open(w) ? R(1) : R(0);
-  if (moved) nopen = ryr_open_count(w);
+  if (moved) nopen = ryr_open_masked(w);
   F.nsub++;
 }
 
@@ -841,28 +858,8 @@ __device__ __forceinline__ void sub_begin(Sub4<double>& S) {
   for (int i = 0; i < kRyR; i++) S.exw[i] = 0u;
 }
 
-// The five RyR states of a channel word as masks over their nibbles (bit 0 of
-// nibble i set when RyR i is in the state).
-struct RyrMasks {
-  uint32_t s1, s2, s3, s4, s5, s6, s7, s8;
-};
-__device__ __forceinline__ RyrMasks ryr_masks(uint32_t w) {
-  const uint32_t r = w >> 8;
-  const uint32_t b0 = r & 0x11111u, b1 = (r >> 1) & 0x11111u, b2 = (r >> 2) & 0x11111u;
-  RyrMasks m;
-  m.s1 = b0 & ~b1 & ~b2;
-  m.s2 = ~b0 & b1 & ~b2;
-  m.s3 = b0 & b1 & ~b2;
-  m.s4 = ~b0 & ~b1 & b2;
-  m.s5 = b0 & ~b1 & b2;
-  m.s6 = ~b0 & b1 & b2;
-  m.s7 = b0 & b1 & b2;
-  m.s8 = (r >> 3) & 0x11111u;
-  return m;
-}
 __device__ __forceinline__ double jryr_open(uint32_t w) {
-  const RyrMasks m = ryr_masks(w);
-  const int n = __popc(m.s3 | m.s4 | m.s7);
+  const int n = ryr_open_masked(w);
   double v = 0.0;
   v = (n == 1) ? JRyRmax * 1.0 : v;
   v = (n == 2) ? JRyRmax * 2.0 : v;
@@ -945,18 +942,7 @@ __device__ __forceinline__ void substep_a(Fru4<double>& F, Sub4<double>& S, cons
     const double cc = imin(cass, threshMAXCa);
     S.regime = ilt(cc, threshCa56to8) ? 0 : (ilt(cc, threshCa34to7) ? 1 : 2);
   }
-  {
-    // extra draws: regime 0 resolves 7 and 8, regime 1 resolves 7 (in cleft,
-    // then RyR order); the four counts travel as the bytes of one word
-    const RyrMasks m = ryr_masks(w);
-    S.exmask = (S.regime == 0) ? (m.s7 | m.s8) : (S.regime == 1) ? m.s7 : 0u;
-    S.ne = __popc(S.exmask);
-    uint32_t n = (uint32_t)S.ne << (8 * g.c);
-    n |= __shfl_xor_sync(g.mask, n, 1);
-    n |= __shfl_xor_sync(g.mask, n, 2);
-    S.etot = (int)((n * 0x01010101u) >> 24);
-    S.pre = (int)(((n & ((1u << (8 * g.c)) - 1u)) * 0x01010101u) >> 24);
-  }
+  draw_layout(g, w, S.regime, S.exmask, S.ne, S.pre, S.etot);
   fetch_old(sc, g, F.mti, S.pre, S.ne, S.etot, S.exw, S.bw);
   // ---- voltage terms at the substep start, one exponential per lane ----
   const double V = F.dep[0];
@@ -1072,17 +1058,8 @@ __device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, cons
       else s = u_below(y, fast_div(k56, k56 + k65)) ? 6u : 5u;
       w = set_field(w, 8 + b, (int)s);
     }
-    m = ryr_masks(w);
   }
-  // merged states: 3, 4 -> 7 in regime 2; 5, 6 -> 8 in regimes 1 and 2
-  if (regime == 2) {
-    const uint32_t c = (m.s3 | m.s4) << 8;
-    w = (w & ~(c * 15u)) | (c * 7u);
-  }
-  if (regime != 0) {
-    const uint32_t c = (m.s5 | m.s6) << 8;
-    w = (w & ~(c * 15u)) | (c << 3);
-  }
+  w = merge_ryr(w, regime);
   m = ryr_masks(w);
   // ---- exit totals of the RyR states present, and their maximum ----
   double mx = imax(S.Rl, S.Rv);
