@@ -202,28 +202,40 @@ __device__ __forceinline__ R gmax(const Group& g, R v) {
   return v;
 }
 
-// In-place regeneration of one FRU's 624 words (mt19937_local.c:97-154) by
-// all 32 lanes of the warp, 32 consecutive words per step.  Word k < 227
-// reads the old word k + 397 (not reached yet), word k >= 227 the new word
-// k - 227 (written at least seven steps earlier) and word 623 the new words 0
-// and 396, as in the sequential loop; every lane reads before the barrier
-// and writes after it.
-__device__ __forceinline__ void regen32(uint32_t* m, int lane) {
-  for (int k0 = 0; k0 < kMtN; k0 += 32) {
-    const int k = k0 + lane;
-    const bool in = k < kMtN;
-    uint32_t nw = 0u;
-    if (in) {
+// Words k0 .. k0 + 32*STEPS - 1 of a row's regeneration (below 624), by the
+// warp: every lane reads all its words before the barrier and writes after it.
+template <int STEPS>
+__device__ __forceinline__ void regen_chunk(uint32_t* m, int k0, int lane) {
+  uint32_t nw[STEPS];
+#pragma unroll
+  for (int j = 0; j < STEPS; j++) {
+    const int k = k0 + 32 * j + lane;
+    if (k < kMtN) {
       const uint32_t cur = m[k];
       const uint32_t nxt = m[(k + 1 == kMtN) ? 0 : k + 1];
       const uint32_t far = m[(k + kMtM < kMtN) ? k + kMtM : k + kMtM - kMtN];
       const uint32_t y = (cur & 0x80000000u) | (nxt & 0x7fffffffu);
-      nw = far ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+      nw[j] = far ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
     }
-    __syncwarp();
-    if (in) m[k] = nw;
-    __syncwarp();
   }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < STEPS; j++) {
+    const int k = k0 + 32 * j + lane;
+    if (k < kMtN) m[k] = nw[j];
+  }
+  __syncwarp();
+}
+// In-place regeneration of one FRU's 624 words (mt19937_local.c:97-154) by
+// all 32 lanes of the warp, in three chunks of 224, 224 and 176 words whose
+// loads are all in flight together: word k < 227 reads the old word k + 397,
+// word k >= 227 the new word k - 227, which is in an earlier chunk, and word
+// 623 the new words 0 and 396, as in the sequential loop.  (One step of 32
+// words after another waited for 20 loads in turn.)
+__device__ __forceinline__ void regen32(uint32_t* m, int lane) {
+  regen_chunk<7>(m, 0, lane);
+  regen_chunk<7>(m, 224, lane);
+  regen_chunk<6>(m, 448, lane);
 }
 __device__ __forceinline__ void copy4(uint32_t* dst, const uint32_t* src, const Group& g) {
   for (int k = g.c; k < kMtN; k += 4) dst[k] = src[k];
