@@ -3,6 +3,7 @@
 // / save / resume operations that replace the MPI layer of mpi_master.c.
 #include <cuda_runtime.h>
 #include <stdarg.h>
+#include <math.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -14,6 +15,7 @@
 #include "gw_diag.h"
 #include "gw_fru.h"
 #include "gw_kernels.h"
+#include "gw_fru_core.cuh"
 #include "gw_fru_model.cuh"
 #include "gw_ctx_impl.h"
 
@@ -101,9 +103,10 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   AL(d.mti_s, nf * sizeof(int));
   AL(d.mt_hold, nf * gw::kMtStride * sizeof(uint32_t));
   AL(d.hold_epoch, nf * sizeof(uint32_t));
-  // partial sums of the widest grid: 8-FRU blocks of the cleft-parallel kernel
-  AL(d.partials, (size_t)((nfru + 7) / 8) * 16 * sizeof(double));
-  AL(d.ticket, sizeof(unsigned));
+  // partial sums of the 8-FRU groups and of the chunks of 32 groups
+  const size_t ngroups = (size_t)(nfru + 7) / 8, nchunks = (ngroups + 31) / 32;
+  AL(d.partials, (ngroups + nchunks) * 16 * sizeof(double));
+  AL(d.ticket, (1 + nchunks) * sizeof(unsigned));
   AL(d.out, 32 * sizeof(double));
   AL(d.substeps, sizeof(unsigned long long));
   AL(d.qctl, 8 * sizeof(unsigned));
@@ -111,10 +114,14 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   AL(d.heavy_tag, 2 * nf * sizeof(uint32_t));
 #undef AL
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_out, 32 * sizeof(double));
+  if (e == cudaSuccess) e = cudaHostAlloc((void**)&c->h_out, 32 * sizeof(double), cudaHostAllocMapped);
+  if (e == cudaSuccess) {
+    memset(c->h_out, 0, 32 * sizeof(double));
+    e = cudaHostGetDevicePointer((void**)&d.res, c->h_out, 0);
+  }
   for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
   for (int i = 0; i < 2 && e == cudaSuccess; i++) e = cudaEventCreate(&c->pev[i]);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d.ticket, 0, sizeof(unsigned), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.ticket, 0, (1 + nchunks) * sizeof(unsigned), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.out, 0, 32 * sizeof(double), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.substeps, 0, sizeof(unsigned long long), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.hold_epoch, 0xff, nf * sizeof(uint32_t), c->stream);
@@ -354,32 +361,24 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
   if (c->batch) {
     int rc = gw_batch_post(c, p, c->h_out);
     if (rc) return rc;
-    if (c->h_out[gw::kOutError] != 0.0)
-      return set_err(GW_EINVAL, "FRU stage [%g, %g]: substep limit reached (corrupted FRU state: NaN or "
-                     "out-of-range concentrations)", t0, tf);
-    if (num)
-      for (int k = 0; k < 5; k++) num[k] = c->h_out[k];
-    if (out)
-      for (int k = 0; k < 4; k++) out[k] = c->h_out[5 + k];
-    return GW_OK;
-  }
-  if (c->profiling) CK(cudaEventRecord(c->pev[0], c->stream));
-  CK(launch_stage_variant(c, p));
-  c->launches++;
-  if (c->sum_order == GW_SUM_REFERENCE) {
-    CK(gw::launch_flux_seq(c->d, p, c->stream));
+  } else {
+    // the kernels write the sums into h_out itself
+    if (c->profiling) CK(cudaEventRecord(c->pev[0], c->stream));
+    CK(launch_stage_variant(c, p));
     c->launches++;
+    if (c->sum_order == GW_SUM_REFERENCE) {
+      CK(gw::launch_flux_seq(c->d, c->stream));
+      c->launches++;
+    }
+    if (c->profiling) CK(cudaEventRecord(c->pev[1], c->stream));
+    CK(cudaStreamSynchronize(c->stream));
   }
-  if (c->profiling) CK(cudaEventRecord(c->pev[1], c->stream));
-  CK(cudaMemcpyAsync(c->h_out, c->d.out, 32 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   if (c->h_out[gw::kOutError] != 0.0) {
-    double z = 0.0;
-    CK(cudaMemcpy(c->d.out + gw::kOutError, &z, sizeof z, cudaMemcpyHostToDevice));
+    c->h_out[gw::kOutError] = 0.0;
     return set_err(GW_EINVAL, "FRU stage [%g, %g]: substep limit reached (corrupted FRU state: NaN or "
                    "out-of-range concentrations)", t0, tf);
   }
-  if (c->profiling) {
+  if (c->profiling && !c->batch) {
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, c->pev[0], c->pev[1]));
     c->prof_ms += ms;
@@ -387,8 +386,11 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
   }
   if (num)
     for (int k = 0; k < 5; k++) num[k] = c->h_out[k];
-  if (out)
-    for (int k = 0; k < 4; k++) out[k] = c->h_out[5 + k];
+  if (out) {
+    // mpi_master.c:447-468; on one GPU lane this algebra took 4 us of every launch
+    gw::currents_from_sums(c->d.nfru, c->nfru_scale, depf, c->h_out, out);
+    out[2] = out[2] * c->pca_scale;  // ICa is proportional to the LCC permeability
+  }
   return GW_OK;
 }
 
@@ -412,7 +414,6 @@ extern "C" int gw_avg_sums(gw_ctx* c, double num[11]) {
   else
     CK(gw::launch_avg(c->d, c->stream));
   c->launches++;
-  CK(cudaMemcpyAsync(c->h_out + 16, c->d.out + 16, 11 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   for (int k = 0; k < 11; k++) num[k] = c->h_out[16 + k];
   return GW_OK;

@@ -45,9 +45,9 @@ struct gw_batch {
   gw::DevState* d_cells = nullptr;
   gw::StageParams* d_params = nullptr;
   int* d_block0 = nullptr;
-  double* d_outs = nullptr;
   gw::StageParams* h_params = nullptr;
-  double* h_outs = nullptr;
+  double* h_outs = nullptr;  // mapped at outs
+  double* outs = nullptr;
   int* h_block0 = nullptr;
   gw::DevState* h_cells = nullptr;
   cudaEvent_t ev[2] = {};
@@ -61,7 +61,6 @@ static void free_arrays(gw_batch* b) {
   if (b->d_cells) cudaFree(b->d_cells);
   if (b->d_params) cudaFree(b->d_params);
   if (b->d_block0) cudaFree(b->d_block0);
-  if (b->d_outs) cudaFree(b->d_outs);
   if (b->h_params) cudaFreeHost(b->h_params);
   if (b->h_outs) cudaFreeHost(b->h_outs);
   if (b->h_block0) cudaFreeHost(b->h_block0);
@@ -69,7 +68,6 @@ static void free_arrays(gw_batch* b) {
   b->d_cells = nullptr;
   b->d_params = nullptr;
   b->d_block0 = nullptr;
-  b->d_outs = nullptr;
   b->h_params = nullptr;
   b->h_outs = nullptr;
   b->h_block0 = nullptr;
@@ -84,12 +82,15 @@ static cudaError_t ensure_capacity(gw_batch* b, int n) {
   cudaError_t e = cudaMalloc(&b->d_cells, sizeof(gw::DevState) * cap);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_params, sizeof(gw::StageParams) * cap);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_block0, sizeof(int) * (cap + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_outs, sizeof(double) * gw::kBatchOutStride * cap);
   if (e == cudaSuccess) e = cudaMallocHost(&b->h_params, sizeof(gw::StageParams) * cap);
-  if (e == cudaSuccess) e = cudaMallocHost(&b->h_outs, sizeof(double) * gw::kBatchOutStride * cap);
+  if (e == cudaSuccess)
+    e = cudaHostAlloc((void**)&b->h_outs, sizeof(double) * gw::kBatchOutStride * cap, cudaHostAllocMapped);
   if (e == cudaSuccess) e = cudaMallocHost(&b->h_block0, sizeof(int) * (cap + 1));
   if (e == cudaSuccess) e = cudaMallocHost(&b->h_cells, sizeof(gw::DevState) * cap);
-  if (e == cudaSuccess) e = cudaMemset(b->d_outs, 0, sizeof(double) * gw::kBatchOutStride * cap);
+  if (e == cudaSuccess) {
+    memset(b->h_outs, 0, sizeof(double) * gw::kBatchOutStride * cap);
+    e = cudaHostGetDevicePointer((void**)&b->outs, b->h_outs, 0);
+  }
   if (e != cudaSuccess) {
     free_arrays(b);
     b->cap = 0;
@@ -127,7 +128,7 @@ static cudaError_t launch_round(gw_batch* b) {
   a.cells = b->d_cells;
   a.params = b->d_params;
   a.block0 = b->d_block0;
-  a.outs = b->d_outs;
+  a.outs = b->outs;
   a.ncells = n;
   if (b->profiling) cudaEventRecord(b->ev[0], b->stream);
   e = (b->precision == 1) ? gw::launch_stage_mixed_batch(a, b->nblocks, b->warps, b->stream)
@@ -135,9 +136,7 @@ static cudaError_t launch_round(gw_batch* b) {
   if (e != cudaSuccess) return e;
   b->launches++;
   if (b->profiling) cudaEventRecord(b->ev[1], b->stream);
-  e = cudaMemcpyAsync(b->h_outs, b->d_outs, sizeof(double) * gw::kBatchOutStride * n, cudaMemcpyDeviceToHost,
-                      b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  e = cudaStreamSynchronize(b->stream);  // the kernel has written h_outs
   if (e == cudaSuccess && b->profiling) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);

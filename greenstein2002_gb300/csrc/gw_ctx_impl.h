@@ -11,7 +11,7 @@ struct gw_batch;
 struct gw_ctx {
   gw::DevState d;
   cudaStream_t stream = nullptr;
-  double* h_out = nullptr;  // pinned [32]
+  double* h_out = nullptr;  // pinned [32], mapped at d.res
   double nfru_scale = 1.0;
   uint32_t epoch = 0;
   int pending = 0;          // kFlagSave / kFlagResume to fold into the next launch

@@ -1250,48 +1250,6 @@ __device__ __forceinline__ void advance4(StageCtx& sc, const Group& g, bool live
   nsub = F.nsub;
 }
 
-// Sum over the 32 lanes of a warp: one fixed shuffle tree.
-template <int NV>
-__device__ __forceinline__ void warp_sum(double v[NV]) {
-#pragma unroll
-  for (int k = 0; k < NV; k++)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-}
-
-// Cross-FRU sums of one cell, independent of the launch shape: every warp
-// (8 FRUs, group grp of the cell's ngroups) stores its warp total, and the
-// last warp to arrive adds the group totals in a fixed lane-strided order
-// and one warp tree.  Whatever the warps per block, the sums are the same
-// bits.  Returns true in lane 0 of that last warp, with the totals in tot[].
-template <int NV>
-__device__ __forceinline__ bool cell_finish(const double v[NV], double* partials, unsigned* ticket, double tot[NV],
-                                            int grp, int ngroups) {
-  const int lane = threadIdx.x & 31;
-  unsigned last = 0u;
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; k++) partials[grp * NV + k] = v[k];
-    __threadfence();
-    last = (atomicAdd(ticket, 1u) == (unsigned)ngroups - 1u) ? 1u : 0u;
-  }
-  last = __shfl_sync(0xffffffffu, last, 0);
-  if (!last) return false;
-  __threadfence();
-  double s[NV];
-#pragma unroll
-  for (int k = 0; k < NV; k++) s[k] = 0.0;
-  for (int b = lane; b < ngroups; b += 32)
-#pragma unroll
-    for (int k = 0; k < NV; k++) s[k] += __ldcg(&partials[b * NV + k]);
-  warp_sum<NV>(s);
-  if (lane == 0) {
-    *ticket = 0u;
-#pragma unroll
-    for (int k = 0; k < NV; k++) tot[k] = s[k];
-  }
-  return lane == 0;
-}
-
 // The stage of one cell, block bidx of the cell's blocks (blockDim.x / 32
 // warps of 8 FRUs each): load, optional snapshot save/restore, advance,
 // store, and the fused deterministic flux reduction
@@ -1303,44 +1261,19 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// Where a launch's cell totals go: OutFin writes them to the cell's out[]
-// slots (the host reads them back); the device-resident integrator passes
-// its own finisher.  Called by one lane, with the 5 flux numerators, the
-// currents (Jxfer, Jtr, ICa, Ito2) and, when the launch carried
-// kFlagAvg, the 11 output-average sums (else null).
+// Where a launch's cell totals go: OutFin writes the 5 flux numerators to the
+// launch's out[] slots (host memory, where the host forms the currents); the
+// device-resident integrators pass their own finishers.  Called by one lane,
+// with the flux numerators and, when the launch carried kFlagAvg, the 11
+// output-average sums (else null).
 struct OutFin {
   double* out;
-  __device__ void operator()(const double tot[5], const double cur[4], const double*) const {
+  __device__ void operator()(const double tot[5], const double*) const {
 #pragma unroll
     for (int k = 0; k < 5; k++) out[k] = tot[k];
-#pragma unroll
-    for (int k = 0; k < 4; k++) out[5 + k] = cur[k];
   }
   __device__ void error() const { out[kOutError] = 1.0; }
 };
-
-// The 11 output-average terms of one cleft (calc_fru_avg_local.c:27-105):
-// the FRU-level ones (CaJSR and its buffered total) on the cleft-0 lane.
-__device__ __forceinline__ void avg_terms(int c, double jsr, double ss, uint32_t w, double a[11]) {
-  int no = 0, ready = 0;
-#pragma unroll
-  for (int i = 0; i < kRyR; i++) {
-    const int r = ryr_of(w, i);
-    no += ryr_open(r);
-    ready += (r == 1 || r == 2);
-  }
-  a[0] = ss;
-  a[1] = (c == 0) ? jsr : 0.0;
-  a[2] = JRyRmax * ((double)no) * (jsr - ss);
-  a[3] = (double)no;
-  a[4] = (double)ready;
-  a[5] = ss * (1.0 + BSRtot / (KBSR + ss) + BSLtot / (KBSL + ss));
-  a[6] = (c == 0) ? jsr * (1.0 + CSQNtot / (KmCSQN + jsr)) : 0.0;
-  a[7] = (lcc_of(w) <= 6) ? 1.0 : 0.0;
-  a[8] = (vdi_of(w) == 2) ? 1.0 : 0.0;
-  a[9] = lcc_open(w) ? 1.0 : 0.0;
-  a[10] = (cl_of(w) == 2) ? 1.0 : 0.0;
-}
 
 template <typename R, typename Fin>
 __device__ __forceinline__ void stage_body_fin(const DevState& s, const StageParams& p, int bidx, const Fin& fin) {
@@ -1364,7 +1297,6 @@ __device__ __forceinline__ void stage_body_fin(const DevState& s, const StagePar
   g.base = lane & ~3;
   g.mask = 0xfu << g.base;
   const int f = grp * 8 + (lane >> 2);
-  double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   uint32_t nsub = 0;
   bool overflow = false;
   const bool active = f < s.nfru;  // uniform over each 4-lane group
@@ -1420,48 +1352,32 @@ __device__ __forceinline__ void stage_body_fin(const DevState& s, const StagePar
     }
     s.frus[(g.c + 1) * nf + f] = cass;
     s.chan[g.c * nf + f] = w;
-    v[0] = cass;
-    v[1] = (g.c == 0) ? cajsr : 0.0;
-    if (lcc_open(w)) {
-      v[2] = cass;
-      v[3] = 1.0;
-    }
-    if (cl_of(w) == 2) v[4] = 1.0;
   }
   __syncwarp();
   if (s.trace_ns && lane == 0) s.trace_ns[2 * grp + 1] = global_ns();
   if (overflow) fin.error();
   if (s.substeps) {
-    unsigned long long c = (g.c == 0) ? nsub : 0;
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if (lane == 0 && c) atomicAdd(s.substeps, c);
+    unsigned c = __reduce_add_sync(0xffffffffu, (g.c == 0) ? nsub : 0u);
+    if (lane == 0 && c) atomicAdd(s.substeps, (unsigned long long)c);
   }
   if (p.flags & kFlagAvg) {
-    // flux numerators and output averages in one pass (16 partials per group)
-    double u[16];
-#pragma unroll
-    for (int k = 0; k < 5; k++) u[k] = v[k];
-    double a[11];
-    avg_terms(g.c, cajsr, cass, w, a);
-#pragma unroll
-    for (int k = 0; k < 11; k++) u[5 + k] = active ? a[k] : 0.0;
-    warp_sum<16>(u);
-    double tot[16];
-    if (cell_finish<16>(u, s.partials, s.ticket, tot, grp, ngroups)) {
-      double cur[4];
-      currents_from_sums(s.nfru, p.nfru_scale, p.depf, tot, cur);
-      cur[2] = cur[2] * p.pca_scale;  // ICa is proportional to the LCC permeability
-      fin(tot, cur, tot + 5);
+    AvgSums v = {};
+    if (active) avg_terms(g.c, cajsr, cass, w, v);
+    store_group(s, grp, v, lane);
+    if (finish_groups(s, v, grp >> 5, 1u, lane) && lane == 0) {
+      double tot[16];
+      unpack_avg(v, tot);
+      fin(tot, tot + 5);
     }
     return;
   }
-  warp_sum<5>(v);
-  double tot[5];
-  if (cell_finish<5>(v, s.partials, s.ticket, tot, grp, ngroups)) {
-    double cur[4];
-    currents_from_sums(s.nfru, p.nfru_scale, p.depf, tot, cur);
-    cur[2] = cur[2] * p.pca_scale;  // ICa is proportional to the LCC permeability
-    fin(tot, cur, nullptr);
+  FluxSums v = {};
+  if (active) flux_terms(g.c, cajsr, cass, w, v);
+  store_group(s, grp, v, lane);
+  if (finish_groups(s, v, grp >> 5, 1u, lane) && lane == 0) {
+    double tot[5];
+    unpack_flux(v, tot);
+    fin(tot, nullptr);
   }
 }
 

@@ -66,8 +66,144 @@ __device__ __forceinline__ bool grid_finish(const double v[NV], double* partials
   return threadIdx.x == 0;
 }
 
+// ---- sums over the FRUs of a cell, the same bits for every launch shape ---------
+// ND double sums and NI words of two 32-bit counts each: the counts (open
+// channels and the like) are integers and need no FP64 additions.
+template <int ND, int NI>
+struct Sums {
+  double d[ND];
+  unsigned long long n[NI];
+};
+using FluxSums = Sums<3, 1>;  // CaSS, CaJSR, CaSS of open LCCs; open LCCs, open Cl channels
+using AvgSums = Sums<6, 3>;   // FluxSums, JRyR, buffered CaSS and CaJSR; open and ready RyRs; LCCs in mode normal, open VDIs
+
+// This lane's cleft (c; the FRU-level terms on the cleft-0 lane):
+// calc_fru_flux_local.c:45-70 and calc_fru_avg_local.c:27-105.
+template <int ND, int NI>
+__device__ __forceinline__ void flux_terms(int c, double jsr, double ss, uint32_t w, Sums<ND, NI>& v) {
+  v.d[0] = ss;
+  v.d[1] = (c == 0) ? jsr : 0.0;
+  v.d[2] = lcc_open(w) ? ss : 0.0;
+  v.n[0] = (unsigned long long)(lcc_open(w) ? 1u : 0u) | ((unsigned long long)((cl_of(w) == 2) ? 1u : 0u) << 32);
+}
+__device__ __forceinline__ void avg_terms(int c, double jsr, double ss, uint32_t w, AvgSums& v) {
+  flux_terms(c, jsr, ss, w, v);
+  unsigned no = 0, ready = 0;
+#pragma unroll
+  for (int i = 0; i < kRyR; i++) {
+    const int r = ryr_of(w, i);
+    no += ryr_open(r);
+    ready += (r == 1 || r == 2);
+  }
+  v.d[3] = JRyRmax * ((double)no) * (jsr - ss);
+  v.d[4] = ss * (1.0 + BSRtot / (KBSR + ss) + BSLtot / (KBSL + ss));
+  v.d[5] = (c == 0) ? jsr * (1.0 + CSQNtot / (KmCSQN + jsr)) : 0.0;
+  v.n[1] = (unsigned long long)no | ((unsigned long long)ready << 32);
+  v.n[2] = (unsigned long long)((lcc_of(w) <= 6) ? 1u : 0u) | ((unsigned long long)((vdi_of(w) == 2) ? 1u : 0u) << 32);
+}
+// the 5 flux numerators, and the 11 output sums after them
+template <int ND, int NI>
+__device__ __forceinline__ void unpack_flux(const Sums<ND, NI>& v, double tot[5]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) tot[k] = v.d[k];
+  tot[3] = (double)(uint32_t)v.n[0];
+  tot[4] = (double)(uint32_t)(v.n[0] >> 32);
+}
+__device__ __forceinline__ void unpack_avg(const AvgSums& v, double tot[16]) {
+  unpack_flux(v, tot);
+  const double a[11] = {v.d[0], v.d[1], v.d[3], (double)(uint32_t)v.n[1], (double)(uint32_t)(v.n[1] >> 32), v.d[4], v.d[5],
+                        (double)(uint32_t)v.n[2], (double)(uint32_t)(v.n[2] >> 32), tot[3], tot[4]};
+#pragma unroll
+  for (int k = 0; k < 11; k++) tot[5 + k] = a[k];
+}
+
+// Over the 32 lanes of a warp by one fixed shuffle tree; the total in lane 0.
+template <int ND, int NI>
+__device__ __forceinline__ void warp_sum(Sums<ND, NI>& v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < ND; k++) v.d[k] += __shfl_down_sync(0xffffffffu, v.d[k], o);
+#pragma unroll
+    for (int k = 0; k < NI; k++) v.n[k] += __shfl_down_sync(0xffffffffu, v.n[k], o);
+  }
+}
+// Partial sums of slot i (a group, or past the groups a chunk) in partials.
+template <int ND, int NI>
+__device__ __forceinline__ void put_partial(const DevState& s, int i, const Sums<ND, NI>& v) {
+  double* q = s.partials + (size_t)i * (ND + NI);
+#pragma unroll
+  for (int k = 0; k < ND; k++) q[k] = v.d[k];
+#pragma unroll
+  for (int k = 0; k < NI; k++) q[ND + k] = __longlong_as_double((long long)v.n[k]);
+}
+template <int ND, int NI>
+__device__ __forceinline__ void get_partial(const DevState& s, int i, Sums<ND, NI>& v) {
+  const double* q = s.partials + (size_t)i * (ND + NI);
+#pragma unroll
+  for (int k = 0; k < ND; k++) v.d[k] = __ldcg(q + k);
+#pragma unroll
+  for (int k = 0; k < NI; k++) v.n[k] = (unsigned long long)__double_as_longlong(__ldcg(q + ND + k));
+}
+// The warp's lanes (8 FRUs x 4 clefts) into group grp's partial sums.
+template <int ND, int NI>
+__device__ __forceinline__ void store_group(const DevState& s, int grp, Sums<ND, NI>& v, int lane) {
+  warp_sum(v);
+  if (lane == 0) put_partial(s, grp, v);
+}
+
+// Cross-FRU sums of one cell, independent of the launch shape: groups of 8
+// FRUs are summed by chunks of 32 (one group per lane, a shuffle tree), the
+// chunks lane-strided and by one more tree.  The warp that completes a chunk
+// sums it and the one that completes the last chunk the cell, both told by
+// tickets (ticket[1 + chunk] counts groups, ticket[0] chunks; each is reset by
+// the warp that completes it).  Summing all groups in the cell's last warp
+// instead kept that one warp at 5 dependent FP64 additions per 32 groups:
+// the flux launch of a 12,500-FRU cell took 30 us, against 15 us now (with the
+// counts as integers and the current algebra on the host).
+// Called by a warp that has stored `count` groups of `chunk`; true (in every
+// lane) when that completed the cell, with the totals in lane 0's v.
+template <int ND, int NI>
+__device__ __forceinline__ bool finish_groups(const DevState& s, Sums<ND, NI>& v, int chunk, unsigned count, int lane) {
+  const int ngroups = (s.nfru + 7) >> 3, nchunks = (ngroups + 31) >> 5;
+  const int size = min(32, ngroups - 32 * chunk);
+  unsigned last = 0u;
+  if (lane == 0) {
+    __threadfence();
+    last = (atomicAdd(&s.ticket[1 + chunk], count) + count == (unsigned)size) ? 1u : 0u;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+  __threadfence();
+  v = {};
+  if (lane < size) get_partial(s, 32 * chunk + lane, v);
+  warp_sum(v);
+  if (lane == 0) s.ticket[1 + chunk] = 0u;
+  if (nchunks == 1) return true;
+  last = 0u;
+  if (lane == 0) {
+    put_partial(s, ngroups + chunk, v);
+    __threadfence();
+    last = (atomicAdd(&s.ticket[0], 1u) == (unsigned)nchunks - 1u) ? 1u : 0u;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+  __threadfence();
+  v = {};
+  for (int b = lane; b < nchunks; b += 32) {
+    Sums<ND, NI> t;
+    get_partial(s, ngroups + b, t);
+#pragma unroll
+    for (int k = 0; k < ND; k++) v.d[k] += t.d[k];
+#pragma unroll
+    for (int k = 0; k < NI; k++) v.n[k] += t.n[k];
+  }
+  warp_sum(v);
+  if (lane == 0) s.ticket[0] = 0u;
+  return true;
+}
+
 // Flux numerators -> (Jxfer, Jtr, ICa, Ito2): mpi_master.c:447-468.
-static __device__ void currents_from_sums(int nfru, double scale, const double dep[3], const double num[5], double out[4]) {
+// Host code uses the host libm's exp, device code CUDA's.
+static __host__ __device__ inline void currents_from_sums(int nfru, double scale, const double dep[3], const double num[5], double out[4]) {
   const double V = dep[0], Cai = dep[1], CaNSR = dep[2];
   const double VFRT = V / RT_over_F, VFsqRT = (1000.0 * Faraday) * VFRT;
   const double e1 = exp(VFRT), e2 = e1 * e1;

@@ -10,7 +10,7 @@
 namespace gw {
 
 __global__ void __launch_bounds__(kMaxStageWarps * 32) fru_stage_mixed_kernel(DevState s, StageParams p) {
-  cleft::stage_body<float>(s, p, blockIdx.x, s.out);
+  cleft::stage_body<float>(s, p, blockIdx.x, s.res);
 }
 
 cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, cudaStream_t st) {
@@ -31,7 +31,7 @@ cudaError_t launch_stage_mixed_batch(const BatchArgs& a, int nblocks, int warps,
 }
 
 __global__ void __launch_bounds__(32, 16) fru_stage_mixed_packed_kernel(DevState s, StageParams p) {
-  cleft::stage_body_packed<float>(s, p, s.out);
+  cleft::stage_body_packed<float>(s, p, s.res);
 }
 
 cudaError_t launch_stage_mixed_packed(const DevState& s, const StageParams& p, int warps, cudaStream_t st) {

@@ -22,25 +22,21 @@
 
 namespace gw {
 
-// Flux numerators of the cell, summed in exactly the order of the
-// cleft-parallel kernels (gw_fru_cleft.cuh), so every stage kernel gives the
-// same bits: per 8-FRU group and cleft a fixed tree over the FRUs
-// ((x0+x4)+(x2+x6))+((x1+x5)+(x3+x7)), then (S0+S2)+(S1+S3) over the clefts,
-// then the lane-strided last-warp pass over the groups.
+// The partial sums of the warp's four 8-FRU groups in exactly the order of the
+// cleft-parallel kernels (store_group's tree over 32 lanes of 8 FRUs x 4
+// clefts), so every stage kernel gives the same bits: per group and cleft the
+// tree over the FRUs ((x0+x4)+(x2+x6))+((x1+x5)+(x3+x7)), then (S0+S2)+(S1+S3)
+// over the clefts; valid in lanes 0, 8, 16, 24.
 __device__ __forceinline__ double group8_sum(double x) {
   x += __shfl_down_sync(0xffffffffu, x, 4);
   x += __shfl_down_sync(0xffffffffu, x, 2);
   x += __shfl_down_sync(0xffffffffu, x, 1);
-  return x;  // valid in lanes 0, 8, 16, 24
+  return x;
 }
 
 __global__ void __launch_bounds__(kStageThreads) fru_stage_kernel(DevState s, StageParams p) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  double x[kClefts][5];
-#pragma unroll
-  for (int c = 0; c < kClefts; c++)
-#pragma unroll
-    for (int k = 0; k < 5; k++) x[c][k] = 0.0;
+  FluxSums x[kClefts] = {};
   uint32_t nsub = 0;
   bool overflow = false;
   if (f < s.nfru) {
@@ -80,23 +76,14 @@ __global__ void __launch_bounds__(kStageThreads) fru_stage_kernel(DevState s, St
     }
     rng.mti = mti;
     if (p.flags & kFlagAdvance) advance_fru(p, y, w, rng, nsub, overflow);
-    if (overflow) s.out[kOutError] = 1.0;
+    if (overflow) s.res[kOutError] = 1.0;
 #pragma unroll
     for (int i = 0; i < 5; i++) s.frus[i * nf + f] = y[i];
 #pragma unroll
     for (int c = 0; c < kClefts; c++) s.chan[c * nf + f] = w[c];
     s.mti[f] = rng.mti;
-    // flux numerators of this FRU's clefts (calc_fru_flux_local.c:45-70)
 #pragma unroll
-    for (int c = 0; c < kClefts; c++) {
-      x[c][0] = y[c + 1];
-      if (lcc_open(w[c])) {
-        x[c][2] = y[c + 1];
-        x[c][3] = 1.0;
-      }
-      if (cl_of(w[c]) == 2) x[c][4] = 1.0;
-    }
-    x[0][1] = y[0];
+    for (int c = 0; c < kClefts; c++) flux_terms(c, y[0], y[c + 1], w[c], x[c]);
   }
   if (s.substeps) {
     // substep counter (workload accounting): warp-aggregated atomic
@@ -104,45 +91,26 @@ __global__ void __launch_bounds__(kStageThreads) fru_stage_kernel(DevState s, St
     for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(s.substeps, c);
   }
-  double v[5];
+  FluxSums v;
 #pragma unroll
-  for (int k = 0; k < 5; k++) {
-    const double s0 = group8_sum(x[0][k]), s1 = group8_sum(x[1][k]);
-    const double s2 = group8_sum(x[2][k]), s3 = group8_sum(x[3][k]);
-    v[k] = (s0 + s2) + (s1 + s3);
+  for (int k = 0; k < 3; k++) {
+    const double s0 = group8_sum(x[0].d[k]), s1 = group8_sum(x[1].d[k]);
+    const double s2 = group8_sum(x[2].d[k]), s3 = group8_sum(x[3].d[k]);
+    v.d[k] = (s0 + s2) + (s1 + s3);
   }
+  v.n[0] = x[0].n[0] + x[1].n[0] + x[2].n[0] + x[3].n[0];
+  for (int o = 4; o > 0; o >>= 1) v.n[0] += __shfl_down_sync(0xffffffffu, v.n[0], o);
   // lanes 0, 8, 16, 24 hold the totals of their 8-FRU groups
   const int lane = threadIdx.x & 31;
   const int ngroups = (s.nfru + 7) >> 3, grp0 = (blockIdx.x * blockDim.x) >> 3;
   const int mine = min(4, ngroups - grp0);  // groups of this warp that hold FRUs
-  unsigned last = 0u;
-  if ((lane & 7) == 0 && (lane >> 3) < mine) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) s.partials[(grp0 + (lane >> 3)) * 5 + k] = v[k];
-  }
+  if ((lane & 7) == 0 && (lane >> 3) < mine) put_partial(s, grp0 + (lane >> 3), v);
   __syncwarp();
-  if (lane == 0) {
-    __threadfence();
-    last = (atomicAdd(s.ticket, (unsigned)mine) == (unsigned)(ngroups - mine)) ? 1u : 0u;
-  }
-  last = __shfl_sync(0xffffffffu, last, 0);
-  if (!last) return;
-  __threadfence();
-  double tot[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int b = lane; b < ngroups; b += 32)
+  if (finish_groups(s, v, grp0 >> 5, (unsigned)mine, lane) && lane == 0) {
+    double tot[5];
+    unpack_flux(v, tot);
 #pragma unroll
-    for (int k = 0; k < 5; k++) tot[k] += __ldcg(&s.partials[b * 5 + k]);
-#pragma unroll
-  for (int k = 0; k < 5; k++)
-    for (int o = 16; o > 0; o >>= 1) tot[k] += __shfl_down_sync(0xffffffffu, tot[k], o);
-  if (lane == 0) {
-    *s.ticket = 0u;
-    double cur[4];
-    currents_from_sums(s.nfru, p.nfru_scale, p.depf, tot, cur);
-#pragma unroll
-    for (int k = 0; k < 5; k++) s.out[k] = tot[k];
-#pragma unroll
-    for (int k = 0; k < 4; k++) s.out[5 + k] = cur[k];
+    for (int k = 0; k < 5; k++) s.res[k] = tot[k];
   }
 }
 
@@ -184,22 +152,21 @@ __global__ void __launch_bounds__(kStageThreads) fru_avg_kernel(DevState s) {
   double tot[11];
   if (grid_finish<11>(v, s.partials, s.ticket, smem, tot))
 #pragma unroll
-    for (int k = 0; k < 11; k++) s.out[16 + k] = tot[k];
+    for (int k = 0; k < 11; k++) s.res[16 + k] = tot[k];
 }
 
 // Reference-order sums (the parity mode of gw_set_sum_order): the flux
 // numerators added one FRU and one cleft after another, as
-// calc_fru_flux_local.c:44-70 does, then the currents of
-// mpi_master.c:447-468.  A sequential FP64 sum has exactly one rounding
+// calc_fru_flux_local.c:44-70 does.  A sequential FP64 sum has exactly one rounding
 // order, so each sum is one thread's dependent chain; the block stages the
 // stored FRU states in shared memory in coalesced chunks and three warps (on
 // three SM sub-partitions) run the three chains side by side: the CaSS sum,
 // the CaJSR sum, and the open-LCC CaSS sum with the two counts (integers,
 // exact).  About 4 dependent FP64 additions per FRU, so this mode is for
 // parity runs of small cells.  Runs after the stage launch and overwrites
-// out[0..8].
+// res[0..4].
 constexpr int kSeqThreads = 128, kSeqChunk = 512;
-__global__ void __launch_bounds__(kSeqThreads) fru_flux_seq_kernel(DevState s, StageParams p) {
+__global__ void __launch_bounds__(kSeqThreads) fru_flux_seq_kernel(DevState s) {
   __shared__ double sf[5][kSeqChunk];
   __shared__ uint32_t sw[kClefts][kSeqChunk];
   __shared__ double res[5];
@@ -242,14 +209,8 @@ __global__ void __launch_bounds__(kSeqThreads) fru_flux_seq_kernel(DevState s, S
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    const double tot[5] = {res[0], res[1], res[2], res[3], res[4]};
-    double cur[4];
-    currents_from_sums(s.nfru, p.nfru_scale, p.depf, tot, cur);
-    cur[2] = cur[2] * p.pca_scale;
 #pragma unroll
-    for (int k = 0; k < 5; k++) s.out[k] = tot[k];
-#pragma unroll
-    for (int k = 0; k < 4; k++) s.out[5 + k] = cur[k];
+    for (int k = 0; k < 5; k++) s.res[k] = res[k];
   }
 }
 
@@ -289,7 +250,7 @@ __global__ void __launch_bounds__(32) fru_avg_seq_kernel(DevState s) {
   }
   v[4] = (double)ready;
 #pragma unroll
-  for (int k = 0; k < 11; k++) s.out[16 + k] = v[k];
+  for (int k = 0; k < 11; k++) s.res[16 + k] = v[k];
 }
 
 // Knuth initialisation of every FRU's MT19937 state (mt19937_local.c:76-92),
@@ -333,8 +294,8 @@ cudaError_t launch_avg(const DevState& s, cudaStream_t st) {
   fru_avg_kernel<<<s.nblocks, kStageThreads, 0, st>>>(s);
   return cudaGetLastError();
 }
-cudaError_t launch_flux_seq(const DevState& s, const StageParams& p, cudaStream_t st) {
-  fru_flux_seq_kernel<<<1, kSeqThreads, 0, st>>>(s, p);
+cudaError_t launch_flux_seq(const DevState& s, cudaStream_t st) {
+  fru_flux_seq_kernel<<<1, kSeqThreads, 0, st>>>(s);
   return cudaGetLastError();
 }
 cudaError_t launch_avg_seq(const DevState& s, cudaStream_t st) {

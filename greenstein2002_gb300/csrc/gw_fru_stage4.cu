@@ -8,7 +8,7 @@
 namespace gw {
 
 __global__ void __launch_bounds__(kMaxStageWarps * 32) fru_stage4_kernel(DevState s, StageParams p) {
-  cleft::stage_body<double>(s, p, blockIdx.x, s.out);
+  cleft::stage_body<double>(s, p, blockIdx.x, s.res);
 }
 
 cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, cudaStream_t st) {
@@ -32,7 +32,7 @@ cudaError_t launch_stage4_batch(const BatchArgs& a, int nblocks, int warps, cuda
 // thread; 168 used, so twelve fit) against 191 uncapped (measured 4-13%
 // faster on the 16-cell ensemble, where the FP64 pipe is ~75% busy).
 __global__ void __launch_bounds__(32, 11) fru_stage4_packed_kernel(DevState s, StageParams p) {
-  cleft::stage_body_packed<double>(s, p, s.out);
+  cleft::stage_body_packed<double>(s, p, s.res);
 }
 
 cudaError_t launch_stage4_packed(const DevState& s, const StageParams& p, int warps, cudaStream_t st) {

@@ -38,10 +38,12 @@ enum : int { kSeedBase = 0, kSeedReference = 1 };
 //   mti[stride], mt[nfru][640] (FRU-major MT19937 rows)
 //   *_s               snapshot taken at the last save
 //   mt_hold/hold_epoch  copy-on-twist protection of the saved MT words
-//   partials[max(nblocks, ceil(nfru/8))][16], ticket: scratch of the
-//                     deterministic grid reduction
-//   out[32]           [0..4] flux sums, [5..8] Jxfer,Jtr,ICa,Ito2, [16..26] averages,
-//                     [31] error flag
+//   partials[groups + chunks][16], ticket[1 + chunks]: scratch of the
+//                     deterministic reductions (groups of 8 FRUs, chunks of 32 groups)
+//   res[32]           results the host reads, in its own (pinned, mapped) memory:
+//                     [0..4] flux sums, [16..26] averages, [31] error flag
+//   out[32]           the same of the round-based device integrator, in device
+//                     memory, with [5..8] Jxfer,Jtr,ICa,Ito2
 struct DevState {
   int nfru, stride, nblocks;
   double* frus;
@@ -56,6 +58,7 @@ struct DevState {
   double* partials;
   unsigned* ticket;
   double* out;
+  double* res;
   unsigned long long* substeps;
   // stage trace (null unless enabled): substeps of every FRU in the last
   // 4-lane launch, and each 8-FRU warp's begin/end global time (ns)
@@ -83,13 +86,13 @@ struct StageParams {
 // Many cells in one launch (cleft-parallel kernels): cell i owns blocks
 // block0[i] .. block0[i+1]-1 (8 FRUs per warp); params[i].flags < 0 means
 // the cell has no operation this round; its totals go to outs[i*32 ..] in the
-// layout of DevState::out.
+// layout of DevState::res.
 constexpr int kBatchOutStride = 32;
 struct BatchArgs {
   const DevState* cells;
   const StageParams* params;
   const int* block0;  // ncells + 1 prefix sums
-  double* outs;       // [ncells][kBatchOutStride]
+  double* outs;       // [ncells][kBatchOutStride], host memory
   int ncells;
 };
 
@@ -109,8 +112,8 @@ cudaError_t launch_stage4_packed(const DevState& s, const StageParams& p, int wa
 cudaError_t launch_stage_mixed_packed(const DevState& s, const StageParams& p, int warps, cudaStream_t st);
 cudaError_t launch_avg(const DevState& s, cudaStream_t st);
 // reference-order (sequential) flux and output sums of the stored FRU states,
-// one thread; the flux launch overwrites out[0..8], the average one out[16..26]
-cudaError_t launch_flux_seq(const DevState& s, const StageParams& p, cudaStream_t st);
+// one thread; the flux launch overwrites res[0..4], the average one res[16..26]
+cudaError_t launch_flux_seq(const DevState& s, cudaStream_t st);
 cudaError_t launch_avg_seq(const DevState& s, cudaStream_t st);
 // FP64 FMA throughput of the device (TFLOP/s, best of a few launches).
 cudaError_t probe_fp64(int sms, double* tflops);

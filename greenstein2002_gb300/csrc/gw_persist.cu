@@ -16,7 +16,7 @@
 // forms each group's flux (and output-average) partial sums exactly as the
 // fixed-layout stage kernel does -- same lanes, same shuffle tree -- from
 // the stored FRUs.  The warp that stores the operation's last batch adds
-// the partials in the fixed order of cell_finish, forms the currents, runs
+// the partials in the fixed order of finish_groups, forms the currents, runs
 // the cell's integrator step on the whole warp (dp_after_warp: the
 // arithmetic of gw_dp.c, the 37-state vectors split over the lanes and
 // fcn's exponentials one per lane) and posts the cell's next operation.
@@ -68,7 +68,6 @@ constexpr unsigned long long kDefaultWaitNs = 2000000000ull;
 // the operation's parameters after the increment.
 struct PCell {
   unsigned long long take;  // next 8-FRU group of the open operation (>= ngroups: none)
-  unsigned done;            // groups of the open operation stored and summed
   unsigned overflow;        // an FRU of the operation reached the substep limit
   int finished;
 };
@@ -128,7 +127,6 @@ __device__ __forceinline__ int mask_pick(const unsigned long long* m, int nwords
 // Post the operation dp_after has just set up in the cell's DpCell (one thread).
 static __device__ void post(const Args& a, int ci) {
   PCell& pc = a.pc[ci];
-  pc.done = 0u;
   pc.overflow = 0u;
   __threadfence();
   atomicExch(&pc.take, 0ull);
@@ -136,22 +134,17 @@ static __device__ void post(const Args& a, int ci) {
   mask_set(a.open_mask, ci);
 }
 
-// The cell's totals from its group partials in cell_finish's order, the
-// currents, and the integrator step; then the next operation is posted (or
-// the cell is done).  Whole warp.
-template <int NV>
-__device__ __forceinline__ void finish_op(const Args& a, int ci, int lane) {
+// From the cell's totals (lane 0's v) the currents and the integrator step;
+// then the next operation is posted (or the cell is done).  Whole warp.
+__device__ __forceinline__ void unpack(const FluxSums& v, double tot[5]) { unpack_flux(v, tot); }
+__device__ __forceinline__ void unpack(const AvgSums& v, double tot[16]) { unpack_avg(v, tot); }
+template <int ND, int NI>
+__device__ __forceinline__ void finish_op(const Args& a, int ci, const Sums<ND, NI>& v, int lane) {
+  constexpr int NV = ND == 6 ? 16 : 5;
   const DevState& s = a.cells[ci];
   DpCell& c = a.dp[ci];
-  const int ngroups = ngroups_of(s);
-  __threadfence();
   double tot[NV];
-#pragma unroll
-  for (int k = 0; k < NV; k++) tot[k] = 0.0;
-  for (int b = lane; b < ngroups; b += 32)
-#pragma unroll
-    for (int k = 0; k < NV; k++) tot[k] += __ldcg(&s.partials[b * NV + k]);
-  cleft::warp_sum<NV>(tot);
+  unpack(v, tot);
 #pragma unroll
   for (int k = 0; k < NV; k++) tot[k] = __shfl_sync(kFull, tot[k], 0);
   PCell& pc = a.pc[ci];
@@ -180,43 +173,36 @@ __device__ __forceinline__ void finish_op(const Args& a, int ci, int lane) {
   __syncwarp();
 }
 
-// One 8-FRU group's partial sums into partials[grp * NV ..], by the whole
-// warp in the lanes of the fixed-layout kernel (FRU grp*8 + lane/4, cleft
-// lane%4), from the FRUs as stored: stage_body_fin's epilogue.
-template <int NV>
+// One 8-FRU group's partial sums, by the whole warp in the lanes of the
+// fixed-layout kernel (FRU grp*8 + lane/4, cleft lane%4), from the FRUs as
+// stored: stage_body_fin's epilogue.
+__device__ __forceinline__ void terms(int c, double jsr, double ss, uint32_t w, FluxSums& v) {
+  flux_terms(c, jsr, ss, w, v);
+}
+__device__ __forceinline__ void terms(int c, double jsr, double ss, uint32_t w, AvgSums& v) {
+  avg_terms(c, jsr, ss, w, v);
+}
+template <typename V>
 __device__ __forceinline__ void group_partials(const DevState& s, int grp, const cleft::Group& g, int lane) {
   const int f = grp * 8 + (lane >> 2);
-  const bool active = f < s.nfru;
   const size_t nf = (size_t)s.stride;
-  double cajsr = 0.0, cass = 0.0;
-  uint32_t w = 0u;
-  if (active) {
-    cajsr = s.frus[f];
-    cass = s.frus[(g.c + 1) * nf + f];
-    w = s.chan[g.c * nf + f];
-  }
-  double v[NV];
-#pragma unroll
-  for (int k = 0; k < NV; k++) v[k] = 0.0;
-  if (active) {
-    v[0] = cass;
-    v[1] = (g.c == 0) ? cajsr : 0.0;
-    if (lcc_open(w)) {
-      v[2] = cass;
-      v[3] = 1.0;
-    }
-    if (cl_of(w) == 2) v[4] = 1.0;
-  }
-  if (NV == 16) {
-    double t[11];
-    cleft::avg_terms(g.c, cajsr, cass, w, t);
-#pragma unroll
-    for (int k = 0; k < 11; k++) v[(5 + k) % NV] = active ? t[k] : 0.0;
-  }
-  cleft::warp_sum<NV>(v);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NV; k++) s.partials[grp * NV + k] = v[k];
+  V v = {};
+  if (f < s.nfru) terms(g.c, s.frus[f], s.frus[(g.c + 1) * nf + f], s.chan[g.c * nf + f], v);
+  store_group(s, grp, v, lane);
+}
+// The partial sums of a batch's groups, and their tickets (a batch may end a
+// chunk of groups and begin the next); the warp that completes the operation
+// finishes it.
+template <typename V>
+__device__ __forceinline__ void sum_batch(const Args& a, int ci, const DevState& s, int grp0, int ng,
+                                          const cleft::Group& g, int lane) {
+  for (int grp = grp0; grp < grp0 + ng; grp++) group_partials<V>(s, grp, g, lane);
+  if (lane == 0) atomicAdd(a.progress, 1ull);
+  const int next = min((grp0 | 31) + 1, grp0 + ng);  // the first chunk's groups end here
+  V v;
+  bool all = finish_groups(s, v, grp0 >> 5, (unsigned)(next - grp0), lane);
+  if (next < grp0 + ng) all = finish_groups(s, v, next >> 5, (unsigned)(grp0 + ng - next), lane);
+  if (all) finish_op(a, ci, v, lane);
 }
 
 // One batch of cell ci's open operation: groups [grp0, grp0 + ng).  The
@@ -229,7 +215,6 @@ __device__ __forceinline__ void run_batch(const Args& a, int ci, int grp0, int n
   const DevState& s = a.cells[ci];
   const StageParams& p = a.dp[ci].sp;
   const int n = s.nfru;
-  const int ngroups = ngroups_of(s);
   const int f_begin = grp0 * 8;
   const int f_end = min(n, (grp0 + ng) * 8);
   const size_t nf = (size_t)s.stride;
@@ -374,29 +359,13 @@ __device__ __forceinline__ void run_batch(const Args& a, int ci, int grp0, int n
     }
   }
   __syncwarp();  // the stores above are visible to the whole warp
-  const bool avg = (p.flags & kFlagAvg) != 0;
-  for (int grp = grp0; grp < grp0 + ng; grp++) {
-    if (avg) group_partials<16>(s, grp, g, lane);
-    else group_partials<5>(s, grp, g, lane);
-  }
   if (s.substeps) {
     for (int o = 16; o > 0; o >>= 1) nsub_sum += __shfl_down_sync(kFull, nsub_sum, o);
     if (lane == 0 && nsub_sum) atomicAdd(s.substeps, nsub_sum);
   }
-  PCell& pc = a.pc[ci];
-  if (__any_sync(kFull, overflow) && lane == 0) atomicOr(&pc.overflow, 1u);
-  __threadfence();
-  __syncwarp();
-  unsigned last = 0u;
-  if (lane == 0) {
-    last = (atomicAdd(&pc.done, (unsigned)ng) + (unsigned)ng == (unsigned)ngroups) ? 1u : 0u;
-    atomicAdd(a.progress, 1ull);
-  }
-  last = __shfl_sync(kFull, last, 0);
-  if (last) {
-    if (avg) finish_op<16>(a, ci, lane);
-    else finish_op<5>(a, ci, lane);
-  }
+  if (__any_sync(kFull, overflow) && lane == 0) atomicOr(&a.pc[ci].overflow, 1u);
+  if (p.flags & kFlagAvg) sum_batch<AvgSums>(a, ci, s, grp0, ng, g, lane);
+  else sum_batch<FluxSums>(a, ci, s, grp0, ng, g, lane);
 }
 
 template <typename R>
@@ -642,6 +611,9 @@ int run_persistent(int n, gw_ctx** cells, const gw_settings* sets, double* t, do
   if (e != cudaSuccess) {
     rc = gw_internal_error(GW_ECUDA, (std::string(who) + ": " + cudaGetErrorString(e)).c_str());
   } else if (hc[3] != gw::persist::kStatusOk) {
+    // operations may be half summed: their tickets start afresh
+    for (int i = 0; i < n; i++)
+      cudaMemset(cells[i]->d.ticket, 0, (1 + ((cells[i]->d.nfru + 7) / 8 + 31) / 32) * sizeof(unsigned));
     rc = gw_internal_error(GW_ECUDA, "gw_run_persistent: no progress within the wait limit (watchdog); the cells' "
                                      "state is that of an unfinished run");
   } else {
