@@ -3,7 +3,6 @@
 // / save / resume operations that replace the MPI layer of mpi_master.c.
 #include <cuda_runtime.h>
 #include <stdarg.h>
-#include <math.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -15,7 +14,6 @@
 #include "gw_diag.h"
 #include "gw_fru.h"
 #include "gw_kernels.h"
-#include "gw_fru_core.cuh"
 #include "gw_fru_model.cuh"
 #include "gw_ctx_impl.h"
 
@@ -103,10 +101,9 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   AL(d.mti_s, nf * sizeof(int));
   AL(d.mt_hold, nf * gw::kMtStride * sizeof(uint32_t));
   AL(d.hold_epoch, nf * sizeof(uint32_t));
-  // partial sums of the 8-FRU groups and of the chunks of 32 groups
-  const size_t ngroups = (size_t)(nfru + 7) / 8, nchunks = (ngroups + 31) / 32;
-  AL(d.partials, (ngroups + nchunks) * 16 * sizeof(double));
-  AL(d.ticket, (1 + nchunks) * sizeof(unsigned));
+  // partial sums of the 8-FRU groups
+  AL(d.partials, (size_t)((nfru + 7) / 8) * 16 * sizeof(double));
+  AL(d.ticket, sizeof(unsigned));
   AL(d.out, 32 * sizeof(double));
   AL(d.substeps, sizeof(unsigned long long));
   AL(d.qctl, 8 * sizeof(unsigned));
@@ -121,7 +118,7 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   }
   for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
   for (int i = 0; i < 2 && e == cudaSuccess; i++) e = cudaEventCreate(&c->pev[i]);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d.ticket, 0, (1 + nchunks) * sizeof(unsigned), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.ticket, 0, sizeof(unsigned), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.out, 0, 32 * sizeof(double), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.substeps, 0, sizeof(unsigned long long), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.hold_epoch, 0xff, nf * sizeof(uint32_t), c->stream);
@@ -367,7 +364,7 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
     CK(launch_stage_variant(c, p));
     c->launches++;
     if (c->sum_order == GW_SUM_REFERENCE) {
-      CK(gw::launch_flux_seq(c->d, c->stream));
+      CK(gw::launch_flux_seq(c->d, p, c->stream));
       c->launches++;
     }
     if (c->profiling) CK(cudaEventRecord(c->pev[1], c->stream));
@@ -386,11 +383,8 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
   }
   if (num)
     for (int k = 0; k < 5; k++) num[k] = c->h_out[k];
-  if (out) {
-    // mpi_master.c:447-468; on one GPU lane this algebra took 4 us of every launch
-    gw::currents_from_sums(c->d.nfru, c->nfru_scale, depf, c->h_out, out);
-    out[2] = out[2] * c->pca_scale;  // ICa is proportional to the LCC permeability
-  }
+  if (out)
+    for (int k = 0; k < 4; k++) out[k] = c->h_out[5 + k];
   return GW_OK;
 }
 

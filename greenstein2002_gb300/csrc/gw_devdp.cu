@@ -50,24 +50,6 @@ struct DpArgs {
 
 // FRU work of one round: every cell's requested launch, totals to its out[]
 // slots ([0..4] flux numerators, [5..8] currents, [16..26] averages).
-struct RoundFin {
-  const DevState& s;
-  const StageParams& p;
-  __device__ void operator()(const double tot[5], const double* avg) const {
-    double cur[4], *out = s.out;
-    currents_from_sums(s.nfru, p.nfru_scale, p.depf, tot, cur);
-    cur[2] = cur[2] * p.pca_scale;  // ICa is proportional to the LCC permeability
-#pragma unroll
-    for (int k = 0; k < 5; k++) out[k] = tot[k];
-#pragma unroll
-    for (int k = 0; k < 4; k++) out[5 + k] = cur[k];
-    if (avg)
-#pragma unroll
-      for (int k = 0; k < 11; k++) out[16 + k] = avg[k];
-  }
-  __device__ void error() const { s.out[kOutError] = 1.0; }
-};
-
 template <typename R>
 __global__ void __launch_bounds__(kMaxStageWarps * 32) dp_round_kernel(DpArgs a) {
   int lo = 0, hi = a.ncells - 1;
@@ -81,7 +63,7 @@ __global__ void __launch_bounds__(kMaxStageWarps * 32) dp_round_kernel(DpArgs a)
   if (c->done || c->err) return;  // uniform over the block (one cell per block)
   const DevState& s = a.cells[lo];
   const StageParams& p = c->sp;
-  cleft::stage_body_fin<R>(s, p, b - a.block0[lo], RoundFin{s, p});
+  cleft::stage_body<R>(s, p, b - a.block0[lo], s.out);
 }
 
 // The integrators of all cells, one thread each; the last block to finish

@@ -1261,22 +1261,23 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// Where a launch's cell totals go: OutFin writes the 5 flux numerators to the
-// launch's out[] slots (host memory, where the host forms the currents); the
-// device-resident integrators pass their own finishers.  Called by one lane,
-// with the flux numerators and, when the launch carried kFlagAvg, the 11
-// output-average sums (else null).
-struct OutFin {
-  double* out;
-  __device__ void operator()(const double tot[5], const double*) const {
+// Where a launch's cell totals go: the 5 flux numerators, the currents and,
+// when the launch carried kFlagAvg, the 11 output-average sums, to the
+// launch's out[] slots: host memory, or the device-resident integrator's.
+// Whole warp, with the totals in lane 0
+__device__ __forceinline__ void put_totals(const DevState& s, const StageParams& p, double* out, double tot[5], int lane) {
 #pragma unroll
-    for (int k = 0; k < 5; k++) out[k] = tot[k];
-  }
-  __device__ void error() const { out[kOutError] = 1.0; }
-};
+  for (int k = 0; k < 5; k++) tot[k] = __shfl_sync(0xffffffffu, tot[k], 0);
+  const double cur = lane_current(s, p, tot, lane);
+  double v = tot[0];
+#pragma unroll
+  for (int k = 1; k < 5; k++) v = (lane == 4 + k) ? tot[k] : v;
+  if (lane < 4) out[5 + lane] = cur;
+  else if (lane < 9) out[lane - 4] = v;
+}
 
-template <typename R, typename Fin>
-__device__ __forceinline__ void stage_body_fin(const DevState& s, const StageParams& p, int bidx, const Fin& fin) {
+template <typename R>
+__device__ __forceinline__ void stage_body(const DevState& s, const StageParams& p, int bidx, double* out) {
   const int lane = threadIdx.x & 31;
   const int grp = bidx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
   const int ngroups = (s.nfru + 7) >> 3;
@@ -1355,7 +1356,7 @@ __device__ __forceinline__ void stage_body_fin(const DevState& s, const StagePar
   }
   __syncwarp();
   if (s.trace_ns && lane == 0) s.trace_ns[2 * grp + 1] = global_ns();
-  if (overflow) fin.error();
+  if (overflow) out[kOutError] = 1.0;
   if (s.substeps) {
     unsigned c = __reduce_add_sync(0xffffffffu, (g.c == 0) ? nsub : 0u);
     if (lane == 0 && c) atomicAdd(s.substeps, (unsigned long long)c);
@@ -1364,26 +1365,24 @@ __device__ __forceinline__ void stage_body_fin(const DevState& s, const StagePar
     AvgSums v = {};
     if (active) avg_terms(g.c, cajsr, cass, w, v);
     store_group(s, grp, v, lane);
-    if (finish_groups(s, v, grp >> 5, 1u, lane) && lane == 0) {
+    if (finish_groups(s, v, 1u, lane)) {
       double tot[16];
       unpack_avg(v, tot);
-      fin(tot, tot + 5);
+      put_totals(s, p, out, tot, lane);
+      if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 11; k++) out[16 + k] = tot[5 + k];
     }
     return;
   }
   FluxSums v = {};
   if (active) flux_terms(g.c, cajsr, cass, w, v);
   store_group(s, grp, v, lane);
-  if (finish_groups(s, v, grp >> 5, 1u, lane) && lane == 0) {
+  if (finish_groups(s, v, 1u, lane)) {
     double tot[5];
     unpack_flux(v, tot);
-    fin(tot, nullptr);
+    put_totals(s, p, out, tot, lane);
   }
-}
-
-template <typename R>
-__device__ __forceinline__ void stage_body(const DevState& s, const StageParams& p, int bidx, double* out) {
-  stage_body_fin<R>(s, p, bidx, OutFin{out});
 }
 
 // ---- packed stage: a queue of FRUs per 4-lane group -----------------------------

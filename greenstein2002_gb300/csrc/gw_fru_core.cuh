@@ -128,7 +128,7 @@ __device__ __forceinline__ void warp_sum(Sums<ND, NI>& v) {
     for (int k = 0; k < NI; k++) v.n[k] += __shfl_down_sync(0xffffffffu, v.n[k], o);
   }
 }
-// Partial sums of slot i (a group, or past the groups a chunk) in partials.
+// Partial sums of group i.
 template <int ND, int NI>
 __device__ __forceinline__ void put_partial(const DevState& s, int i, const Sums<ND, NI>& v) {
   double* q = s.partials + (size_t)i * (ND + NI);
@@ -152,58 +152,41 @@ __device__ __forceinline__ void store_group(const DevState& s, int grp, Sums<ND,
   if (lane == 0) put_partial(s, grp, v);
 }
 
-// Cross-FRU sums of one cell, independent of the launch shape: groups of 8
-// FRUs are summed by chunks of 32 (one group per lane, a shuffle tree), the
-// chunks lane-strided and by one more tree.  The warp that completes a chunk
-// sums it and the one that completes the last chunk the cell, both told by
-// tickets (ticket[1 + chunk] counts groups, ticket[0] chunks; each is reset by
-// the warp that completes it).  Summing all groups in the cell's last warp
-// instead kept that one warp at 5 dependent FP64 additions per 32 groups:
-// the flux launch of a 12,500-FRU cell took 30 us, against 15 us now (with the
-// counts as integers and the current algebra on the host).
-// Called by a warp that has stored `count` groups of `chunk`; true (in every
-// lane) when that completed the cell, with the totals in lane 0's v.
+// Cross-FRU sums of one cell, independent of the launch shape: the warp that
+// stores the cell's last group adds the groups lane-strided (groups lane,
+// lane + 32, ... one after another) and by one warp tree.  Three dependent
+// FP64 additions per 32 groups: the counts are integers (as doubles they made
+// it five).
+// Called by a warp that has stored `count` groups; true (in every lane) when
+// that completed the cell, with the totals in lane 0's v.  The ticket counts
+// groups and is reset by the warp that completes the cell.
 template <int ND, int NI>
-__device__ __forceinline__ bool finish_groups(const DevState& s, Sums<ND, NI>& v, int chunk, unsigned count, int lane) {
-  const int ngroups = (s.nfru + 7) >> 3, nchunks = (ngroups + 31) >> 5;
-  const int size = min(32, ngroups - 32 * chunk);
+__device__ __forceinline__ bool finish_groups(const DevState& s, Sums<ND, NI>& v, unsigned count, int lane) {
+  const int ngroups = (s.nfru + 7) >> 3;
   unsigned last = 0u;
   if (lane == 0) {
     __threadfence();
-    last = (atomicAdd(&s.ticket[1 + chunk], count) + count == (unsigned)size) ? 1u : 0u;
+    last = (atomicAdd(s.ticket, count) + count == (unsigned)ngroups) ? 1u : 0u;
   }
   if (!__shfl_sync(0xffffffffu, last, 0)) return false;
   __threadfence();
   v = {};
-  if (lane < size) get_partial(s, 32 * chunk + lane, v);
-  warp_sum(v);
-  if (lane == 0) s.ticket[1 + chunk] = 0u;
-  if (nchunks == 1) return true;
-  last = 0u;
-  if (lane == 0) {
-    put_partial(s, ngroups + chunk, v);
-    __threadfence();
-    last = (atomicAdd(&s.ticket[0], 1u) == (unsigned)nchunks - 1u) ? 1u : 0u;
-  }
-  if (!__shfl_sync(0xffffffffu, last, 0)) return false;
-  __threadfence();
-  v = {};
-  for (int b = lane; b < nchunks; b += 32) {
+#pragma unroll 8
+  for (int b = lane; b < ngroups; b += 32) {
     Sums<ND, NI> t;
-    get_partial(s, ngroups + b, t);
+    get_partial(s, b, t);
 #pragma unroll
     for (int k = 0; k < ND; k++) v.d[k] += t.d[k];
 #pragma unroll
     for (int k = 0; k < NI; k++) v.n[k] += t.n[k];
   }
   warp_sum(v);
-  if (lane == 0) s.ticket[0] = 0u;
+  if (lane == 0) *s.ticket = 0u;
   return true;
 }
 
 // Flux numerators -> (Jxfer, Jtr, ICa, Ito2): mpi_master.c:447-468.
-// Host code uses the host libm's exp, device code CUDA's.
-static __host__ __device__ inline void currents_from_sums(int nfru, double scale, const double dep[3], const double num[5], double out[4]) {
+static __device__ inline void currents_from_sums(int nfru, double scale, const double dep[3], const double num[5], double out[4]) {
   const double V = dep[0], Cai = dep[1], CaNSR = dep[2];
   const double VFRT = V / RT_over_F, VFsqRT = (1000.0 * Faraday) * VFRT;
   const double e1 = exp(VFRT), e2 = e1 * e1;
@@ -227,6 +210,47 @@ static __host__ __device__ inline void currents_from_sums(int nfru, double scale
   out[1] = scale * jtr;
   out[2] = scale * ica;
   out[3] = scale * ito2;
+}
+
+// The currents of a launch's totals, one per lane: on return lanes 0..3 hold
+// Jxfer, Jtr, ICa, Ito2 in cur.  num: the flux numerators, the same in every
+// lane.  One instruction stream for the four (36 FP64 instructions; on one
+// lane one after another about 120, 4 us of every launch): a product and a
+// difference, two quotients and the scale, the operands selected by lane.
+// GW_CONTRACT (the mixed-precision unit): products feeding a difference are
+// fused, as the compiler fuses currents_from_sums there.
+__device__ __forceinline__ double lane_current(const DevState& s, const StageParams& p, const double num[5], int lane) {
+  const double V = p.depf[0];
+  const long long av = __double_as_longlong(V) & 0x7fffffffffffffffLL;
+  if (av < __double_as_longlong(1.e-6) || av >= __double_as_longlong(500.0)) {
+    double cur[4];
+    currents_from_sums(s.nfru, p.nfru_scale, p.depf, num, cur);
+    const double c = lane == 0 ? cur[0] : lane == 1 ? cur[1] : lane == 2 ? cur[2] * p.pca_scale : cur[3];
+    return c;
+  }
+  const double VFRT = const_div(V, kDivRTF), VFsqRT = (1000.0 * Faraday) * VFRT;
+  const double e1 = exp(VFRT), e2 = e1 * e1;
+  const double n = (double)s.nfru;
+  const double c = num[3] * Cao;
+  // x * y, subtracted from or less the other operand z (lane 2: z = (num3 Cao) 0.341)
+  const double x = lane == 0 ? n * (double)kClefts : lane == 1 ? n : lane == 2 ? num[2] : Clo;
+  const double y = lane == 0 ? p.depf[1] : lane == 1 ? p.depf[2] : lane == 2 ? e2 : e1;
+  const double z = lane == 0 ? num[0] : lane == 1 ? num[1] : lane == 2 ? c * 0.341 : Cli;
+  const bool minus = lane == 0 || lane == 3;  // z - x y, else x y - z
+#ifdef GW_CONTRACT
+  double b = fma(minus ? -x : x, y, minus ? z : -z);
+#else
+  const double xy = x * y;
+  double b = (minus ? z : xy) - (minus ? xy : z);
+#endif
+  const double a = (lane == 2 ? PCa * 4.0 : num[4] * PCl) * VFsqRT;
+  const double ab = a * b;
+  b = lane >= 2 ? ab : b;
+  const double em1 = (lane == 2 ? e2 : 1.0) - (lane == 2 ? 1.0 : e1);
+  const double q = fast_div(b, lane == 0 ? tauxfer : lane == 1 ? tautr : em1);
+  const double r = fast_div(q, Acap);
+  const double cur = p.nfru_scale * (lane >= 2 ? r : q);
+  return lane == 2 ? cur * p.pca_scale : cur;  // ICa is proportional to the LCC permeability
 }
 
 // Categorical selection of simfru_local.c:217-226 for a channel that has left

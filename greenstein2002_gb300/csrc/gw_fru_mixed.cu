@@ -5,6 +5,7 @@
 // the FP64 method's (gw_fru_cleft.cuh), so both share every random number.
 //
 // Reference: simfru_local.c:32-278, fru_rates_local.c:30-798, fcn_fru.c:23-137.
+#define GW_CONTRACT
 #include "gw_fru_cleft.cuh"
 
 namespace gw {

@@ -106,11 +106,14 @@ __global__ void __launch_bounds__(kStageThreads) fru_stage_kernel(DevState s, St
   const int mine = min(4, ngroups - grp0);  // groups of this warp that hold FRUs
   if ((lane & 7) == 0 && (lane >> 3) < mine) put_partial(s, grp0 + (lane >> 3), v);
   __syncwarp();
-  if (finish_groups(s, v, grp0 >> 5, (unsigned)mine, lane) && lane == 0) {
-    double tot[5];
+  if (finish_groups(s, v, (unsigned)mine, lane) && lane == 0) {
+    double tot[5], cur[4];
     unpack_flux(v, tot);
+    currents_from_sums(s.nfru, p.nfru_scale, p.depf, tot, cur);
 #pragma unroll
     for (int k = 0; k < 5; k++) s.res[k] = tot[k];
+#pragma unroll
+    for (int k = 0; k < 4; k++) s.res[5 + k] = cur[k];
   }
 }
 
@@ -157,16 +160,17 @@ __global__ void __launch_bounds__(kStageThreads) fru_avg_kernel(DevState s) {
 
 // Reference-order sums (the parity mode of gw_set_sum_order): the flux
 // numerators added one FRU and one cleft after another, as
-// calc_fru_flux_local.c:44-70 does.  A sequential FP64 sum has exactly one rounding
+// calc_fru_flux_local.c:44-70 does, then the currents of
+// mpi_master.c:447-468.  A sequential FP64 sum has exactly one rounding
 // order, so each sum is one thread's dependent chain; the block stages the
 // stored FRU states in shared memory in coalesced chunks and three warps (on
 // three SM sub-partitions) run the three chains side by side: the CaSS sum,
 // the CaJSR sum, and the open-LCC CaSS sum with the two counts (integers,
 // exact).  About 4 dependent FP64 additions per FRU, so this mode is for
 // parity runs of small cells.  Runs after the stage launch and overwrites
-// res[0..4].
+// res[0..8].
 constexpr int kSeqThreads = 128, kSeqChunk = 512;
-__global__ void __launch_bounds__(kSeqThreads) fru_flux_seq_kernel(DevState s) {
+__global__ void __launch_bounds__(kSeqThreads) fru_flux_seq_kernel(DevState s, StageParams p) {
   __shared__ double sf[5][kSeqChunk];
   __shared__ uint32_t sw[kClefts][kSeqChunk];
   __shared__ double res[5];
@@ -209,8 +213,14 @@ __global__ void __launch_bounds__(kSeqThreads) fru_flux_seq_kernel(DevState s) {
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    const double tot[5] = {res[0], res[1], res[2], res[3], res[4]};
+    double cur[4];
+    currents_from_sums(s.nfru, p.nfru_scale, p.depf, tot, cur);
+    cur[2] = cur[2] * p.pca_scale;
 #pragma unroll
-    for (int k = 0; k < 5; k++) s.res[k] = res[k];
+    for (int k = 0; k < 5; k++) s.res[k] = tot[k];
+#pragma unroll
+    for (int k = 0; k < 4; k++) s.res[5 + k] = cur[k];
   }
 }
 
@@ -294,8 +304,8 @@ cudaError_t launch_avg(const DevState& s, cudaStream_t st) {
   fru_avg_kernel<<<s.nblocks, kStageThreads, 0, st>>>(s);
   return cudaGetLastError();
 }
-cudaError_t launch_flux_seq(const DevState& s, cudaStream_t st) {
-  fru_flux_seq_kernel<<<1, kSeqThreads, 0, st>>>(s);
+cudaError_t launch_flux_seq(const DevState& s, const StageParams& p, cudaStream_t st) {
+  fru_flux_seq_kernel<<<1, kSeqThreads, 0, st>>>(s, p);
   return cudaGetLastError();
 }
 cudaError_t launch_avg_seq(const DevState& s, cudaStream_t st) {

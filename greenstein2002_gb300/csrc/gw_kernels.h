@@ -38,12 +38,12 @@ enum : int { kSeedBase = 0, kSeedReference = 1 };
 //   mti[stride], mt[nfru][640] (FRU-major MT19937 rows)
 //   *_s               snapshot taken at the last save
 //   mt_hold/hold_epoch  copy-on-twist protection of the saved MT words
-//   partials[groups + chunks][16], ticket[1 + chunks]: scratch of the
-//                     deterministic reductions (groups of 8 FRUs, chunks of 32 groups)
+//   partials[groups][16], ticket: scratch of the deterministic reductions
+//                     over the groups of 8 FRUs
 //   res[32]           results the host reads, in its own (pinned, mapped) memory:
-//                     [0..4] flux sums, [16..26] averages, [31] error flag
-//   out[32]           the same of the round-based device integrator, in device
-//                     memory, with [5..8] Jxfer,Jtr,ICa,Ito2
+//                     [0..4] flux sums, [5..8] Jxfer,Jtr,ICa,Ito2, [16..26] averages,
+//                     [31] error flag
+//   out[32]           the same of the round-based device integrator, in device memory
 struct DevState {
   int nfru, stride, nblocks;
   double* frus;
@@ -112,8 +112,8 @@ cudaError_t launch_stage4_packed(const DevState& s, const StageParams& p, int wa
 cudaError_t launch_stage_mixed_packed(const DevState& s, const StageParams& p, int warps, cudaStream_t st);
 cudaError_t launch_avg(const DevState& s, cudaStream_t st);
 // reference-order (sequential) flux and output sums of the stored FRU states,
-// one thread; the flux launch overwrites res[0..4], the average one res[16..26]
-cudaError_t launch_flux_seq(const DevState& s, cudaStream_t st);
+// one thread; the flux launch overwrites res[0..8], the average one res[16..26]
+cudaError_t launch_flux_seq(const DevState& s, const StageParams& p, cudaStream_t st);
 cudaError_t launch_avg_seq(const DevState& s, cudaStream_t st);
 // FP64 FMA throughput of the device (TFLOP/s, best of a few launches).
 cudaError_t probe_fp64(int sms, double* tflops);

@@ -148,9 +148,10 @@ __device__ __forceinline__ void finish_op(const Args& a, int ci, const Sums<ND, 
 #pragma unroll
   for (int k = 0; k < NV; k++) tot[k] = __shfl_sync(kFull, tot[k], 0);
   PCell& pc = a.pc[ci];
+  const double mine = lane_current(s, c.sp, tot, lane);
   double cur[4];
-  currents_from_sums(s.nfru, c.sp.nfru_scale, c.sp.depf, tot, cur);
-  cur[2] = cur[2] * c.sp.pca_scale;  // ICa is proportional to the LCC permeability
+#pragma unroll
+  for (int k = 0; k < 4; k++) cur[k] = __shfl_sync(kFull, mine, k);
   const bool ovf = vload(&pc.overflow) != 0u;
   __syncwarp();
   if (ovf) {
@@ -190,19 +191,15 @@ __device__ __forceinline__ void group_partials(const DevState& s, int grp, const
   if (f < s.nfru) terms(g.c, s.frus[f], s.frus[(g.c + 1) * nf + f], s.chan[g.c * nf + f], v);
   store_group(s, grp, v, lane);
 }
-// The partial sums of a batch's groups, and their tickets (a batch may end a
-// chunk of groups and begin the next); the warp that completes the operation
-// finishes it.
+// The partial sums of a batch's groups; the warp that stores the operation's
+// last group finishes it.
 template <typename V>
 __device__ __forceinline__ void sum_batch(const Args& a, int ci, const DevState& s, int grp0, int ng,
                                           const cleft::Group& g, int lane) {
   for (int grp = grp0; grp < grp0 + ng; grp++) group_partials<V>(s, grp, g, lane);
   if (lane == 0) atomicAdd(a.progress, 1ull);
-  const int next = min((grp0 | 31) + 1, grp0 + ng);  // the first chunk's groups end here
   V v;
-  bool all = finish_groups(s, v, grp0 >> 5, (unsigned)(next - grp0), lane);
-  if (next < grp0 + ng) all = finish_groups(s, v, next >> 5, (unsigned)(grp0 + ng - next), lane);
-  if (all) finish_op(a, ci, v, lane);
+  if (finish_groups(s, v, (unsigned)ng, lane)) finish_op(a, ci, v, lane);
 }
 
 // One batch of cell ci's open operation: groups [grp0, grp0 + ng).  The
@@ -612,8 +609,7 @@ int run_persistent(int n, gw_ctx** cells, const gw_settings* sets, double* t, do
     rc = gw_internal_error(GW_ECUDA, (std::string(who) + ": " + cudaGetErrorString(e)).c_str());
   } else if (hc[3] != gw::persist::kStatusOk) {
     // operations may be half summed: their tickets start afresh
-    for (int i = 0; i < n; i++)
-      cudaMemset(cells[i]->d.ticket, 0, (1 + ((cells[i]->d.nfru + 7) / 8 + 31) / 32) * sizeof(unsigned));
+    for (int i = 0; i < n; i++) cudaMemset(cells[i]->d.ticket, 0, sizeof(unsigned));
     rc = gw_internal_error(GW_ECUDA, "gw_run_persistent: no progress within the wait limit (watchdog); the cells' "
                                      "state is that of an unfinished run");
   } else {
