@@ -12,15 +12,15 @@
 // instructions (what bounds the kernels, see gw_fp64_math.cuh):
 //   - quotients, reciprocals and exponentials from gw_fp64_math.cuh;
 //   - max/min/compares of non-negative doubles on their bit patterns;
-//   - the products of an LCC's exit row are kept and reused when it leaves;
-//     the RyR rates are formed per state present in the cleft, not per RyR;
-//   - a draw is first compared in FP32 with an upper bound of dt*rate; only
-//     channels that may leave form 1 - dt*rate, which is compared with the
-//     draw in the integer domain (u = y/2^32 > P  <=>  y > floor(P*2^32));
+//   - rates are estimated in FP32 and formed in FP64 only where the estimate
+//     leaves a decision open: which rate is the largest (when 0.1 over it is
+//     below the substep's cap) and which side of its threshold a draw is on;
+//     there 1 - dt*rate is compared with the draw in the integer domain
+//     (u = y/2^32 > P  <=>  y > floor(P*2^32));
 //   - products with 0/1 flags are selections, halvings are folded into FMAs
-//     (both exact), the three interpolated voltages/concentrations and the
-//     four voltage exponentials are computed one per lane, and
-//     exp(2VF/RT) at the end of a substep is reused at the start of the
+//     (both exact), the three interpolated voltages/concentrations are
+//     computed one per lane, and exp(2VF/RT) at the end of a substep is reused
+//     at the start of the
 //     next (and at the stage start computed once per lane, not per FRU).
 // R = float: the mixed-precision method.  Transition rates, the local Ca ODE
 // and the FRU clock are evaluated in FP32, the Ca states and the clock
@@ -483,9 +483,11 @@ __device__ __forceinline__ void lane_stage(const StageParams& p, const Group& g,
 // range the hardware's division).
 __device__ __forceinline__ void ghk_terms(double V, double pca4, double& e2, double& a2j, bool& small) {
   constexpr double JDHconstant = 1.0 / (2.0 * VSS * Faraday * 1000.0);
-  const double VFRT = const_div(V, kDivRTF);
-  const double VFsqRT = (1000.0 * Faraday) * VFRT;
-  e2 = fexp(2.0 * VFRT);
+  // 2VF/RT is V over half the divisor and 1000 F VF/RT half of 1000 F times
+  // it: exact scalings by two of the reference's products
+  const double VF2 = fma(V, 2.0 * kDivRTF.rhi, V * (2.0 * kDivRTF.rlo));
+  const double VFsqRT = (500.0 * Faraday) * VF2;
+  e2 = fexp(VF2);
   small = abs_lt(V, 1.e-6);
   a2j = 0.0;
   if (!small) {
@@ -501,8 +503,7 @@ struct LaneStage<double> {
   double t0, tf, interval, rhi, rlo;  // rhi + rlo = 1/interval to about 105 bits
   double e2, a2j;                  // ghk_terms at t0
   bool small, isdiv, tpos;         // tpos: times are >= 0 (and tf is not NaN)
-  double cA, cCF, cK, cM;          // per-lane voltage exponential (see LaneStage<R>)
-  ConstDiv cR;                     // as a factor (rhi; lanes 0, 1) or a divisor (lanes 2, 3)
+  float cA, cR, cCF, cK, cM;       // per-lane voltage exponential in FP32 (see LaneStage<R>)
 };
 __device__ __forceinline__ void lane_stage(const StageParams& p, const Group& g, LaneStage<double>& L) {
 #pragma unroll
@@ -519,12 +520,11 @@ __device__ __forceinline__ void lane_stage(const StageParams& p, const Group& g,
   L.rlo = fma(-L.interval, L.rhi, 1.0) * L.rhi;
   ghk_terms(L.dep0[0], L.pca4, L.e2, L.a2j, L.small);
   L.isdiv = g.c >= 2;
-  L.cA = L.isdiv ? (g.c == 2 ? 12.5 : 30.0) : -35.0;
-  L.cR.rhi = L.isdiv ? (g.c == 2 ? kDiv5.rhi : kDiv12.rhi) : (g.c == 0 ? 0.012 : -0.05);
-  L.cR.rlo = L.isdiv ? (g.c == 2 ? kDiv5.rlo : kDiv12.rlo) : 0.0;
-  L.cCF = g.c == 0 ? alphacf : betacf;
-  L.cK = g.c == 2 ? 0.4 : 340.0;
-  L.cM = g.c == 2 ? 1.0 - 0.4 : 60.0;
+  L.cA = L.isdiv ? (g.c == 2 ? 12.5f : 30.0f) : -35.0f;
+  L.cR = L.isdiv ? (g.c == 2 ? 1.0f / 5.0f : 1.0f / 12.0f) : (g.c == 0 ? 0.012f : -0.05f);
+  L.cCF = g.c == 0 ? (float)alphacf : (float)betacf;
+  L.cK = g.c == 2 ? 0.4f : 340.0f;
+  L.cM = g.c == 2 ? 0.6f : 60.0f;
 }
 
 // Accumulator of an FRU Ca concentration over the substeps.  FP64: a double,
@@ -852,7 +852,10 @@ struct Fru4<double> {
 };
 template <>
 struct Sub4<double> {
-  double cajsr, cass, X, Y, Z, Rl, Rv, k12, sat;  // LCC exit products and total, VDI rate, RyR k12 and saturation
+  double cajsr, cass;
+  float X, Y, Z, Rl, Rv, sat, sat2;  // FP32 estimates: LCC exit rates and total, VDI rate, RyR saturations
+  uint32_t code;                     // the LCC state's row (LccRow64)
+  bool ok;                           // the estimates hold (concentrations and potential in range)
   int regime, ne, pre, etot;
   uint32_t exmask;  // RyRs that draw an extra uniform (bit 0 of their nibbles)
   uint32_t exw[kRyR], bw[8];
@@ -921,6 +924,80 @@ static __device__ const LccRow64 g_lcc_row64[13] = {
     {gLprime, 0.0, 0.0, lcc_code(0x000, 2, 11, 0, 0, 0), 0},                      // 12
 };
 
+// The same coefficients in FP32.
+struct __align__(16) LccRow32 {
+  float x, y, z;
+  uint32_t code;
+};
+#define GW_ROW32(x, y, z, code) {(float)(x), (float)(y), (float)(z), code}
+static __device__ const LccRow32 g_lcc_row32[13] = {
+    GW_ROW32(0.0, 0.0, 0.0, lcc_code(0x000, 1, 0, 0, 0, 0)),
+    GW_ROW32(4.0, 1.0, 0.0, lcc_code(0x031, 3, 2, 7, 0, 0)),
+    GW_ROW32(1.0, 3.0, aL, lcc_code(0x312, 4, 1, 3, 8, 0)),
+    GW_ROW32(2.0, 2.0, aL * aL, lcc_code(0x312, 4, 2, 4, 9, 0)),
+    GW_ROW32(3.0, 1.0, aL * aL * aL, lcc_code(0x312, 4, 3, 5, 10, 0)),
+    GW_ROW32(4.0, fL, aL * aL * aL * aL, lcc_code(0x302, 4, 4, 6, 11, 0)),
+    GW_ROW32(gL, 0.0, 0.0, lcc_code(0x000, 2, 5, 0, 0, 0)),
+    GW_ROW32(4.0 * aL, CCa0_to_C0, 0.0, lcc_code(0x001, 3, 1, 8, 0, 1)),
+    GW_ROW32(1.0, 3.0 * aL, CCa1_to_C1, lcc_code(0x015, 4, 7, 2, 9, 2)),
+    GW_ROW32(2.0, 2.0 * aL, CCa2_to_C2, lcc_code(0x015, 4, 8, 3, 10, 2)),
+    GW_ROW32(3.0, aL, CCa3_to_C3, lcc_code(0x015, 4, 9, 4, 11, 2)),
+    GW_ROW32(4.0, CCa4_to_C4, fLprime, lcc_code(0x005, 4, 10, 5, 12, 0)),
+    GW_ROW32(gLprime, 0.0, 0.0, lcc_code(0x000, 2, 11, 0, 0, 0)),
+};
+#undef GW_ROW32
+
+// ---- exact rates and transitions, for what the FP32 estimates leave open -------
+// LCC exit products X, Y, Z of the reference's total X + Y + Z.
+__device__ __forceinline__ void lcc_exact(uint32_t w, double alpha, double beta, double cass, double& X, double& Y,
+                                          double& Z) {
+  const LccRow64* row = &g_lcc_row64[lcc_of(w)];
+  const double2 xy = __ldg(reinterpret_cast<const double2*>(row));
+  const double z = __ldg(&row->z);
+  const uint32_t code = __ldg(&row->code);
+  const int bx = code & 15u, by = (code >> 4) & 15u, bz = (code >> 8) & 15u;
+  const double gam = gammacf * cass;
+  double v = (bx == 1) ? alpha : 1.0;
+  v = (bx == 2) ? beta : v;
+  v = (bx == 5) ? const_div(beta, kDivBL) : v;  // / (bL * kappa)
+  X = xy.x * v;
+  v = (by == 1) ? alpha : 1.0;
+  v = (by == 3) ? gam : v;
+  Y = xy.y * v;
+  v = (bz == 3) ? gam : 1.0;
+  Z = z * v;
+}
+static __device__ __noinline__ double vdi_rate_exact(uint32_t w, double V) {
+  const double yinf = 0.4 / (1.0 + fexp(const_div(V + 12.5, kDiv5))) + (1.0 - 0.4);
+  const double tau = 60.0 + 340.0 / (1.0 + fexp(const_div(V + 30.0, kDiv12)));
+  return ((vdi_of(w) == 2) ? 1.0 - yinf : yinf) / tau;
+}
+__device__ __forceinline__ double sat_exact(double cass) { return imin(threshMAX, const_div(cass * cass, kDivKrate)); }
+// Exit total of RyR state s and the first two rates of its row, its length
+// and destinations (fru_rates_local.c:374-736).
+static __device__ __noinline__ double ryr_total_exact(int s, double cass, int regime, double& r1, double& r2, int& len,
+                                               uint32_t& d) {
+  const uint32_t to5 = (regime == 0) ? 5u : 8u, to7 = (regime == 2) ? 7u : 3u;
+  const double sat = sat_exact(cass);
+  r1 = r2 = 0.0;
+  len = 2;
+  switch (s) {
+    case 1: d = 2u; return k12cf * imin(threshMAX, const_div(cass * cass, kDivKrate2));
+    case 2: r1 = k21; r2 = k23cf * sat; len = 4; d = 1u | (to7 << 4) | (to5 << 8); return k21 + r2 + k25cf * sat;
+    case 3: r1 = k32; len = 3; d = 0x42u; return k32 + k34cf * sat;
+    case 4: r1 = k43; len = 3; d = 3u | (to5 << 4); return k43 + k45;
+    case 5: r1 = k52; r2 = k54cf * sat; len = 4; d = 0x642u; return k52 + r2 + k56cf * sat;
+    case 6: d = 5u; return k65;
+    case 7: {
+      const double k34 = k34cf * sat, a1 = fast_div(k34, k34 + k43);
+      r1 = (1.0 - a1) * k32; len = 3; d = 0x82u; return r1 + a1 * k45;
+    }
+    default: {
+      const double a1 = fast_div(k65, k56cf * sat + k65);
+      r1 = a1 * k52; len = 3; d = (regime == 2) ? 0x72u : 0x42u; return r1 + a1 * (k54cf * sat);
+    }
+  }
+}
 // Destination of a channel that leaves its state (simfru_local.c:215-253):
 // the cumulative walk from P = 1 - dt*total over the row r1, r2, (r3), the
 // draw compared with each sum in the integer domain.  d holds d1, d2, d3 in
@@ -935,66 +1012,40 @@ __device__ __forceinline__ uint32_t walk(uint32_t y, double P, double dt, double
   }
   return d & 15u;
 }
-
-// a value's leading 20 mantissa bits as FP32, for the upper bounds below
-__device__ __forceinline__ float head32(double x) {
-  return __uint_as_float((uint32_t)__double2hiint(x) * 8u + 0x40000000u);
+// The transitions of one cleft's 8 channels (simfru_local.c:215-276): every
+// rate and probability in FP64, the draws compared in the integer domain.
+static __device__ __noinline__ uint32_t transitions_exact(uint32_t w, double V, double cass, double dt, int regime, uint4 ya,
+                                                   uint4 yb) {
+  const uint32_t y[8] = {ya.x, ya.y, ya.z, ya.w, yb.x, yb.y, yb.z, yb.w};
+  {
+    const double alpha = alphacf * fexp(0.012 * (V - 35.0)), beta = betacf * fexp(-0.05 * (V - 35.0));
+    double X, Y, Z;
+    lcc_exact(w, alpha, beta, cass, X, Y, Z);
+    const double P = 1.0 - dt * (X + Y + Z);
+    if (u_above(y[0], P)) {
+      const uint32_t code = g_lcc_row64[lcc_of(w)].code, perm = code >> 28;
+      const double r1 = (perm == 1) ? Y : X, r2 = (perm == 2) ? Z : (perm == 1) ? X : Y;
+      w = set_field(w, 0, (int)walk(y[0], P, dt, r1, r2, (int)((code >> 12) & 15u), code >> 16));
+    }
+  }
+  if (u_reaches(y[1], 1.0 - dt * vdi_rate_exact(w, V))) w = set_field(w, 4, 3 - vdi_of(w));
+#pragma unroll
+  for (int i = 0; i < kRyR; i++) {
+    double r1, r2;
+    int len;
+    uint32_t d;
+    const double P = 1.0 - dt * ryr_total_exact(ryr_of(w, i), cass, regime, r1, r2, len, d);
+    if (u_above(y[2 + i], P)) w = set_field(w, 8 + 4 * i, (int)walk(y[2 + i], P, dt, r1, r2, len, d));
+  }
+  if (u_reaches(y[7], 1.0 - dt * ((cl_of(w) == 1) ? kfIto2 * cass : kbIto2))) w = set_field(w, 28, 3 - cl_of(w));
+  return w;
 }
 
-// First half of one FP64 substep (simfru_local.c:83-146 up to the draws):
-// the layout of the extra draws and the words that precede word 624 first
-// (their loads overlap the rest), then the voltage terms and exit totals.
-__device__ __forceinline__ void substep_a(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const Group& g,
-                                          const StageCtx& sc) {
-  const uint32_t w = F.w;
-  const double cass = F.ss.v;
-  S.cajsr = F.jsr.v;
-  S.cass = cass;
-  {
-    const double cc = imin(cass, threshMAXCa);
-    S.regime = ilt(cc, threshCa56to8) ? 0 : (ilt(cc, threshCa34to7) ? 1 : 2);
-  }
-  draw_layout(g, w, S.regime, S.exmask, S.ne, S.pre, S.etot);
-  fetch_old(sc, g, F.mti, S.pre, S.ne, S.etot, S.exw, S.bw);
-  // ---- voltage terms at the substep start, one exponential per lane ----
-  const double V = F.dep[0];
-  const double x = V + L.cA;
-  const double ev = fexp(L.isdiv ? const_div(x, L.cR) : x * L.cR.rhi);
-  double vterm;
-  if (L.isdiv) {
-    const double den = 1.0 + ev;
-    vterm = (abs_lt(V, 500.0) ? fast_div(L.cK, den) : L.cK / den) + L.cM;
-  } else {
-    vterm = L.cCF * ev;
-  }
-  const double alpha = from(g, vterm, 0), beta = from(g, vterm, 1);
-  const double yinf = from(g, vterm, 2), tau = from(g, vterm, 3);
-  const double bp = const_div(beta, kDivBL);  // / (bL * kappa)
-  const double gam = gammacf * cass;
-  {
-    const LccRow64* row = &g_lcc_row64[lcc_of(w)];
-    const double2 xy = __ldg(reinterpret_cast<const double2*>(row));
-    const double z = __ldg(&row->z);
-    const uint32_t code = __ldg(&row->code);
-    const int bx = code & 15u, by = (code >> 4) & 15u, bz = (code >> 8) & 15u;
-    double v = (bx == 1) ? alpha : 1.0;
-    v = (bx == 2) ? beta : v;
-    v = (bx == 5) ? bp : v;
-    S.X = xy.x * v;
-    v = (by == 1) ? alpha : 1.0;
-    v = (by == 3) ? gam : v;
-    S.Y = xy.y * v;
-    v = (bz == 3) ? gam : 1.0;
-    S.Z = z * v;
-    S.Rl = S.X + S.Y + S.Z;
-  }
-  {
-    const double num = (vdi_of(w) == 2) ? (1.0 - yinf) : yinf;
-    S.Rv = abs_lt(V, 500.0) ? fast_div(num, tau) : num / tau;
-  }
-  const double c2 = cass * cass;
-  S.sat = imin(threshMAX, const_div(c2, kDivKrate));
-  S.k12 = k12cf * imin(threshMAX, const_div(c2, kDivKrate2));
+// x truncated to FP32, for 0 or 2^-126 <= |x| < 2^127, without an FP64 instruction
+__device__ __forceinline__ float trunc32(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t ah = max(hi & 0x7fffffffu, 0x38000000u) - 0x38000000u;
+  return __uint_as_float(__funnelshift_l(lo, ah, 3) | (hi & 0x80000000u));
 }
 
 // Buffer factors of the local ODE: 1/(1 + a1 + a2) of the subspace and
@@ -1032,12 +1083,65 @@ __device__ __forceinline__ void fcn_fru4(const Group& g, double cajsr, double ca
   const double Jss = const_div(cass - cnext, kDivTauss2ss);
   const double Jss_prev = from(g, Jss, (g.c + 3) & 3);
   const double Jxfer = const_div(cass - Cai, kDivTauxfer);
-  double JDH = -(cass * e2 - Cao * 0.341) * a2j;
-  if (small) JDH = pca2 * (cass - Cao * 0.341) * JDHconstant;
-  JDH = lopen ? JDH : 0.0;
+  double JDH = 0.0;
+  if (lopen) {
+    if (small) JDH = pca2 * (cass - Cao * 0.341) * JDHconstant;
+    else JDH = -(cass * e2 - Cao * 0.341) * a2j;
+  }
   dSS = bSS * (JDH + JRyR - Jxfer - Jss + Jss_prev);
   const double Jtr = const_div(CaNSR - cajsr, kDivTautr);
   dJSR = bJSR * (Jtr - (VSS / VJSR) * JRyRtot);
+}
+
+// The rates of a substep decide two things: its size dt = min(0.1 / the
+// largest rate, a cap), and, against the draws, which channels change state.
+// Both are settled by FP32 estimates of the rates (relative error below
+// 2^-17: two or three roundings, an exponential of an argument below 10 and
+// truncated inputs) wherever the comparison is clear by kRateTol; the rates
+// that could be the largest, and all of a cleft with a draw too close to its
+// threshold (about one substep in 10^4), are formed in FP64 as the reference
+// does.  Rates in FP64 throughout took about 60 of a substep's 190 FP64
+// instructions.
+constexpr float kRateTol = 0x1p-13f;
+
+// First half of one FP64 substep (simfru_local.c:83-146 up to the draws):
+// the layout of the extra draws and the words that precede word 624 first
+// (their loads overlap the rest), then the estimates of the voltage terms and
+// exit totals.
+__device__ __forceinline__ void substep_a(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const Group& g,
+                                          const StageCtx& sc) {
+  const uint32_t w = F.w;
+  const double cass = F.ss.v, V = F.dep[0];
+  S.cajsr = F.jsr.v;
+  S.cass = cass;
+  {
+    const double cc = imin(cass, threshMAXCa);
+    S.regime = ilt(cc, threshCa56to8) ? 0 : (ilt(cc, threshCa34to7) ? 1 : 2);
+  }
+  draw_layout(g, w, S.regime, S.exmask, S.ne, S.pre, S.etot);
+  fetch_old(sc, g, F.mti, S.pre, S.ne, S.etot, S.exw, S.bw);
+  S.ok = fits(cass) && conc_ok(cass) && abs_lt(V, 150.0);
+  // ---- voltage terms at the substep start, one exponential per lane ----
+  const float c = trunc32(cass);
+  const float ev = __expf((trunc32(V) + L.cA) * L.cR);
+  const float vterm = L.isdiv ? __fdividef(L.cK, 1.0f + ev) + L.cM : L.cCF * ev;
+  const float alpha = from(g, vterm, 0), beta = from(g, vterm, 1);
+  const float yinf = from(g, vterm, 2), tau = from(g, vterm, 3);
+  const float bp = beta * (float)(1.0 / (bL * kappa)), gam = (float)gammacf * c;
+  {
+    const float4 row = __ldg(reinterpret_cast<const float4*>(&g_lcc_row32[lcc_of(w)]));
+    const uint32_t code = __float_as_uint(row.w);
+    const int bx = code & 15u, by = (code >> 4) & 15u, bz = (code >> 8) & 15u;
+    S.code = code;
+    S.X = row.x * ((bx == 1) ? alpha : (bx == 2) ? beta : (bx == 5) ? bp : 1.0f);
+    S.Y = row.y * ((by == 1) ? alpha : (by == 3) ? gam : 1.0f);
+    S.Z = row.z * ((bz == 3) ? gam : 1.0f);
+    S.Rl = S.X + S.Y + S.Z;
+  }
+  S.Rv = __fdividef((vdi_of(w) == 2) ? 1.0f - yinf : yinf, tau);
+  const float c2 = c * c;
+  S.sat = fminf((float)threshMAX, c2 * (float)(1.0 / k_rate));
+  S.sat2 = fminf((float)threshMAX, c2 * (float)(1.0 / k_rate2));
 }
 
 // Second half: the remaining words, the RyR pseudo-states, the substep size,
@@ -1045,17 +1149,12 @@ __device__ __forceinline__ void fcn_fru4(const Group& g, double cajsr, double ca
 __device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const Group& g,
                                           StageCtx& sc) {
   uint32_t w = F.w;
-  const double cajsr = S.cajsr, cass = S.cass, sat = S.sat;
+  const double cajsr = S.cajsr, cass = S.cass, V = F.dep[0];
   const int regime = S.regime;
   uint32_t* bw = S.bw;
   fetch_new(sc, g, F.mti, S.pre, S.ne, S.etot, S.exw, bw);
-  const double k34 = k34cf * sat, k56 = k56cf * sat;
-  RyrMasks m = ryr_masks(w);
-  // k34/(k34+k43): for the draws of regimes 0/1 or for the merged state 7 of
-  // regime 2 (never both)
-  double p34 = 0.0;
-  if (m.s7 | (regime == 2 ? m.s3 | m.s4 : 0u)) p34 = fast_div(k34, k34 + k43);
   if (S.ne) {
+    const double sat = sat_exact(cass), k34 = k34cf * sat, k56 = k56cf * sat;
     uint32_t ex = S.exmask;
     while (ex) {
       const int b = __ffs(ex) - 1;  // the RyR's nibble
@@ -1066,55 +1165,74 @@ __device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, cons
       S.exw[2] = S.exw[3];
       S.exw[3] = S.exw[4];
       uint32_t s;
-      if (((w >> (8 + b)) & 15u) == 7u) s = u_below(y, p34) ? 4u : 3u;
+      if (((w >> (8 + b)) & 15u) == 7u) s = u_below(y, fast_div(k34, k34 + k43)) ? 4u : 3u;
       else s = u_below(y, fast_div(k56, k56 + k65)) ? 6u : 5u;
       w = set_field(w, 8 + b, (int)s);
     }
   }
   w = merge_ryr(w, regime);
-  m = ryr_masks(w);
-  // ---- exit totals of the RyR states present, and their maximum ----
-  double mx = imax(S.Rl, S.Rv);
-  const double Rc = (cl_of(w) == 1) ? kfIto2 * cass : kbIto2;
-  mx = imax(mx, Rc);
-  double k23 = 0.0, k25 = 0.0, k54 = 0.0, T2 = 0.0, T5 = 0.0, t7a = 0.0, t7b = 0.0, T7 = 0.0, t8a = 0.0, t8b = 0.0,
-         T8 = 0.0;
-  mx = m.s1 ? imax(mx, S.k12) : mx;
-  if (m.s2) {
-    k23 = k23cf * sat;
-    k25 = k25cf * sat;
-    T2 = k21 + k23 + k25;
-    mx = imax(mx, T2);
+  // ---- exit totals of the RyR states (estimates) ----
+  const float k34 = (float)k34cf * S.sat, k56 = (float)k56cf * S.sat, k54 = (float)k54cf * S.sat,
+              k23 = (float)k23cf * S.sat, k25 = (float)k25cf * S.sat;
+  const float p7 = __fdividef(k34, k34 + (float)k43), p8 = __fdividef((float)k65, k56 + (float)k65);
+  const float t7 = (1.0f - p7) * (float)k32, t8 = p8 * (float)k52;
+  const float T1 = (float)k12cf * S.sat2, T2 = (float)k21 + k23 + k25, T3 = (float)k32 + k34, T4 = (float)(k43 + k45),
+              T5 = (float)k52 + k54 + k56, T6 = (float)k65, T7 = t7 + p7 * (float)k45, T8 = t8 + p8 * k54;
+  const float Rc = (cl_of(w) == 1) ? (float)kfIto2 * trunc32(cass) : (float)kbIto2;
+  float r[kRyR];
+#pragma unroll
+  for (int i = 0; i < kRyR; i++) {
+    const bool b0 = (w >> (8 + 4 * i)) & 1u, b1 = (w >> (9 + 4 * i)) & 1u, b2 = (w >> (10 + 4 * i)) & 1u;
+    const float lo = b1 ? (b0 ? T3 : T2) : (b0 ? T1 : T8), hi = b1 ? (b0 ? T7 : T6) : (b0 ? T5 : T4);
+    r[i] = b2 ? hi : lo;
   }
-  const double T3 = k32 + k34;
-  mx = m.s3 ? imax(mx, T3) : mx;
-  mx = m.s4 ? imax(mx, k43 + k45) : mx;
-  if (m.s5 | m.s8) k54 = k54cf * sat;
-  if (m.s5) {
-    T5 = k52 + k54 + k56;
-    mx = imax(mx, T5);
-  }
-  mx = m.s6 ? imax(mx, k65) : mx;
-  if (m.s7) {
-    t7a = (1.0 - p34) * k32;  // p34 = k34 / (k43 + k34)
-    t7b = p34 * k45;
-    T7 = t7a + t7b;
-    mx = imax(mx, T7);
-  }
-  if (m.s8) {
-    const double a1 = fast_div(k65, k56 + k65);
-    t8a = a1 * k52;
-    t8b = a1 * k54;
-    T8 = t8a + t8b;
-    mx = imax(mx, T8);
-  }
-  mx = gmax(g, mx);
   // ---- substep size (simfru_local.c:135-146) ----
-  double dtr = imin(fits(mx) ? fast_div(0.1, mx) : 0.1 / mx, 10.001e-3);
-  if (__any_sync(g.mask, ilt(1.5e-3, cass))) dtr = imin(dtr, 5.001e-3);
+  const bool ok = __all_sync(g.mask, S.ok);
+  const bool fast_ca = __any_sync(g.mask, ilt(1.5e-3, cass));
+  double dtr = fast_ca ? 5.001e-3 : 10.001e-3;
+  float mx = fmaxf(fmaxf(fmaxf(S.Rl, S.Rv), Rc), fmaxf(fmaxf(fmaxf(r[0], r[1]), fmaxf(r[2], r[3])), r[4]));
+  mx = fmaxf(mx, __shfl_xor_sync(g.mask, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(g.mask, mx, 2));
+  // 0.1 / cap = 19.996 or 9.999: below these the cap is the smaller
+  if (!ok || !(mx < (fast_ca ? 19.99f : 9.998f))) {
+    const float near = ok ? mx * (1.0f - kRateTol) : -1.0f;  // -1: every rate
+    double m = 0.0;
+    const bool lcc = !(S.Rl < near);
+    if (__any_sync(g.mask, lcc)) {
+      // alpha on the even lanes, beta on the odd ones
+      const bool odd = g.c & 1;
+      const double t = (odd ? betacf : alphacf) * fexp((odd ? -0.05 : 0.012) * (V - 35.0));
+      const double alpha = from(g, t, 0), beta = from(g, t, 1);
+      double X, Y, Z;
+      lcc_exact(w, alpha, beta, cass, X, Y, Z);
+      if (lcc) m = imax(m, X + Y + Z);
+    }
+    if (!(S.Rv < near)) m = imax(m, vdi_rate_exact(w, V));
+    if (!(Rc < near)) m = imax(m, (cl_of(w) == 1) ? kfIto2 * cass : kbIto2);
+    const RyrMasks q = ryr_masks(w);
+    if (q.s3 && !(T3 < near)) m = imax(m, k32 + k34cf * sat_exact(cass));
+    if (q.s4 && !(T4 < near)) m = imax(m, k43 + k45);
+    if (q.s6 && !(T6 < near)) m = imax(m, k65);
+    const uint32_t rest = q.s1 | q.s2 | q.s5 | q.s7 | q.s8;
+    if (rest) {
+#pragma unroll 1
+      for (int k = 0; k < 5; k++) {
+        const int s = (k < 2) ? k + 1 : (k == 2) ? 5 : k + 4;  // 1, 2, 5, 7, 8
+        const uint32_t there = (k == 0) ? q.s1 : (k == 1) ? q.s2 : (k == 2) ? q.s5 : (k == 3) ? q.s7 : q.s8;
+        const float T = (k == 0) ? T1 : (k == 1) ? T2 : (k == 2) ? T5 : (k == 3) ? T7 : T8;
+        if (there && !(T < near)) {
+          double r1, r2;
+          int len;
+          uint32_t d;
+          m = imax(m, ryr_total_exact(s, cass, regime, r1, r2, len, d));
+        }
+      }
+    }
+    m = gmax(g, m);
+    dtr = imin(fits(m) ? fast_div(0.1, m) : 0.1 / m, dtr);
+  }
   const double dt = F.clk.advance(dtr, L);
   // ---- Heun step (simfru_local.c:149-173) ----
-  const bool in_range = conc_ok(cass) && abs_lt(F.dep[0], 500.0);
   double dJ, dS;
   fcn_fru4(g, cajsr, cass, F.dep, F.e2, F.a2j, F.small, F.lopen, F.jcoef, L.pca2, dJ, dS);
   const double k1J = dt * dJ, k1S = dt * dS;
@@ -1130,73 +1248,74 @@ __device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, cons
   F.jsr.v = fma(k1J + dt * dJ, 0.5, cajsr);
   F.ss.v = fma(k1S + dt * dS, 0.5, cass);
   // ---- transitions of this cleft's 8 channels (:215-276) ----
-  // A channel leaves when c = 2^32 - y is below about dt*R*2^32.  First an
-  // upper bound of that in FP32 (dt and R by their heads, raised by 2^-16,
-  // and 2^-22 for the dropped bits of c); the few channels within it form
-  // 1 - dt*R.  The RyRs that may leave take one pass each: the lanes of a
-  // warp share the pass.  Each RyR's row depends only on its own state and
-  // its cleft's constants, so the order of the passes does not matter.
-  const float dth = __fmul_rn(head32(dt), 1.0f + 0x1p-16f);
-  auto near_leaving = [&](uint32_t y, float R) {
-    return __uint_as_float((~y >> 9) | 0x3f800000u) <= __fmaf_rn(R, dth, 1.0f + 0x1p-22f);
+  // A channel leaves when c = 2^32 - y is below about dt*R*2^32; `open` is set
+  // where c is within the tolerance of a threshold (or of the 2 that
+  // roundings of the exact one can move it).  The RyRs that leave take one
+  // pass each: the lanes of a warp share the pass.  Each RyR's row depends
+  // only on its own state and its cleft's constants, so the order of the
+  // passes does not matter.
+  const float dts = trunc32(dt) * 4294967296.0f;
+  bool open = !S.ok;
+  auto below = [&](float c, float t, float tol) {
+    open = open || fabsf(c - t) <= tol;
+    return c < t;
   };
-  uint32_t cand = 0u;
-  {
-    const float f1 = head32(S.k12), f2 = head32(T2), f3 = head32(T3), f4 = head32(k43 + k45), f5 = head32(T5),
-                f6 = head32(k65), f7 = head32(T7), f8 = head32(T8);
+  auto leaves = [&](uint32_t y, float R) {
+    const float t = dts * R;
+    return below(comp_u32(y), t, __fmaf_rn(t, kRateTol, 2.0f));
+  };
+  uint32_t n = w;
+  if (leaves(bw[0], S.Rl)) {
+    const uint32_t perm = S.code >> 28, len = (S.code >> 12) & 15u;
+    uint32_t d = S.code >> 16;
+    const float r1 = (perm == 1) ? S.Y : S.X, r2 = (perm == 2) ? S.Z : (perm == 1) ? S.X : S.Y;
+    const float cc = comp_u32(bw[0]), tol = __fmaf_rn(dts * S.Rl, kRateTol, 2.0f);
+    if (len > 2u && below(cc, dts * (S.Rl - r1), tol)) {
+      d >>= 4;
+      if (len > 3u && below(cc, dts * (S.Rl - r1 - r2), tol)) d >>= 4;
+    }
+    n = set_field(n, 0, (int)(d & 15u));
+  }
+  if (leaves(bw[1], S.Rv)) n = set_field(n, 4, 3 - vdi_of(w));
+  uint32_t pend = 0u;
 #pragma unroll
-    for (int i = 0; i < kRyR; i++) {
-      const bool b0 = (w >> (8 + 4 * i)) & 1u, b1 = (w >> (9 + 4 * i)) & 1u, b2 = (w >> (10 + 4 * i)) & 1u;
-      const float lo = b1 ? (b0 ? f3 : f2) : (b0 ? f1 : f8), hi = b1 ? (b0 ? f7 : f6) : (b0 ? f5 : f4);
-      cand |= near_leaving(bw[2 + i], b2 ? hi : lo) ? (1u << i) : 0u;
-    }
-  }
-  bool lcc = near_leaving(bw[0], head32(S.Rl));
-  bool vdi = near_leaving(bw[1], head32(S.Rv)), cl = near_leaving(bw[7], head32(Rc));
-  if (!in_range) {
-    cand = 31u;
-    lcc = vdi = cl = true;
-  }
-  const uint32_t w0 = w;
-  if (lcc) {
-    const double P = 1.0 - dt * S.Rl;
-    if (u_above(bw[0], P)) {
-      const uint32_t code = __ldg(&g_lcc_row64[lcc_of(w)].code);
-      const uint32_t perm = code >> 28;
-      const double r1 = (perm == 1) ? S.Y : S.X, r2 = (perm == 2) ? S.Z : (perm == 1) ? S.X : S.Y;
-      w = set_field(w, 0, (int)walk(bw[0], P, dt, r1, r2, (int)((code >> 12) & 15u), code >> 16));
-    }
-  }
-  if (vdi && u_reaches(bw[1], 1.0 - dt * S.Rv)) w = set_field(w, 4, 3 - vdi_of(w));
-  while (cand) {
-    const int i = __ffs(cand) - 1;
-    cand &= cand - 1u;
+  for (int i = 0; i < kRyR; i++) pend |= leaves(bw[2 + i], r[i]) ? (1u << i) : 0u;
+  while (pend) {
+    const int i = __ffs(pend) - 1;
+    pend &= pend - 1u;
     uint32_t y = bw[2];  // the RyR's uniform, by selection (no dynamic register indexing)
     y = (i == 1) ? bw[3] : y;
     y = (i == 2) ? bw[4] : y;
     y = (i == 3) ? bw[5] : y;
     y = (i == 4) ? bw[6] : y;
     const int s = ryr_of(w, i);
-    // exit total, first two rates, row length and destinations of the state
-    // (fru_rates_local.c:374-736)
+    // the total less the first one and the first two rates, row length and
+    // destinations (fru_rates_local.c:374-736)
     const uint32_t to5 = (regime == 0) ? 5u : 8u, to7 = (regime == 2) ? 7u : 3u;
-    double T = S.k12, r1 = 0.0, r2 = 0.0;
+    float T = T1, u1 = 0.0f, u2 = 0.0f;
     int len = 2;
     uint32_t d = 2u;  // 1 -> 2
-    if (s == 2) { T = T2; r1 = k21; r2 = k23; len = 4; d = 1u | (to7 << 4) | (to5 << 8); }
-    if (s == 3) { T = T3; r1 = k32; len = 3; d = 0x42u; }
-    if (s == 4) { T = k43 + k45; r1 = k43; len = 3; d = 3u | (to5 << 4); }
-    if (s == 5) { T = T5; r1 = k52; r2 = k54; len = 4; d = 0x642u; }
-    if (s == 6) { T = k65; d = 5u; }
-    if (s == 7) { T = T7; r1 = t7a; len = 3; d = 0x82u; }
-    if (s == 8) { T = T8; r1 = t8a; len = 3; d = (regime == 2) ? 0x72u : 0x42u; }
-    const double P = 1.0 - dt * T;
-    if (u_above(y, P)) w = set_field(w, 8 + 4 * i, (int)walk(y, P, dt, r1, r2, len, d));
+    if (s == 2) { T = T2; u1 = k23 + k25; u2 = k25; len = 4; d = 1u | (to7 << 4) | (to5 << 8); }
+    if (s == 3) { T = T3; u1 = k34; len = 3; d = 0x42u; }
+    if (s == 4) { T = T4; u1 = (float)k45; len = 3; d = 3u | (to5 << 4); }
+    if (s == 5) { T = T5; u1 = k54 + k56; u2 = k56; len = 4; d = 0x642u; }
+    if (s == 6) { T = T6; d = 5u; }
+    if (s == 7) { T = T7; u1 = T7 - t7; len = 3; d = 0x82u; }
+    if (s == 8) { T = T8; u1 = T8 - t8; len = 3; d = (regime == 2) ? 0x72u : 0x42u; }
+    const float cc = comp_u32(y), tol = __fmaf_rn(dts * T, kRateTol, 2.0f);
+    if (len > 2 && below(cc, dts * u1, tol)) {
+      d >>= 4;
+      if (len > 3 && below(cc, dts * u2, tol)) d >>= 4;
+    }
+    n = set_field(n, 8 + 4 * i, (int)(d & 15u));
   }
-  if (cl && u_reaches(bw[7], 1.0 - dt * Rc)) w = set_field(w, 28, 3 - cl_of(w));
-  F.lopen = lcc_open(w);
-  if (w != w0) F.jcoef = jryr_open(w);
-  F.w = w;
+  if (leaves(bw[7], Rc)) n = set_field(n, 28, 3 - cl_of(w));
+  if (open)
+    n = transitions_exact(w, V, cass, dt, regime, make_uint4(bw[0], bw[1], bw[2], bw[3]),
+                          make_uint4(bw[4], bw[5], bw[6], bw[7]));
+  F.lopen = lcc_open(n);
+  if (n != w) F.jcoef = jryr_open(n);
+  F.w = n;
   F.nsub++;
 }
 
