@@ -8,6 +8,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
 #include <new>
 #include <vector>
 
@@ -37,6 +38,19 @@ static int set_err(int code, const char* fmt, ...) {
                                           __FILE__, __LINE__);                                  \
   } while (0)
 
+// Warps (8-FRU groups) of the stages in flight on each device, over all cells
+// and threads: a launch takes the stage kernel's roomy build while they all
+// fit the device with it, else the dense one.  Both give the same results.
+static std::atomic<int> g_stage_warps[64];
+struct StageInFlight {
+  std::atomic<int>& n;
+  const int warps;
+  explicit StageInFlight(const gw_ctx* c) : n(g_stage_warps[c->device & 63]), warps((c->d.nfru + 7) / 8) {
+    n.fetch_add(warps, std::memory_order_relaxed);
+  }
+  ~StageInFlight() { n.fetch_sub(warps, std::memory_order_relaxed); }
+};
+
 static cudaError_t launch_stage_variant(gw_ctx* c, const StageParams& p0) {
   StageParams p = p0;
   p.launch = c->pack_launch;
@@ -49,8 +63,9 @@ static cudaError_t launch_stage_variant(gw_ctx* c, const StageParams& p0) {
     c->pack_launch++;
     c->launches++;
   }
-  if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, c->stream);
-  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, c->stream)
+  const bool dense = g_stage_warps[c->device & 63].load(std::memory_order_relaxed) > gw::kRoomyWarpsPerSm * c->sms;
+  if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, dense, c->stream);
+  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, dense, c->stream)
                            : gw::launch_stage(c->d, p, c->stream);
 }
 
@@ -84,6 +99,7 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   gw_ctx* c = new (std::nothrow) gw_ctx();
   if (!c) return set_err(GW_ENOMEM, "gw_create: host allocation failed");
   cudaGetDevice(&c->device);
+  cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
   DevState& d = c->d;
   d.nfru = nfru;
   d.stride = (nfru + 31) & ~31;
@@ -360,6 +376,7 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
     if (rc) return rc;
   } else {
     // the kernels write the sums into h_out itself
+    const StageInFlight in_flight(c);
     if (c->profiling) CK(cudaEventRecord(c->pev[0], c->stream));
     CK(launch_stage_variant(c, p));
     c->launches++;

@@ -16,6 +16,7 @@ struct gw_ctx {
   uint32_t epoch = 0;
   int pending = 0;          // kFlagSave / kFlagResume to fold into the next launch
   int device = 0;
+  int sms = 0;              // its multiprocessors
   cudaEvent_t ev[8] = {};
   cudaEvent_t pev[2] = {};  // bracket of the last stage launch while profiling
   bool profiling = false;

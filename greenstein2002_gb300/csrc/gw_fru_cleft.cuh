@@ -20,8 +20,8 @@
 //   - products with 0/1 flags are selections, halvings are folded into FMAs
 //     (both exact), the three interpolated voltages/concentrations are
 //     computed one per lane, and exp(2VF/RT) at the end of a substep is reused
-//     at the start of the
-//     next (and at the stage start computed once per lane, not per FRU).
+//     at the start of the next (and at the stage start computed once per
+//     lane, not per FRU).
 // R = float: the mixed-precision method.  Transition rates, the local Ca ODE
 // and the FRU clock are evaluated in FP32, the Ca states and the clock
 // accumulated as compensated FP32 pairs; FP64 is kept for the FRU arrays in

@@ -10,15 +10,25 @@
 
 namespace gw {
 
-__global__ void __launch_bounds__(kMaxStageWarps * 32) fru_stage_mixed_kernel(DevState s, StageParams p) {
+// Two builds, as in gw_fru_stage4.cu: 182 registers (eleven single-warp blocks
+// per SM) and 128 (sixteen).  Alone, five stages with 128 and 182: 1,251 FRUs
+// 0.532 and 0.505 ms, 12,500 FRUs 1.415 and 1.370 ms; 16 cells of 12,500 FRUs
+// at once for 10 ms: 580 and 891 ms.
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage_mixed_kernel(DevState s, StageParams p) {
+  cleft::stage_body<float>(s, p, blockIdx.x, s.res);
+}
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage_mixed_dense_kernel(DevState s, StageParams p) {
   cleft::stage_body<float>(s, p, blockIdx.x, s.res);
 }
 
-cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, cudaStream_t st) {
+cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, bool dense, cudaStream_t st) {
   const int blocks = stage_blocks(s.nfru, warps);
   static const cudaError_t attr = stage_cache_attributes(fru_stage_mixed_kernel);
+  static const cudaError_t attr_dense = stage_cache_attributes(fru_stage_mixed_dense_kernel);
   if (attr != cudaSuccess) return attr;
-  fru_stage_mixed_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  if (attr_dense != cudaSuccess) return attr_dense;
+  if (dense) fru_stage_mixed_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  else fru_stage_mixed_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
   return cudaGetLastError();
 }
 
@@ -31,7 +41,9 @@ cudaError_t launch_stage_mixed_batch(const BatchArgs& a, int nblocks, int warps,
   return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(32, 16) fru_stage_mixed_packed_kernel(DevState s, StageParams p) {
+// 16 cells of 12,500 FRUs for 10 ms, 32 FRUs per warp, with at least 12 / 14 /
+// 16 / 18 / 20 single-warp blocks per SM: 528 / 487 / 501 / 562 / 545 ms.
+__global__ void __launch_bounds__(32, 14) fru_stage_mixed_packed_kernel(DevState s, StageParams p) {
   cleft::stage_body_packed<float>(s, p, s.res);
 }
 

@@ -7,15 +7,25 @@
 
 namespace gw {
 
-__global__ void __launch_bounds__(kMaxStageWarps * 32) fru_stage4_kernel(DevState s, StageParams p) {
+// Two builds of the fixed-layout kernel: with the registers it asks for (180,
+// eleven single-warp blocks per SM) for launches that fit the GPU so, and
+// capped at 128 (sixteen) for more.  Five stages at the peak of release, 128
+// and 180 registers: 12,500 FRUs 6.82 and 6.07 ms, 250 FRUs alike.
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage4_kernel(DevState s, StageParams p) {
+  cleft::stage_body<double>(s, p, blockIdx.x, s.res);
+}
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage4_dense_kernel(DevState s, StageParams p) {
   cleft::stage_body<double>(s, p, blockIdx.x, s.res);
 }
 
-cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, cudaStream_t st) {
+cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, bool dense, cudaStream_t st) {
   const int blocks = stage_blocks(s.nfru, warps);
   static const cudaError_t attr = stage_cache_attributes(fru_stage4_kernel);
+  static const cudaError_t attr_dense = stage_cache_attributes(fru_stage4_dense_kernel);
   if (attr != cudaSuccess) return attr;
-  fru_stage4_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  if (attr_dense != cudaSuccess) return attr_dense;
+  if (dense) fru_stage4_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  else fru_stage4_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
   return cudaGetLastError();
 }
 
@@ -28,10 +38,10 @@ cudaError_t launch_stage4_batch(const BatchArgs& a, int nblocks, int warps, cuda
   return cudaGetLastError();
 }
 
-// At least eleven single-warp blocks per SM: the register cap (<= 186 per
-// thread; 168 used, so twelve fit) against 191 uncapped (measured 4-13%
-// faster on the 16-cell ensemble, where the FP64 pipe is ~75% busy).
-__global__ void __launch_bounds__(32, 11) fru_stage4_packed_kernel(DevState s, StageParams p) {
+// At least thirteen single-warp blocks per SM (<= 152 registers).  16 cells
+// of 12,500 FRUs for 2 ms, 32 FRUs per warp, with 11 / 12 / 13 / 14 / 15 / 16
+// blocks: 617 / 604 / 584 / 592 / 591 / 595 ms.
+__global__ void __launch_bounds__(32, 13) fru_stage4_packed_kernel(DevState s, StageParams p) {
   cleft::stage_body_packed<double>(s, p, s.res);
 }
 
