@@ -2,6 +2,7 @@
 // downloads in the reference's array layout, and the stage / flux / average
 // / save / resume operations that replace the MPI layer of mpi_master.c.
 #include <cuda_runtime.h>
+#include <sched.h>
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -356,6 +357,26 @@ extern "C" int gw_seed(gw_ctx* c, int scheme, uint32_t base) {
   return GW_OK;
 }
 
+// Wait for the totals of launch seq: the kernel's last warp writes its number
+// into h_out after them.  Waiting on the stream instead goes through the
+// driver's locks, which every cell's host thread shares: 24 uneven mixed
+// cells on their own threads (16 cores) took 145 ms for 10 ms, 87 ms with
+// this wait; a thread alone waits as long either way.  The stream is asked
+// now and then, so that a failed launch ends the wait; the kernel may still be
+// retiring when this returns, so all that follows stays ordered by the stream.
+static cudaError_t wait_totals(gw_ctx* c, uint32_t seq) {
+  const unsigned long long* slot = reinterpret_cast<const unsigned long long*>(c->h_out + gw::kOutSeq);
+  for (;;) {
+    for (int i = 0; i < 256; i++) {
+      for (int k = 0; k < 64; k++)
+        if (__atomic_load_n(slot, __ATOMIC_ACQUIRE) == seq) return cudaSuccess;
+      sched_yield();
+    }
+    const cudaError_t e = cudaStreamQuery(c->stream);
+    if (e != cudaErrorNotReady) return e;
+  }
+}
+
 static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], const double depf[3], int advance,
                      double out[4], double num[5]) {
   StageParams p;
@@ -370,6 +391,7 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
   p.pca_scale = c->pca_scale;
   p.epoch = c->epoch;
   p.flags = c->pending | (advance ? gw::kFlagAdvance : 0);
+  p.seq = ++c->seq;
   c->pending = 0;
   if (c->batch) {
     int rc = gw_batch_post(c, p, c->h_out);
@@ -385,7 +407,9 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
       c->launches++;
     }
     if (c->profiling) CK(cudaEventRecord(c->pev[1], c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    // the one-lane kernel and the sequential sums do not number their totals
+    const bool numbered = c->fru_lanes == 4 && c->sum_order == GW_SUM_TREE && !c->profiling;
+    CK(numbered ? wait_totals(c, p.seq) : cudaStreamSynchronize(c->stream));
   }
   if (c->h_out[gw::kOutError] != 0.0) {
     c->h_out[gw::kOutError] = 0.0;

@@ -14,6 +14,7 @@ struct gw_ctx {
   double* h_out = nullptr;  // pinned [32], mapped at d.res
   double nfru_scale = 1.0;
   uint32_t epoch = 0;
+  uint32_t seq = 0;         // stage and flux launches so far (their totals' sequence numbers)
   int pending = 0;          // kFlagSave / kFlagResume to fold into the next launch
   int device = 0;
   int sms = 0;              // its multiprocessors

@@ -1394,6 +1394,14 @@ __device__ __forceinline__ void put_totals(const DevState& s, const StageParams&
   if (lane < 4) out[5 + lane] = cur;
   else if (lane < 9) out[lane - 4] = v;
 }
+// after every total: tell the host that waits for this launch
+__device__ __forceinline__ void put_seq(const StageParams& p, double* out, int lane) {
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence_system();
+    *reinterpret_cast<volatile unsigned long long*>(out + kOutSeq) = p.seq;
+  }
+}
 
 template <typename R>
 __device__ __forceinline__ void stage_body(const DevState& s, const StageParams& p, int bidx, double* out) {
@@ -1491,6 +1499,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
       if (lane == 0)
 #pragma unroll
         for (int k = 0; k < 11; k++) out[16 + k] = tot[5 + k];
+      put_seq(p, out, lane);
     }
     return;
   }
@@ -1501,6 +1510,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
     double tot[5];
     unpack_flux(v, tot);
     put_totals(s, p, out, tot, lane);
+    put_seq(p, out, lane);
   }
 }
 

@@ -22,6 +22,9 @@ cudaError_t stage_cache_attributes(K kernel) {
 inline int stage_blocks(int nfru, int warps) { return ((nfru + 7) / 8 + warps - 1) / warps; }
 // out[] slot of the device error flag (substep limit hit)
 constexpr int kOutError = 31;
+// out[] slot of the sequence number (StageParams::seq) the launch that
+// completes a cell's totals writes after them
+constexpr int kOutSeq = 30;
 
 enum : int {
   kFlagAdvance = 1,  // run the substep loop over [t0, tf]
@@ -42,7 +45,7 @@ enum : int { kSeedBase = 0, kSeedReference = 1 };
 //                     over the groups of 8 FRUs
 //   res[32]           results the host reads, in its own (pinned, mapped) memory:
 //                     [0..4] flux sums, [5..8] Jxfer,Jtr,ICa,Ito2, [16..26] averages,
-//                     [31] error flag
+//                     [30] sequence number of the launch, [31] error flag
 //   out[32]           the same of the round-based device integrator, in device memory
 struct DevState {
   int nfru, stride, nblocks;
@@ -81,6 +84,7 @@ struct StageParams {
   uint32_t epoch;
   int flags;
   uint32_t launch;  // packed launches of the cell so far
+  uint32_t seq;     // number of the launch, for the host that waits for its totals
 };
 
 // Many cells in one launch (cleft-parallel kernels): cell i owns blocks

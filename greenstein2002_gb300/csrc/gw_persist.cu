@@ -430,9 +430,12 @@ __device__ __forceinline__ void persist_body(const Args& a) {
   }
 }
 
-// Single-warp blocks, at least ten per SM (the register cap).
-__global__ void __launch_bounds__(32, 10) persist_kernel_fp64(Args a) { persist_body<double>(a); }
-__global__ void __launch_bounds__(32, 10) persist_kernel_mixed(Args a) { persist_body<float>(a); }
+// Single-warp blocks, at least eight per SM (<= 255 registers).  24 uneven
+// mixed cells for 10 ms with at least 8 / 10 / 13 / 16: 119 / 128 / 135 / 134
+// ms, 16 of 12,500 FRUs 594 / 667 / 706 / 696 ms: the warps' batches, not
+// their number, fill the SMs.
+__global__ void __launch_bounds__(32, 8) persist_kernel_fp64(Args a) { persist_body<double>(a); }
+__global__ void __launch_bounds__(32, 8) persist_kernel_mixed(Args a) { persist_body<float>(a); }
 
 }  // namespace persist
 }  // namespace gw
