@@ -64,9 +64,19 @@ static cudaError_t launch_stage_variant(gw_ctx* c, const StageParams& p0) {
     c->pack_launch++;
     c->launches++;
   }
-  const bool dense = g_stage_warps[c->device & 63].load(std::memory_order_relaxed) > gw::kRoomyWarpsPerSm * c->sms;
-  if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, dense, c->stream);
-  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, dense, c->stream)
+  const int groups = g_stage_warps[c->device & 63].load(std::memory_order_relaxed);
+  const bool dense = groups > gw::kRoomyWarpsPerSm * c->sms;
+  // Few FRUs: fewer of them per warp, as long as that makes at most four warps
+  // per SM (one per sub-partition), because the FRUs of a warp execute each
+  // other's branches.  Five stages at the peak of release with 8, 4, 2 and 1
+  // per warp: FP64 250 FRUs 2.97 / 2.85 / 2.82 / 2.81 ms, 1,250 FRUs 3.72 /
+  // 3.62 / 3.60 / 3.72, 2,500 FRUs 3.69 / 3.60 / 3.87 / 4.67; mixed 250 FRUs
+  // 0.651 / 0.630 / 0.614 / 0.609 ms.
+  int fpw = 8;
+  if ((p.flags & gw::kFlagAdvance) && !c->d.trace_ns)
+    fpw = 4 * groups <= 4 * c->sms ? 2 : 2 * groups <= 4 * c->sms ? 4 : 8;
+  if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, fpw, dense, c->stream);
+  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, fpw, dense, c->stream)
                            : gw::launch_stage(c->d, p, c->stream);
 }
 
@@ -79,7 +89,7 @@ extern "C" int gw_nfru(const gw_ctx* c) { return c ? c->d.nfru : 0; }
 
 static void free_dev(gw_ctx* c) {
   void* ptrs[] = {c->d.frus, c->d.chan, c->d.mti, c->d.mt, c->d.frus_s, c->d.chan_s, c->d.mti_s,
-                  c->d.mt_hold, c->d.hold_epoch, c->d.partials, c->d.ticket, c->d.out, c->d.substeps,
+                  c->d.mt_hold, c->d.hold_epoch, c->d.partials, c->d.ticket, c->d.gcount, c->d.out, c->d.substeps,
                   c->d.trace_sub, c->d.trace_ns, c->d.qctl, c->d.heavy_list, c->d.heavy_tag};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -121,6 +131,7 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   // partial sums of the 8-FRU groups
   AL(d.partials, (size_t)((nfru + 7) / 8) * 16 * sizeof(double));
   AL(d.ticket, sizeof(unsigned));
+  AL(d.gcount, (size_t)((nfru + 7) / 8) * sizeof(unsigned));
   AL(d.out, 32 * sizeof(double));
   AL(d.substeps, sizeof(unsigned long long));
   AL(d.qctl, 8 * sizeof(unsigned));
@@ -136,6 +147,7 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
   for (int i = 0; i < 2 && e == cudaSuccess; i++) e = cudaEventCreate(&c->pev[i]);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.ticket, 0, sizeof(unsigned), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.gcount, 0, (size_t)((nfru + 7) / 8) * sizeof(unsigned), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.out, 0, 32 * sizeof(double), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.substeps, 0, sizeof(unsigned long long), c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.hold_epoch, 0xff, nf * sizeof(uint32_t), c->stream);

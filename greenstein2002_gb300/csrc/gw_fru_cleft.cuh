@@ -1404,10 +1404,10 @@ __device__ __forceinline__ void put_seq(const StageParams& p, double* out, int l
 }
 
 template <typename R>
-__device__ __forceinline__ void stage_body(const DevState& s, const StageParams& p, int bidx, double* out) {
+__device__ __forceinline__ void stage_body(const DevState& s, const StageParams& p, int bidx, double* out, int fpw = 8) {
   const int lane = threadIdx.x & 31;
-  const int grp = bidx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
-  const int ngroups = (s.nfru + 7) >> 3;
+  const int first = (bidx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * fpw;  // the warp's first FRU
+  const int grp = first >> 3;  // their 8-FRU group
   if ((p.flags & kFlagQueueReset) && bidx == 0 && threadIdx.x == 0) {
     // after a packed launch: ready the queue for the next one (the heavy-FRU
     // threshold becomes 3x this launch's mean substeps per FRU, at least 8)
@@ -1418,16 +1418,17 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
     s.qctl[0] = 0u;
     s.qctl[1 + ((p.launch + 1u) & 1u)] = 0u;
   }
-  if (grp >= ngroups) return;  // whole warps past the cell's last FRU
+  if (first >= s.nfru) return;  // whole warps past the cell's last FRU
   if (s.trace_ns && lane == 0) s.trace_ns[2 * grp] = global_ns();
   Group g;
   g.c = lane & 3;
   g.base = lane & ~3;
   g.mask = 0xfu << g.base;
-  const int f = grp * 8 + (lane >> 2);
+  const int slot = lane >> 2;
+  bool active = slot < fpw && first + slot < s.nfru;  // uniform over each 4-lane group
+  const int f = active ? first + slot : first;
   uint32_t nsub = 0;
   bool overflow = false;
-  const bool active = f < s.nfru;  // uniform over each 4-lane group
   const size_t nf = (size_t)s.stride;
   double cajsr = 0.0, cass = 0.0;
   uint32_t w = 0u;
@@ -1439,7 +1440,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
   sc.hold_base = s.mt_hold;
   sc.hold_epoch_base = s.hold_epoch;
   sc.f = f;
-  sc.my_hold_epoch = s.hold_epoch + f;  // within the padded arrays even past the last FRU
+  sc.my_hold_epoch = s.hold_epoch + f;
   bool restore = false;
   if (active) {
     if (p.flags & kFlagResume) {
@@ -1487,6 +1488,25 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
   if (s.substeps) {
     unsigned c = __reduce_add_sync(0xffffffffu, (g.c == 0) ? nsub : 0u);
     if (lane == 0 && c) atomicAdd(s.substeps, (unsigned long long)c);
+  }
+  if (fpw < 8) {
+    // several warps share the group: the one that completes it sums it, from
+    // the FRUs as stored
+    const unsigned mine = (unsigned)min(fpw, s.nfru - first), size = (unsigned)min(8, s.nfru - grp * 8);
+    unsigned last = 0u;
+    if (lane == 0) {
+      __threadfence();
+      last = (atomicAdd(&s.gcount[grp], mine) + mine == size) ? 1u : 0u;
+      if (last) s.gcount[grp] = 0u;
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    active = slot < (int)size;
+    if (active) {
+      cajsr = __ldcg(&s.frus[grp * 8 + slot]);
+      cass = __ldcg(&s.frus[(g.c + 1) * nf + grp * 8 + slot]);
+      w = __ldcg(&s.chan[g.c * nf + grp * 8 + slot]);
+    }
   }
   if (p.flags & kFlagAvg) {
     AvgSums v = {};

@@ -14,21 +14,21 @@ namespace gw {
 // per SM) and 128 (sixteen).  Alone, five stages with 128 and 182: 1,251 FRUs
 // 0.532 and 0.505 ms, 12,500 FRUs 1.415 and 1.370 ms; 16 cells of 12,500 FRUs
 // at once for 10 ms: 580 and 891 ms.
-__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage_mixed_kernel(DevState s, StageParams p) {
-  cleft::stage_body<float>(s, p, blockIdx.x, s.res);
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage_mixed_kernel(DevState s, StageParams p, int fpw) {
+  cleft::stage_body<float>(s, p, blockIdx.x, s.res, fpw);
 }
-__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage_mixed_dense_kernel(DevState s, StageParams p) {
-  cleft::stage_body<float>(s, p, blockIdx.x, s.res);
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage_mixed_dense_kernel(DevState s, StageParams p, int fpw) {
+  cleft::stage_body<float>(s, p, blockIdx.x, s.res, fpw);
 }
 
-cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, bool dense, cudaStream_t st) {
-  const int blocks = stage_blocks(s.nfru, warps);
+cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, int fpw, bool dense, cudaStream_t st) {
+  const int blocks = stage_blocks(s.nfru, warps, fpw);
   static const cudaError_t attr = stage_cache_attributes(fru_stage_mixed_kernel);
   static const cudaError_t attr_dense = stage_cache_attributes(fru_stage_mixed_dense_kernel);
   if (attr != cudaSuccess) return attr;
   if (attr_dense != cudaSuccess) return attr_dense;
-  if (dense) fru_stage_mixed_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
-  else fru_stage_mixed_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  if (dense) fru_stage_mixed_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p, fpw);
+  else fru_stage_mixed_kernel<<<blocks, 32 * warps, 0, st>>>(s, p, fpw);
   return cudaGetLastError();
 }
 

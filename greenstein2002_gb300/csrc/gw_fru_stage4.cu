@@ -11,21 +11,21 @@ namespace gw {
 // eleven single-warp blocks per SM) for launches that fit the GPU so, and
 // capped at 128 (sixteen) for more.  Five stages at the peak of release, 128
 // and 180 registers: 12,500 FRUs 6.82 and 6.07 ms, 250 FRUs alike.
-__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage4_kernel(DevState s, StageParams p) {
-  cleft::stage_body<double>(s, p, blockIdx.x, s.res);
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage4_kernel(DevState s, StageParams p, int fpw) {
+  cleft::stage_body<double>(s, p, blockIdx.x, s.res, fpw);
 }
-__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage4_dense_kernel(DevState s, StageParams p) {
-  cleft::stage_body<double>(s, p, blockIdx.x, s.res);
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage4_dense_kernel(DevState s, StageParams p, int fpw) {
+  cleft::stage_body<double>(s, p, blockIdx.x, s.res, fpw);
 }
 
-cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, bool dense, cudaStream_t st) {
-  const int blocks = stage_blocks(s.nfru, warps);
+cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, int fpw, bool dense, cudaStream_t st) {
+  const int blocks = stage_blocks(s.nfru, warps, fpw);
   static const cudaError_t attr = stage_cache_attributes(fru_stage4_kernel);
   static const cudaError_t attr_dense = stage_cache_attributes(fru_stage4_dense_kernel);
   if (attr != cudaSuccess) return attr;
   if (attr_dense != cudaSuccess) return attr_dense;
-  if (dense) fru_stage4_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
-  else fru_stage4_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  if (dense) fru_stage4_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p, fpw);
+  else fru_stage4_kernel<<<blocks, 32 * warps, 0, st>>>(s, p, fpw);
   return cudaGetLastError();
 }
 

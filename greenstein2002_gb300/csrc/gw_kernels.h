@@ -19,7 +19,7 @@ template <typename K>
 cudaError_t stage_cache_attributes(K kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
 }
-inline int stage_blocks(int nfru, int warps) { return ((nfru + 7) / 8 + warps - 1) / warps; }
+inline int stage_blocks(int nfru, int warps, int fpw = 8) { return ((nfru + fpw - 1) / fpw + warps - 1) / warps; }
 // out[] slot of the device error flag (substep limit hit)
 constexpr int kOutError = 31;
 // out[] slot of the sequence number (StageParams::seq) the launch that
@@ -43,6 +43,7 @@ enum : int { kSeedBase = 0, kSeedReference = 1 };
 //   mt_hold/hold_epoch  copy-on-twist protection of the saved MT words
 //   partials[groups][16], ticket: scratch of the deterministic reductions
 //                     over the groups of 8 FRUs
+//   gcount[groups]    FRUs of a group done, where several warps share it
 //   res[32]           results the host reads, in its own (pinned, mapped) memory:
 //                     [0..4] flux sums, [5..8] Jxfer,Jtr,ICa,Ito2, [16..26] averages,
 //                     [30] sequence number of the launch, [31] error flag
@@ -60,6 +61,7 @@ struct DevState {
   uint32_t* hold_epoch;
   double* partials;
   unsigned* ticket;
+  unsigned* gcount;
   double* out;
   double* res;
   unsigned long long* substeps;
@@ -105,11 +107,12 @@ cudaError_t launch_stage4_batch(const BatchArgs& a, int nblocks, int warps, cuda
 cudaError_t launch_stage_mixed_batch(const BatchArgs& a, int nblocks, int warps, cudaStream_t st);
 // cleft-parallel variants: 4 lanes per FRU, 8 FRUs per warp, `warps` warps
 // per block; FP64 (the plain method) and mixed precision (FP32 rates and
-// local ODE); `dense`: the build with fewer registers, for more warps than
+// local ODE); `fpw`: FRUs per warp (8, 4, 2 or 1; launches that advance);
+// `dense`: the build with fewer registers, for more warps than
 // kRoomyWarpsPerSm per SM
 constexpr int kRoomyWarpsPerSm = 11;
-cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, bool dense, cudaStream_t st);
-cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, bool dense, cudaStream_t st);
+cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, int fpw, bool dense, cudaStream_t st);
+cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, int fpw, bool dense, cudaStream_t st);
 // packed variants: `warps` single-warp blocks whose 4-lane groups take the
 // cell's FRUs from a queue (heaviest of the previous launch first); they
 // advance and store the FRUs only -- the sums come from a following

@@ -55,3 +55,22 @@ def test_substep_matches_oracle(gw, n, v, dv, ca, ms, packed):
     for k in ("ltype", "ryr", "ito2", "mti", "mt"):
         np.testing.assert_array_equal(got[k], s[k], err_msg=k)
     np.testing.assert_allclose(got["frus"], s["frus"], rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("n", [3, 9, 1216, 1217, 2427, 2433])
+def test_few_frus_per_warp_match_oracle(gw, n):
+    """Launches with 2, 4 and 8 FRUs per warp (by FRU count), whose groups are
+    summed by the warp that completes them; the sums over n FRUs of values
+    equal to 1e-12 are equal to 1e-12."""
+    s = random_set(n, 11 + n, (-4.0, -1.5))
+    cell = gw.Cell(n)
+    cell.upload(s)
+    d0, df = np.array([5.0, 3e-4, 0.5]), np.array([5.4, 3e-4, 0.49])
+    for t in (0.0, 0.02, 0.04):
+        _, num = cell.stage(t, t + 0.02, d0, df)
+        O.simfru(s, t, t + 0.02, d0, df)
+        np.testing.assert_allclose(num, O.flux_sums(s), rtol=1e-12)
+    got = cell.download()
+    for k in ("ltype", "ryr", "ito2", "mti", "mt"):
+        np.testing.assert_array_equal(got[k], s[k], err_msg=k)
+    np.testing.assert_allclose(got["frus"], s["frus"], rtol=1e-12, atol=0)
