@@ -18,10 +18,22 @@
 #include "gw_fru.h"
 
 #ifdef __CUDACC__
+#include "gw_fp64_math.cuh"
 #define GW_HD __host__ __device__ static inline
 #else
 #define GW_HD static inline
 #endif
+
+/* a / b; on the device with the FP64 quotient of three instructions
+ * (gw_fp64_math.cuh) where the operands are in its range: the 45 quotients
+ * of an evaluation were two thirds of its FP64 instructions. */
+GW_HD double gw_div(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return gw::checked_div(a, b);
+#else
+  return a / b;
+#endif
+}
 
 /* state indices (indices.h:5-41) */
 enum {
@@ -183,7 +195,7 @@ GW_HD double gw_x_arg(int k, double V) {
   const int f = gw_x_form(k, &d, &c, &e);
   double t = (f & GW_XF_V) ? V : 0.0;
   if (f & GW_XF_ADD) t = t + d;
-  t = (f & GW_XF_DIV) ? t / c : t * c;
+  t = (f & GW_XF_DIV) ? gw_div(t, c) : t * c;
   if (f & GW_XF_MUL2) t = t * e;
   return t;
 }
@@ -195,19 +207,19 @@ GW_HD double gw_cai_clamped(const double* state) { return state[GW_Cai] <= 0.0 ?
 GW_HD double gw_lg_arg(int k, const double* state) {
   const double Nai = state[GW_Nai], Ki = state[GW_Ki];
   switch (k) {
-    case 0: return GWC_Nao / Nai;
-    case 1: return GWC_Ko / Ki;
-    case 2: return (GWC_Ko + 0.01833 * GWC_Nao) / (Ki + 0.01833 * Nai);
-    default: return GWC_Cao / gw_cai_clamped(state);
+    case 0: return gw_div(GWC_Nao, Nai);
+    case 1: return gw_div(GWC_Ko, Ki);
+    case 2: return gw_div(GWC_Ko + 0.01833 * GWC_Nao, Ki + 0.01833 * Nai);
+    default: return gw_div(GWC_Cao, gw_cai_clamped(state));
   }
 }
 GW_HD double gw_pw_arg(int k, const double* state, double* y) {
   const double Cai = gw_cai_clamped(state);
   switch (k) {
     case 0: *y = 0.5; return GWC_Ko / 4.0;
-    case 1: *y = 1.5; return 10.0 / state[GW_Nai];            /* KmNai / Nai */
-    case 2: *y = 0.75; return Cai / 0.26e-3;                   /* Cai / Kfb, Nfb */
-    case 3: *y = 0.75; return state[GW_CaNSR] / 1.8;           /* CaNSR / Krb, Nrb */
+    case 1: *y = 1.5; return gw_div(10.0, state[GW_Nai]);            /* KmNai / Nai */
+    case 2: *y = 0.75; return gw_div(Cai, 0.26e-3);                   /* Cai / Kfb, Nfb */
+    case 3: *y = 0.75; return gw_div(state[GW_CaNSR], 1.8);           /* CaNSR / Krb, Nrb */
     case 4: *y = 2.0; return Cai + GWC_KmCMDN;
     default: *y = 2.0; return Cai + GWC_KmEGTA;
   }
@@ -216,6 +228,92 @@ GW_HD double gw_pw_arg(int k, const double* state, double* y) {
 GW_HD double gw_k1_arg(double V, const double* tx_lg) {
   const double EK = GWC_RT_over_F * tx_lg[1];
   return 1.76 / GWC_RT_over_F * (V - EK);
+}
+
+/* ---- Kv4.3 and Kv1.4, fcn.c:846-917, :927-998 ---------------------------------
+ * One model with two sets of constants: f1..f4, b1..b4; al, be, ali, bei the
+ * activation and inactivation rates; s = C0..C3, O, CI0..CI3, OI; d = the
+ * derivatives of the first nine. */
+typedef struct gw_kv {
+  double f1, f2, f3, f4, b1, b2, b3, b4, al, be, ali, bei, s[10];
+} gw_kv;
+
+GW_HD void gw_kv_model(const gw_kv* m, double d[9]) {
+  const double al = m->al, be = m->be, ali = m->ali, bei = m->bei;
+  const double f1 = m->f1, f2 = m->f2, f3 = m->f3, f4 = m->f4, b1 = m->b1, b2 = m->b2, b3 = m->b3, b4 = m->b4;
+  const double C0 = m->s[0], C1 = m->s[1], C2 = m->s[2], C3 = m->s[3], O = m->s[4];
+  const double CI0 = m->s[5], CI1 = m->s[6], CI2 = m->s[7], CI3 = m->s[8], OI = m->s[9];
+  const double C0C1 = 4.0 * al, C1C2 = 3.0 * al, C2C3 = 2.0 * al, C3O = al;
+  const double CI0CI1 = 4.0 * b1 * al, CI1CI2 = gw_div(3.0 * b2 * al, b1);
+  const double CI2CI3 = gw_div(2.0 * b3 * al, b2), CI3OI = gw_div(b4 * al, b3);
+  const double C1C0 = be, C2C1 = 2.0 * be, C3C2 = 3.0 * be, OC3 = 4.0 * be;
+  const double CI1CI0 = gw_div(be, f1), CI2CI1 = gw_div(2.0 * f1 * be, f2);
+  const double CI3CI2 = gw_div(3.0 * f2 * be, f3), OICI3 = gw_div(4.0 * f3 * be, f4);
+  const double C0CI0 = bei, C1CI1 = f1 * bei, C2CI2 = f2 * bei, C3CI3 = f3 * bei, OOI = f4 * bei;
+  const double CI0C0 = ali, CI1C1 = gw_div(ali, b1), CI2C2 = gw_div(ali, b2), CI3C3 = gw_div(ali, b3),
+               OIO = gw_div(ali, b4);
+  double a1, a2;
+  a1 = (C0C1 + C0CI0) * C0; a2 = C1C0 * C1 + CI0C0 * CI0; d[0] = a2 - a1;
+  a1 = (C1C2 + C1C0 + C1CI1) * C1; a2 = C2C1 * C2 + CI1C1 * CI1 + C0C1 * C0; d[1] = a2 - a1;
+  a1 = (C2C3 + C2C1 + C2CI2) * C2; a2 = C3C2 * C3 + CI2C2 * CI2 + C1C2 * C1; d[2] = a2 - a1;
+  a1 = (C3O + C3C2 + C3CI3) * C3; a2 = OC3 * O + CI3C3 * CI3 + C2C3 * C2; d[3] = a2 - a1;
+  a1 = (OC3 + OOI) * O; a2 = C3O * C3 + OIO * OI; d[4] = a2 - a1;
+  a1 = (CI0C0 + CI0CI1) * CI0; a2 = C0CI0 * C0 + CI1CI0 * CI1; d[5] = a2 - a1;
+  a1 = (CI1CI2 + CI1C1 + CI1CI0) * CI1; a2 = CI2CI1 * CI2 + C1CI1 * C1 + CI0CI1 * CI0;
+  d[6] = a2 - a1;
+  a1 = (CI2CI3 + CI2C2 + CI2CI1) * CI2; a2 = CI3CI2 * CI3 + C2CI2 * C2 + CI1CI2 * CI1;
+  d[7] = a2 - a1;
+  a1 = (CI3OI + CI3C3 + CI3CI2) * CI3; a2 = OICI3 * OI + C3CI3 * C3 + CI2CI3 * CI2;
+  d[8] = a2 - a1;
+}
+
+/* one set of inputs: Kv1.4 when which != 0, else Kv4.3 (OI: the channel's
+ * remaining state) */
+GW_HD void gw_kv_inputs(int which, const double* state, const gw_tx* tx, double OI, gw_kv* m) {
+  int k;
+  m->f1 = which ? 0.20005 : 1.8936; m->f2 = which ? 0.320280 : 14.224647456;
+  m->f3 = which ? 13.50909223 : 158.574378389; m->f4 = which ? 1151.7651385 : 142.936645351;
+  m->b1 = which ? 2.2300 : 6.77348; m->b2 = which ? 12.000299 : 15.6212705152;
+  m->b3 = which ? 5.3701338025 : 28.7532603313; m->b4 = which ? 5.2396395511 : 524.576206679;
+  m->al = (which ? 6.0 * 0.31551 : 0.543708) * (which ? tx->x[GW_X_14A] : tx->x[GW_X_43A]);
+  m->be = (which ? 6.0 * 0.001966 : 0.080185) * (which ? tx->x[GW_X_14B] : tx->x[GW_X_43B]);
+  m->ali = which ? 6.0 * 0.0004938 : 0.0498424 * tx->x[GW_X_43C];
+  m->bei = which ? 6.0 * 0.0000176 : 0.000819482 * tx->x[GW_X_43D];
+  for (k = 0; k < 9; k++) m->s[k] = which ? state[GW_C0Kv14 + k] : state[GW_C0Kv43 + k];
+  m->s[9] = OI;
+}
+
+/* both channels' derivatives into F; lane >= 0: on a whole warp, Kv4.3 on
+ * the even lanes and Kv1.4 on the odd ones */
+GW_HD void gw_kv_both(const double* state, const gw_tx* tx, double OI43, double OI14, double* F, int lane) {
+  double d[2][9];
+  int c, k;
+#ifdef __CUDA_ARCH__
+  if (lane >= 0) {
+    gw_kv m;
+    double mine[9];
+    gw_kv_inputs(lane & 1, state, tx, (lane & 1) ? OI14 : OI43, &m);
+    gw_kv_model(&m, mine);
+    for (k = 0; k < 9; k++) {
+      d[0][k] = __shfl_sync(0xffffffffu, mine[k], 0);
+      d[1][k] = __shfl_sync(0xffffffffu, mine[k], 1);
+    }
+  } else
+#endif
+  {
+    for (c = 0; c < 2; c++) {
+      gw_kv m;
+      gw_kv_inputs(c, state, tx, c ? OI14 : OI43, &m);
+      gw_kv_model(&m, d[c]);
+    }
+  }
+  (void)lane;
+  for (c = 0; c < 2; c++) {
+    const double* e = d[c];
+    double* f = F + (c ? GW_C0Kv14 : GW_C0Kv43);
+    for (k = 0; k < 9; k++) f[k] = e[k];
+    f[9] = -e[5] - e[6] - e[7] - e[8] - e[4] - e[0] - e[1] - e[2] - e[3];
+  }
 }
 
 /* Membrane potential of fcn.c:434-535: the state's V, or the clamp level of
@@ -267,10 +365,11 @@ GW_HD double gw_fcn_voltage(const double time, const double* state, const gw_pro
 /* Global right-hand side (fcn.c:29-1072) given its transcendental terms
  * (gw_tx, filled for this state and time).  May overwrite state[GW_mNa]
  * (V < -90 mV steady state) and state[GW_V] (clamp modes) in place, as the
- * reference does.  current[] is filled when keepc != 0. */
+ * reference does.  current[] is filled when keepc != 0.  lane: -1, or the
+ * lane of a GPU warp whose 32 lanes call it together with the same values. */
 GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* current, const int keepc,
                      const double Jxfer, const double Jtr, const double ICa, const double Ito2, const gw_protocol* P,
-                     const gw_tx* tx) {
+                     const gw_tx* tx, const int lane) {
   /* membrane current parameters, fcn.c:169-264 */
   const double GKr = 0.029 * P->scale_GKr, GKs = 0.035, GK1 = 3.0, GKp = 1.2 * 0.002216, GNa = 12.8;
   /* eta, KmNai, Kfb, Krb, Nfb, Nrb and the exponents' rate constants enter
@@ -283,14 +382,6 @@ GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* curren
   const double KvScale = 1.13 * 1.03 * 1.55, Kv43Frac = 0.77;
   const double GKv43 = Kv43Frac * KvScale * 0.1;
   const double PKv14 = (1.0 - Kv43Frac) * KvScale * 4.792933e-7;
-  const double alphaa0Kv43 = 0.543708, betaa0Kv43 = 0.080185;
-  const double alphai0Kv43 = 0.0498424, betai0Kv43 = 0.000819482;
-  const double alphaa0Kv14 = 6.0 * 0.31551, betaa0Kv14 = 6.0 * 0.001966;
-  const double alphai0Kv14 = 6.0 * 0.0004938, betai0Kv14 = 6.0 * 0.0000176;
-  const double f1Kv43 = 1.8936, f2Kv43 = 14.224647456, f3Kv43 = 158.574378389, f4Kv43 = 142.936645351;
-  const double b1Kv43 = 6.77348, b2Kv43 = 15.6212705152, b3Kv43 = 28.7532603313, b4Kv43 = 524.576206679;
-  const double f1Kv14 = 0.20005, f2Kv14 = 0.320280, f3Kv14 = 13.50909223, f4Kv14 = 1151.7651385;
-  const double b1Kv14 = 2.2300, b2Kv14 = 12.000299, b3Kv14 = 5.3701338025, b4Kv14 = 5.2396395511;
   const double T_Const_HERG = 5.320000001;
   const double A0_HERG = 0.017147641733086, A1_HERG = 0.03969328381141, A2_HERG = 0.02057448605977;
   const double A3_HERG = 0.00134366604423, A4_HERG = 0.10666316491288, A5_HERG = 0.00646393910049;
@@ -333,43 +424,42 @@ GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* curren
   const double IKr = GKr * fKo * OHerg * (V - EK);
   const double IKs = GKs * (xKs * xKs) * (V - EKs);
   double IKv43 = GKv43 * OKv43 * (V - EK);
-  double VF_over_RT = V / RT_over_F;
+  const double VF_over_RT = gw_div(V, RT_over_F);
   const double VFsq_over_RT = (1000.0 * Faraday) * VF_over_RT;
   const double exp_VFRT = tx->x[GW_X_VFRT];
   double IKv14_K, IKv14_Na;
   a1 = Ki * exp_VFRT - Ko;
   a2 = exp_VFRT - 1.0;
   if (fabs(V) < 1.e-6) IKv14_K = PKv14 * OKv14 * 1000.0 * Faraday * (Ki - Ko);
-  else IKv14_K = PKv14 * OKv14 * VFsq_over_RT * (a1 / a2);
+  else IKv14_K = PKv14 * OKv14 * VFsq_over_RT * gw_div(a1, a2);
   a1 = Nai * exp_VFRT - Nao;
   if (fabs(V) < 1.e-6) IKv14_Na = 0.02 * PKv14 * OKv14 * 1000.0 * Faraday * (Nai - Nao);
-  else IKv14_Na = 0.02 * PKv14 * OKv14 * VFsq_over_RT * (a1 / a2);
+  else IKv14_Na = 0.02 * PKv14 * OKv14 * VFsq_over_RT * gw_div(a1, a2);
   const double IKv14 = IKv14_K + IKv14_Na;
   double Ito1 = IKv43 + IKv14;
-  const double K1_inf = 1.0 / (0.94 + tx->k1);
+  const double K1_inf = gw_div(1.0, 0.94 + tx->k1);
   double IK1 = GK1 * Ko / (Ko + KmK1) * K1_inf * (V - EK);
   const double INab = GNab * (V - ENa);
-  const double KpV = 1.0 / (1.0 + tx->x[GW_X_KPV]);
+  const double KpV = gw_div(1.0, 1.0 + tx->x[GW_X_KPV]);
   const double IKp = GKp * KpV * (V - EK);
 
   /* ---- INaK, INaCa, ICab, IpCa, fcn.c:623-649 ---- */
-  VF_over_RT = V / RT_over_F;
-  const double sigma = (tx->x[GW_X_SIGMA] - 1.0) / 7.0;
+  const double sigma = gw_div(tx->x[GW_X_SIGMA] - 1.0, 7.0);
   a1 = 1.0 + 0.1245 * tx->x[GW_X_NAK];
-  a2 = 0.0365 * sigma / exp_VFRT;
-  const double fNaK = 1.0 / (a1 + a2);
+  a2 = gw_div(0.0365 * sigma, exp_VFRT);
+  const double fNaK = gw_div(1.0, a1 + a2);
   a1 = Ko / (Ko + KmKo);
   a2 = 1.0 + tx->pw[1];
-  const double INaK = INaKmax * fNaK * (a1 / a2);
+  const double INaK = INaKmax * fNaK * gw_div(a1, a2);
   const double exp_etaVFRT = tx->x[GW_X_ETA];
   a1 = exp_etaVFRT * (Nai * Nai * Nai) * Cao;
-  a2 = exp_etaVFRT / exp_VFRT * (Nao * Nao * Nao) * Cai;
-  a3 = 1.0 + ksat * exp_etaVFRT / exp_VFRT;
+  a2 = gw_div(exp_etaVFRT, exp_VFRT) * (Nao * Nao * Nao) * Cai;
+  a3 = 1.0 + gw_div(ksat * exp_etaVFRT, exp_VFRT);
   a4 = KmCa + Cao;
   a5 = 5000.0 / (KmNa * KmNa * KmNa + Nao * Nao * Nao);
-  double INaCa = kNaCa * a5 * (a1 - a2) / (a4 * a3);
+  double INaCa = gw_div(kNaCa * a5 * (a1 - a2), a4 * a3);
   const double ICab = GCab * (V - ECa);
-  const double IpCa = IpCamax * Cai / (KmpCa + Cai);
+  const double IpCa = gw_div(IpCamax * Cai, KmpCa + Cai);
 
   /* ---- gating derivatives, fcn.c:654-755 ---- */
   double alpha_m, dmNa;
@@ -377,30 +467,30 @@ GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* curren
     alpha_m = 0.32 / (0.1 - 0.005 * (V + 47.13));
   } else {
     a1 = 0.32 * (V + 47.13);
-    alpha_m = a1 / (1.0 - tx->x[GW_X_AM]);
+    alpha_m = gw_div(a1, 1.0 - tx->x[GW_X_AM]);
   }
   const double beta_m = 0.08 * tx->x[GW_X_BM];
   if (V >= -90.0) {
     dmNa = alpha_m * (1.0 - mNa) - beta_m * mNa;
   } else {
     dmNa = 0.0;
-    mNa = alpha_m / (alpha_m + beta_m);
+    mNa = gw_div(alpha_m, alpha_m + beta_m);
     state[GW_mNa] = mNa;
   }
   const double alpha_h = 0.135 * tx->x[GW_X_AH];
   double beta_h, alpha_j, beta_j;
   if (V < -38.73809636838782) beta_h = 3.56 * tx->x[GW_X_BH1] + 310000 * tx->x[GW_X_BH2];
-  else beta_h = 1 / (0.13 * (1 + tx->x[GW_X_BH3]));
+  else beta_h = gw_div(1, 0.13 * (1 + tx->x[GW_X_BH3]));
   if (V < -37.78) {
     a1 = -127140 * tx->x[GW_X_AJ1];
     a2 = 3.474E-5 * tx->x[GW_X_AJ2];
     a3 = 1.0 + tx->x[GW_X_AJ3];
-    alpha_j = (a1 - a2) * (V + 37.78) / a3;
+    alpha_j = gw_div((a1 - a2) * (V + 37.78), a3);
   } else {
     alpha_j = 0;
   }
-  if (V < -39.82600037702883) beta_j = 0.1212 * tx->x[GW_X_BJ1] / (1.0 + tx->x[GW_X_BJ2]);
-  else beta_j = 0.3 * tx->x[GW_X_BJ3] / (1 + tx->x[GW_X_BJ4]);
+  if (V < -39.82600037702883) beta_j = gw_div(0.1212 * tx->x[GW_X_BJ1], 1.0 + tx->x[GW_X_BJ2]);
+  else beta_j = gw_div(0.3 * tx->x[GW_X_BJ3], 1 + tx->x[GW_X_BJ4]);
   const double dhNa = alpha_h * (1.0 - hNa) - beta_h * hNa;
   const double djNa = alpha_j * (1.0 - jNa) - beta_j * jNa;
 
@@ -412,7 +502,7 @@ GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* curren
   const double OH_to_IH = T_Const_HERG * A4_HERG * tx->x[GW_X_H4];
   const double IH_to_OH = T_Const_HERG * A5_HERG * tx->x[GW_X_H5];
   const double C3H_to_IH = T_Const_HERG * A6_HERG * tx->x[GW_X_H6];
-  const double IH_to_C3H = (OH_to_C3H * IH_to_OH * C3H_to_IH) / (C3H_to_OH * OH_to_IH);
+  const double IH_to_C3H = gw_div(OH_to_C3H * IH_to_OH * C3H_to_IH, C3H_to_OH * OH_to_IH);
   const double dC1Herg = C2H_to_C1H * C2Herg - C1H_to_C2H * C1Herg;
   a1 = C1H_to_C2H * C1Herg + C3H_to_C2H * C3Herg;
   a2 = (C2H_to_C1H + C2H_to_C3H) * C2Herg;
@@ -425,29 +515,29 @@ GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* curren
   const double dOHerg = a1 - a2;
 
   /* IKs */
-  const double xKs_inf = 1.0 / (1.0 + tx->x[GW_X_XKS]);
+  const double xKs_inf = gw_div(1.0, 1.0 + tx->x[GW_X_XKS]);
   if (fabs(V - 10) < 1.e-6) {
     a1 = (7.19e-5) / 0.148;
     a2 = (1.31e-4) / 0.0687;
   } else {
-    a1 = 7.19e-5 * (V - 10.0) / (1.0 - tx->x[GW_X_KS1]);
-    a2 = 1.31e-4 * (V - 10.0) / (tx->x[GW_X_KS2] - 1.0);
+    a1 = gw_div(7.19e-5 * (V - 10.0), 1.0 - tx->x[GW_X_KS1]);
+    a2 = gw_div(1.31e-4 * (V - 10.0), tx->x[GW_X_KS2] - 1.0);
   }
-  const double tau_xKs = 1.0 / (a1 + a2);
-  const double dxKs = (xKs_inf - xKs) / tau_xKs;
+  const double tau_xKs = gw_div(1.0, a1 + a2);
+  const double dxKs = gw_div(xKs_inf - xKs, tau_xKs);
 
   /* ---- SR uptake and troponin, fcn.c:759-776 ---- */
   const double fb = tx->pw[2];
   const double rb = tx->pw[3];
-  double Jup = KSR * (vmaxf * fb - vmaxr * rb) / (1.0 + fb + rb);
+  double Jup = gw_div(KSR * (vmaxf * fb - vmaxr * rb), 1.0 + fb + rb);
   a1 = GWC_kltrpn_minus * LTRPNCa;
   const double dLTRPNCa = GWC_kltrpn_plus * Cai * (1.0 - LTRPNCa) - a1;
   a1 = GWC_khtrpn_minus * HTRPNCa;
   const double dHTRPNCa = GWC_khtrpn_plus * Cai * (1.0 - HTRPNCa) - a1;
   const double Jtrpn = GWC_LTRPNtot * dLTRPNCa + GWC_HTRPNtot * dHTRPNCa;
-  a1 = GWC_CMDNtot * GWC_KmCMDN / (tx->pw[4]);
-  a2 = GWC_EGTAtot * GWC_KmEGTA / (tx->pw[5]);
-  const double beta_i = 1.0 / (1.0 + a1 + a2);
+  a1 = gw_div(GWC_CMDNtot * GWC_KmCMDN, tx->pw[4]);
+  a2 = gw_div(GWC_EGTAtot * GWC_KmEGTA, tx->pw[5]);
+  const double beta_i = gw_div(1.0, 1.0 + a1 + a2);
 
   /* ---- heart-failure scalings, fcn.c:780-786 ---- */
   if (P->chf_flag) {
@@ -464,8 +554,8 @@ GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* curren
   a3 = IKr + IKs + IK1 + IKp;
   const double dKi = -(a3 - 2.0 * INaK + (Ito1 - IKv14_Na) + Istim) * a1;
   a3 = ICab - 2.0 * INaCa + IpCa;
-  const double dCai = beta_i * (Jxfer * VSS / Vmyo - Jup - Jtrpn - a3 * 0.5 * a1);
-  const double dCaNSR = Jup * Vmyo / VNSR - Jtr * VJSR / VNSR;
+  const double dCai = beta_i * (gw_div(Jxfer * VSS, Vmyo) - Jup - Jtrpn - a3 * 0.5 * a1);
+  const double dCaNSR = gw_div(Jup * Vmyo, VNSR) - gw_div(Jtr * VJSR, VNSR);
   const double dCaTOT = -(a3 + ICa) * 0.5 * a1 * Vmyo * 1.0e6;
   a1 = INa + ICa + IKr + IKs;
   a2 = IK1 + IKp + INaCa + INaK + Ito1 + Ito2;
@@ -485,64 +575,8 @@ GW_HD void gw_fcn_tx(const double time, double* state, double* F, double* curren
     Itot = a1 + a2 + a3;
   }
 
-  /* ---- Kv4.3, fcn.c:846-917 ---- */
-  {
-    const double al = alphaa0Kv43 * tx->x[GW_X_43A], be = betaa0Kv43 * tx->x[GW_X_43B];
-    const double ali = alphai0Kv43 * tx->x[GW_X_43C], bei = betai0Kv43 * tx->x[GW_X_43D];
-    const double C0C1 = 4.0 * al, C1C2 = 3.0 * al, C2C3 = 2.0 * al, C3O = al;
-    const double CI0CI1 = 4.0 * b1Kv43 * al, CI1CI2 = 3.0 * b2Kv43 * al / b1Kv43;
-    const double CI2CI3 = 2.0 * b3Kv43 * al / b2Kv43, CI3OI = b4Kv43 * al / b3Kv43;
-    const double C1C0 = be, C2C1 = 2.0 * be, C3C2 = 3.0 * be, OC3 = 4.0 * be;
-    const double CI1CI0 = be / f1Kv43, CI2CI1 = 2.0 * f1Kv43 * be / f2Kv43;
-    const double CI3CI2 = 3.0 * f2Kv43 * be / f3Kv43, OICI3 = 4.0 * f3Kv43 * be / f4Kv43;
-    const double C0CI0 = bei, C1CI1 = f1Kv43 * bei, C2CI2 = f2Kv43 * bei, C3CI3 = f3Kv43 * bei, OOI = f4Kv43 * bei;
-    const double CI0C0 = ali, CI1C1 = ali / b1Kv43, CI2C2 = ali / b2Kv43, CI3C3 = ali / b3Kv43, OIO = ali / b4Kv43;
-    double d[9];
-    a1 = (C0C1 + C0CI0) * C0Kv43; a2 = C1C0 * C1Kv43 + CI0C0 * CI0Kv43; d[0] = a2 - a1;
-    a1 = (C1C2 + C1C0 + C1CI1) * C1Kv43; a2 = C2C1 * C2Kv43 + CI1C1 * CI1Kv43 + C0C1 * C0Kv43; d[1] = a2 - a1;
-    a1 = (C2C3 + C2C1 + C2CI2) * C2Kv43; a2 = C3C2 * C3Kv43 + CI2C2 * CI2Kv43 + C1C2 * C1Kv43; d[2] = a2 - a1;
-    a1 = (C3O + C3C2 + C3CI3) * C3Kv43; a2 = OC3 * OKv43 + CI3C3 * CI3Kv43 + C2C3 * C2Kv43; d[3] = a2 - a1;
-    a1 = (OC3 + OOI) * OKv43; a2 = C3O * C3Kv43 + OIO * OIKv43; d[4] = a2 - a1;
-    a1 = (CI0C0 + CI0CI1) * CI0Kv43; a2 = C0CI0 * C0Kv43 + CI1CI0 * CI1Kv43; d[5] = a2 - a1;
-    a1 = (CI1CI2 + CI1C1 + CI1CI0) * CI1Kv43; a2 = CI2CI1 * CI2Kv43 + C1CI1 * C1Kv43 + CI0CI1 * CI0Kv43;
-    d[6] = a2 - a1;
-    a1 = (CI2CI3 + CI2C2 + CI2CI1) * CI2Kv43; a2 = CI3CI2 * CI3Kv43 + C2CI2 * C2Kv43 + CI1CI2 * CI1Kv43;
-    d[7] = a2 - a1;
-    a1 = (CI3OI + CI3C3 + CI3CI2) * CI3Kv43; a2 = OICI3 * OIKv43 + C3CI3 * C3Kv43 + CI2CI3 * CI2Kv43;
-    d[8] = a2 - a1;
-    F[GW_C0Kv43] = d[0]; F[GW_C1Kv43] = d[1]; F[GW_C2Kv43] = d[2]; F[GW_C3Kv43] = d[3]; F[GW_OKv43] = d[4];
-    F[GW_CI0Kv43] = d[5]; F[GW_CI1Kv43] = d[6]; F[GW_CI2Kv43] = d[7]; F[GW_CI3Kv43] = d[8];
-    F[GW_OIKv43] = -d[5] - d[6] - d[7] - d[8] - d[4] - d[0] - d[1] - d[2] - d[3];
-  }
-  /* ---- Kv1.4, fcn.c:927-998 ---- */
-  {
-    const double al = alphaa0Kv14 * tx->x[GW_X_14A], be = betaa0Kv14 * tx->x[GW_X_14B];
-    const double ali = alphai0Kv14, bei = betai0Kv14;
-    const double C0C1 = 4.0 * al, C1C2 = 3.0 * al, C2C3 = 2.0 * al, C3O = al;
-    const double CI0CI1 = 4.0 * b1Kv14 * al, CI1CI2 = 3.0 * b2Kv14 * al / b1Kv14;
-    const double CI2CI3 = 2.0 * b3Kv14 * al / b2Kv14, CI3OI = b4Kv14 * al / b3Kv14;
-    const double C1C0 = be, C2C1 = 2.0 * be, C3C2 = 3.0 * be, OC3 = 4.0 * be;
-    const double CI1CI0 = be / f1Kv14, CI2CI1 = 2.0 * f1Kv14 * be / f2Kv14;
-    const double CI3CI2 = 3.0 * f2Kv14 * be / f3Kv14, OICI3 = 4.0 * f3Kv14 * be / f4Kv14;
-    const double C0CI0 = bei, C1CI1 = f1Kv14 * bei, C2CI2 = f2Kv14 * bei, C3CI3 = f3Kv14 * bei, OOI = f4Kv14 * bei;
-    const double CI0C0 = ali, CI1C1 = ali / b1Kv14, CI2C2 = ali / b2Kv14, CI3C3 = ali / b3Kv14, OIO = ali / b4Kv14;
-    double d[9];
-    a1 = (C0C1 + C0CI0) * C0Kv14; a2 = C1C0 * C1Kv14 + CI0C0 * CI0Kv14; d[0] = a2 - a1;
-    a1 = (C1C2 + C1C0 + C1CI1) * C1Kv14; a2 = C2C1 * C2Kv14 + CI1C1 * CI1Kv14 + C0C1 * C0Kv14; d[1] = a2 - a1;
-    a1 = (C2C3 + C2C1 + C2CI2) * C2Kv14; a2 = C3C2 * C3Kv14 + CI2C2 * CI2Kv14 + C1C2 * C1Kv14; d[2] = a2 - a1;
-    a1 = (C3O + C3C2 + C3CI3) * C3Kv14; a2 = OC3 * OKv14 + CI3C3 * CI3Kv14 + C2C3 * C2Kv14; d[3] = a2 - a1;
-    a1 = (OC3 + OOI) * OKv14; a2 = C3O * C3Kv14 + OIO * OIKv14; d[4] = a2 - a1;
-    a1 = (CI0C0 + CI0CI1) * CI0Kv14; a2 = C0CI0 * C0Kv14 + CI1CI0 * CI1Kv14; d[5] = a2 - a1;
-    a1 = (CI1CI2 + CI1C1 + CI1CI0) * CI1Kv14; a2 = CI2CI1 * CI2Kv14 + C1CI1 * C1Kv14 + CI0CI1 * CI0Kv14;
-    d[6] = a2 - a1;
-    a1 = (CI2CI3 + CI2C2 + CI2CI1) * CI2Kv14; a2 = CI3CI2 * CI3Kv14 + C2CI2 * C2Kv14 + CI1CI2 * CI1Kv14;
-    d[7] = a2 - a1;
-    a1 = (CI3OI + CI3C3 + CI3CI2) * CI3Kv14; a2 = OICI3 * OIKv14 + C3CI3 * C3Kv14 + CI2CI3 * CI2Kv14;
-    d[8] = a2 - a1;
-    F[GW_C0Kv14] = d[0]; F[GW_C1Kv14] = d[1]; F[GW_C2Kv14] = d[2]; F[GW_C3Kv14] = d[3]; F[GW_OKv14] = d[4];
-    F[GW_CI0Kv14] = d[5]; F[GW_CI1Kv14] = d[6]; F[GW_CI2Kv14] = d[7]; F[GW_CI3Kv14] = d[8];
-    F[GW_OIKv14] = -d[5] - d[6] - d[7] - d[8] - d[4] - d[0] - d[1] - d[2] - d[3];
-  }
+  /* ---- Kv4.3 and Kv1.4, fcn.c:846-917, :927-998 ---- */
+  gw_kv_both(state, tx, OIKv43, OIKv14, F, lane);
 
   F[GW_V] = dV; F[GW_mNa] = dmNa; F[GW_hNa] = dhNa; F[GW_jNa] = djNa; F[GW_Nai] = dNai; F[GW_Ki] = dKi;
   F[GW_Cai] = dCai; F[GW_CaNSR] = dCaNSR; F[GW_xKs] = dxKs; F[GW_LTRPNCa] = dLTRPNCa; F[GW_HTRPNCa] = dHTRPNCa;
@@ -584,7 +618,7 @@ GW_HD void gw_fcn(const double time, double* state, double* F, double* current, 
                   const double Jxfer, const double Jtr, const double ICa, const double Ito2, const gw_protocol* P) {
   gw_tx tx;
   gw_tx_fill(time, state, P, &tx);
-  gw_fcn_tx(time, state, F, current, keepc, Jxfer, Jtr, ICa, Ito2, P, &tx);
+  gw_fcn_tx(time, state, F, current, keepc, Jxfer, Jtr, ICa, Ito2, P, &tx, -1);
 }
 
 /* Rest state of initialize_state.c:167-203 (37 globals). */

@@ -4,7 +4,7 @@
 //
 // A DpCell holds the integrator's state (y, k1..k5, the trial state,
 // start/step/ostep, the accept/reject state) and the parameters of the cell's
-// next FRU launch; dp_after advances it after one FRU launch exactly as the
+// next FRU launch; dp_after_warp advances it after one FRU launch exactly as the
 // host integrator (gw_dp.c) does, operation for operation (compiled with
 // -fmad=false), and sets up the next launch.
 #pragma once
@@ -68,20 +68,6 @@ static __device__ inline void launch_flux(DpCell& c, bool avg) {
   if (avg) c.sp.flags |= kFlagAvg;
 }
 
-// stage 2 (node 1/5) from F1 and the current step (rk_pd54m.c:121-127)
-static __device__ inline void launch_stage2(DpCell& c) {
-  double* k1 = c.k[0];
-  for (int i = 0; i < GW_NSTATE; i++) {
-    k1[i] = c.step * c.F1[i];
-    c.y1[i] = c.y[i] + k1[i] / 5.0;
-  }
-  double depf[3];
-  dep_of(c.y, c.dep0);
-  dep_of(c.y1, depf);
-  set_launch(c, c.start, c.start + c.step / 5.0, c.dep0, depf, 1);
-  c.phase = kPhS2;
-}
-
 // the start of an output step (gw_rk54pd's preamble)
 static __device__ inline void begin_output_step(DpCell& c) {
   c.tstep = c.tnow + c.set.time_step;
@@ -94,185 +80,16 @@ static __device__ inline void begin_output_step(DpCell& c) {
   c.keepc = 1;
 }
 
-// The integrator after one FRU launch of the cell; J = (Jxfer, Jtr, ICa,
-// Ito2) at the launch's end point; avg = the output-average sums when the
-// launch carried them.
-static __device__ __noinline__ void dp_after(DpCell& c, const double J[4], const double* avg) {
-  double F[GW_NSTATE], dummy[GW_NCUR];
-  const double step = c.step, start = c.start;
-  double* k1 = c.k[0];
-  double* k2 = c.k[1];
-  double* k3 = c.k[2];
-  double* k4 = c.k[3];
-  double* k5 = c.k[4];
-  if (c.phase == kPhFlux) {
-    if (avg && c.step_index > 0 && c.tr_other)
-      gw_otherstates(avg, c.nfru, 12500.0 / (double)c.nfru, c.y, c.tr_other + (size_t)(c.step_index - 1) * GW_NOTHER);
-    if (c.final_avg) {
-      c.done = 1;
-      return;
-    }
-    gw_fcn(start, c.y, c.F1, c.cur, c.keepc, J[0], J[1], J[2], J[3], &c.set);
-    c.keepc = 0;
-    c.epoch++;  // gw_save: a new snapshot epoch, folded into the next launch
-    c.pending = kFlagSave;
-    launch_stage2(c);
-    return;
-  }
-  double depf[3];
-  switch (c.phase) {
-    case kPhS2:
-      gw_fcn(start + step / 5.0, c.y1, F, dummy, 0, J[0], J[1], J[2], J[3], &c.set);
-      for (int i = 0; i < GW_NSTATE; i++) {
-        k2[i] = step * F[i];
-        c.y1[i] = c.y[i] + (3.0 / 40.0 * k1[i] + 9.0 / 40.0 * k2[i]);
-      }
-      dep_of(c.y1, depf);
-      set_launch(c, start + step / 5.0, start + step * 3.0 / 10.0, c.dep0, depf, 1);
-      c.phase = kPhS3;
-      return;
-    case kPhS3:
-      gw_fcn(start + step * 3.0 / 10.0, c.y1, F, dummy, 0, J[0], J[1], J[2], J[3], &c.set);
-      for (int i = 0; i < GW_NSTATE; i++) {
-        k3[i] = step * F[i];
-        c.y1[i] = c.y[i] + (3.0 / 10.0 * k1[i] - 9.0 / 10.0 * k2[i] + 6.0 / 5.0 * k3[i]);
-      }
-      dep_of(c.y1, depf);
-      set_launch(c, start + step * 3.0 / 10.0, start + step * 3.0 / 5.0, c.dep0, depf, 1);
-      c.phase = kPhS4;
-      return;
-    case kPhS4:
-      gw_fcn(start + step * 3.0 / 5.0, c.y1, F, dummy, 0, J[0], J[1], J[2], J[3], &c.set);
-      for (int i = 0; i < GW_NSTATE; i++) {
-        k4[i] = F[i] * step;
-        c.y1[i] = c.y[i] + 226.0 / 729.0 * k1[i] - 25.0 / 27.0 * k2[i] + 880.0 / 729.0 * k3[i] +
-                  55.0 / 729.0 * k4[i];
-      }
-      dep_of(c.y1, depf);
-      set_launch(c, start + step * 3.0 / 5.0, start + step * 2.0 / 3.0, c.dep0, depf, 1);
-      c.phase = kPhS5;
-      return;
-    case kPhS5:
-      gw_fcn(start + step * 2.0 / 3.0, c.y1, F, dummy, 0, J[0], J[1], J[2], J[3], &c.set);
-      for (int i = 0; i < GW_NSTATE; i++) {
-        k5[i] = step * F[i];
-        c.y1[i] = c.y[i] - 181.0 / 270.0 * k1[i] + 5.0 / 2.0 * k2[i] - 266.0 / 297.0 * k3[i] -
-                  91.0 / 27.0 * k4[i] + 189.0 / 55.0 * k5[i];
-      }
-      dep_of(c.y1, depf);
-      set_launch(c, start + step * 2.0 / 3.0, start + step, c.dep0, depf, 1);
-      c.phase = kPhS6;
-      return;
-    default:
-      break;
-  }
-  // after stage 6: error estimate and step control (rk_pd54m.c:215-333)
-  gw_fcn(start + step, c.y1, F, dummy, 0, J[0], J[1], J[2], J[3], &c.set);
-  const double huge_number = 1e99, min_tolvalue = 1.e-10;
-  double tr = 0.0, y5[GW_NSTATE];
-  for (int i = 0; i < GW_NSTATE; i++) {
-    const double k6 = step * F[i];
-    y5[i] = c.y[i] + 31.0 / 540.0 * k1[i] + 190.0 / 297.0 * k3[i] - 145.0 / 108.0 * k4[i] + 351.0 / 220.0 * k5[i] +
-            1.0 / 20.0 * k6;
-    const double ym = c.y[i] + 19.0 / 216.0 * k1[i] + 1000.0 / 2079.0 * k3[i] - 125.0 / 216.0 * k4[i] +
-                      81.0 / 88.0 * k5[i] + 5.0 / 56.0 * k6;
-    const double err = fabs((ym - y5[i]) * 0.2 * gw_errweight(i));
-    if (err < huge_number) tr = fmax_ref(err, tr);
-    else tr = huge_number;
-  }
-  const gw_settings& P = c.set;
-  bool finished_output = false;
-  if (tr < P.tolrk || step <= P.step_min) {
-    // an accepted state that is not finite would only be accepted again at
-    // the minimum step, forever: the cell stops with an error instead
-    bool finite = true;
-    for (int i = 0; i < GW_NSTATE; i++) finite = finite && isfinite(y5[i]);
-    if (!finite) {
-      c.err = 2;
-      return;
-    }
-  }
-  if (tr < P.tolrk) {
-    for (int i = 0; i < GW_NSTATE; i++) {
-      if (fabs(y5[i]) < min_tolvalue) y5[i] = 0.0;
-      c.y[i] = y5[i];
-    }
-    c.start = start + step;
-    c.success = 1;
-    if (c.start >= c.tstep) {
-      finished_output = true;
-    } else {
-      double nstep = fmin_ref(0.85 * step * pow(P.tolrk / tr, 0.2), 4.0 * step);
-      c.ostep = nstep;
-      double tts = P.shift - fmod(c.start, P.period);
-      if (tts < 0.0) tts = tts + P.period;
-      if (tts < nstep) nstep = fmax_ref(P.step_min, tts - 0.5 * P.step_min);
-      c.step = nstep;
-    }
-  } else if (step <= P.step_min) {
-    // forced accept at the minimum step
-    for (int i = 0; i < GW_NSTATE; i++) {
-      if (fabs(y5[i]) < min_tolvalue) y5[i] = 0.0;
-      c.y[i] = y5[i];
-    }
-    c.start = start + step;
-    c.success = 1;
-    if (c.start >= c.tstep) {
-      finished_output = true;
-    } else {
-      c.step = P.step_min;
-    }
-    c.ostep = c.step;
-  } else {
-    // reject: roll the FRUs back and retry from stage 2 (no new flux/save)
-    double nstep = 0.85 * step * pow(P.tolrk / tr, 0.2);
-    double tts = P.shift - fmod(start, P.period);
-    if (tts < 0.0) tts = tts + P.period;
-    if (tts < nstep) nstep = fmax_ref(P.step_min, tts - 0.5 * P.step_min);
-    c.success = 0;
-    c.pending = kFlagResume;
-    nstep = fmin_ref(P.step_max, fmax_ref(P.step_min, nstep));
-    c.step = fmin_ref(nstep, c.tstep - c.start);
-    c.oldstep = c.ostep;
-    launch_stage2(c);
-    return;
-  }
-  if (!finished_output && !(tr < P.tolrk)) {
-    // the forced-accept branch clamps like a rejection (rk_pd54m.c:329-331)
-    c.step = fmin_ref(P.step_max, fmax_ref(P.step_min, c.step));
-    c.step = fmin_ref(c.step, c.tstep - c.start);
-  }
-  c.oldstep = c.ostep;
-  if (!finished_output) {
-    launch_flux(c, false);
-    c.phase = kPhFlux;
-    return;
-  }
-  // an output step is complete (gw_run): record it and start the next one
-  const int k = c.step_index;
-  if (c.tr_states)
-    for (int i = 0; i < GW_NSTATE; i++) c.tr_states[(size_t)k * GW_NSTATE + i] = c.y[i];
-  if (c.tr_cur)
-    for (int i = 0; i < GW_NCUR; i++) c.tr_cur[(size_t)k * GW_NCUR + i] = c.cur[i];
-  c.step_index = k + 1;
-  c.steps_left--;
-  c.tnow = c.tnow + P.time_step;
-  if (c.steps_left <= 0) c.final_avg = 1;
-  else begin_output_step(c);
-  launch_flux(c, c.tr_other != nullptr || c.final_avg);
-  c.phase = kPhFlux;
-  if (c.final_avg && !c.tr_other) c.done = 1;
-}
-
-// ---- the same integrator on a whole warp --------------------------------------------
-// dp_after_warp does what dp_after does, with every lane of a warp taking
-// part: the scalar decisions are computed on every lane alike (the FP64
-// pipe issues one warp instruction for one lane or for 32), the 37-element
-// vector operations are split over the lanes (lane l owns states l and
-// l + 32), the exponentials of fcn are evaluated one per lane, and each
-// value is written to the DpCell by one lane only.  Each state's arithmetic
-// is dp_after's, operation for operation, and the error norm is the same
-// maximum, so the results are the same bits.
+// ---- the integrator on a whole warp ------------------------------------------------
+// dp_after_warp advances a cell's integrator after one FRU launch (gw_dp.c,
+// operation for operation) with every lane of a warp taking part; J = (Jxfer,
+// Jtr, ICa, Ito2) at the launch's end point, avg the output-average sums when
+// the launch carried them.  The scalar decisions are computed on every lane
+// alike (the FP64 pipe issues one warp instruction for one lane or for 32), the
+// 37-element vector operations are split over the lanes (lane l owns states l
+// and l + 32), the exponentials of fcn are evaluated one per lane, its two Kv
+// channels on even and odd lanes, and each value is written to the DpCell by
+// one lane only.
 
 // fcn's transcendental terms for `state` at `time`: lane k evaluates
 // exponent k, lanes 0-1 the last two exponents, 2-5 the logs, 6-11 the pows
@@ -307,7 +124,7 @@ __device__ __forceinline__ void fcn_warp(DpCell& c, double time, double* y, doub
 #pragma unroll
   for (int i = 0; i < GW_NSTATE; i++) ys[i] = y[i];
   tx_fill_warp(time, ys, &c.set, &c.tx, lane);
-  gw_fcn_tx(time, ys, F, cur, keepc, J[0], J[1], J[2], J[3], &c.set, &c.tx);
+  gw_fcn_tx(time, ys, F, cur, keepc, J[0], J[1], J[2], J[3], &c.set, &c.tx, lane);
   __syncwarp();
   if (lane == 0) {
     y[GW_mNa] = ys[GW_mNa];
@@ -433,7 +250,7 @@ static __device__ __noinline__ void dp_after_warp(DpCell& c, const double J[4], 
     finite = finite && isfinite(y5);
     c.y5[i] = y5;
   }
-  // dp_after's running maximum: huge_number once any error is not below it
+  // the running maximum of gw_dp.c: huge_number once any error is not below it
   tr = warp_max_ref(tr);
   if (__any_sync(0xffffffffu, bad)) tr = huge_number;
   finite = __all_sync(0xffffffffu, finite);

@@ -65,6 +65,11 @@ __device__ __forceinline__ bool fits(double x) {
   return (uint32_t)__double2hiint(x) - (uint32_t)((1023 - 100) << 20) < (uint32_t)(200 << 20);
 }
 
+// a / b for any operands: the hardware's division where one is out of range.
+__device__ __forceinline__ double checked_div(double a, double b) {
+  return fits(fabs(a)) && fits(fabs(b)) ? fast_div(a, b) : a / b;
+}
+
 // x / d for a constant d: rhi = 1/d rounded, rlo = 1/d - rhi rounded; the
 // two-instruction form returns the correctly rounded quotient for every x
 // for the constants below (N. Brisebarre, J.-M. Muller and S. K. Raina,

@@ -124,7 +124,7 @@ __device__ __forceinline__ int mask_pick(const unsigned long long* m, int nwords
   return -1;
 }
 
-// Post the operation dp_after has just set up in the cell's DpCell (one thread).
+// Post the operation dp_after_warp has just set up in the cell's DpCell (one thread).
 static __device__ void post(const Args& a, int ci) {
   PCell& pc = a.pc[ci];
   pc.overflow = 0u;

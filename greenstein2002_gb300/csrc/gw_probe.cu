@@ -353,7 +353,7 @@ __global__ void fcn_compare_kernel(const double* states, int n, const gw_protoco
   }
   __syncwarp();
   tx_fill_warp(time, y, P, &tx, lane);
-  gw_fcn_tx(time, y, F, cur, 1, 2e-6, 1e-6, -2e-3, 1e-4, P, &tx);
+  gw_fcn_tx(time, y, F, cur, 1, 2e-6, 1e-6, -2e-3, 1e-4, P, &tx, lane);
   if (lane == 0) {
     for (int k = 0; k < GW_NSTATE; k++) Fw[(size_t)i * GW_NSTATE + k] = F[k];
     for (int k = 0; k < GW_NCUR; k++) Cw[(size_t)i * GW_NCUR + k] = cur[k];
@@ -400,7 +400,7 @@ __global__ void fcn_chain_warp(const gw_protocol* P, int calls, double* out) {
   gw_rest_state(y);
   for (int i = 0; i < calls; i++) {
     tx_fill_warp(10.5, y, P, &tx, lane);
-    gw_fcn_tx(10.5, y, F, cur, 1, 1e-6, 1e-6, -1e-3, 0.0, P, &tx);
+    gw_fcn_tx(10.5, y, F, cur, 1, 1e-6, 1e-6, -1e-3, 0.0, P, &tx, lane);
     y[GW_V] = y[GW_V] + fcn_feedback(F, cur);
     __syncwarp();
   }
