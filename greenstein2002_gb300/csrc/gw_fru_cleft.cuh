@@ -792,6 +792,12 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
   const R cmax = gmax(g, imax(R(0.e-3), cass));
   if (ilt(R(1.5e-3), cmax)) dtr = imin(dtr, R(5.001e-3));
   const R dt = F.clk.advance(dtr, L);
+  // which channels leave (:215-276), beside the Heun step
+  const bool lcc_leaves = leave_gt(bw[0], dt, R0[0]), vdi_leaves = leave_ge(bw[1], dt, R0[1]),
+             cl_leaves = leave_ge(bw[7], dt, R0[7]);
+  unsigned pend = 0u;
+  #pragma unroll
+  for (int i = 0; i < kRyR; i++) pend |= leave_gt(bw[2 + i], dt, R0[2 + i]) ? (1u << i) : 0u;
   // ---- Heun step (simfru_local.c:149-173) ----
   R dJ, dS;
   fcn_fru4(g, cajsr, cass, dep, e2, a2j, small, lopen, nopen, pca_scale, dJ, dS);
@@ -806,23 +812,20 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
   F.ss.add((k1S + dt * dS) / R(2));
   // ---- transitions of this cleft's 8 channels (:215-276) ----
   bool moved = false;
-  if (leave_gt(bw[0], dt, R0[0])) {
+  if (lcc_leaves) {
     const LccBasisT<R> lb{alpha, beta, bp};
     R r[4];
     int d[4];
     const int len = lcc_row(lcc_of(w), lb, gam, r, d);
     w = set_field(w, 0, choose_dest(r, d, len, dt, bw[0]));
   }
-  if (leave_ge(bw[1], dt, R0[1])) w = set_field(w, 4, 3 - vdi_of(w));
+  if (vdi_leaves) w = set_field(w, 4, 3 - vdi_of(w));
   // The RyRs that leave their state, then one pass per leaving RyR: the
   // lanes of a warp share the pass (one rate row and destination walk per
   // pass for every lane that has a RyR left), instead of one divergent body
   // per RyR index taken whenever any lane's RyR of that index leaves.  Each
   // RyR's row depends only on its own state and its cleft's constants, so
   // the order of the passes does not matter.
-  unsigned pend = 0u;
-  #pragma unroll
-  for (int i = 0; i < kRyR; i++) pend |= leave_gt(bw[2 + i], dt, R0[2 + i]) ? (1u << i) : 0u;
   moved = pend != 0u;
   while (pend) {
     const int i = __ffs(pend) - 1;
@@ -838,7 +841,7 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
     const int len = ryr_row(ryr_of(w, i), k, r, d);
     w = set_field(w, 8 + 4 * i, choose_dest(r, d, len, dt, y));
   }
-  if (leave_ge(bw[7], dt, R0[7])) w = set_field(w, 28, 3 - cl_of(w));
+  if (cl_leaves) w = set_field(w, 28, 3 - cl_of(w));
   lopen = lcc_open(w) ? R(1) : R(0);
   if (moved) nopen = ryr_open_masked(w);
   F.nsub++;
