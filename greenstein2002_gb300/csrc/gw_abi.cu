@@ -66,17 +66,18 @@ static cudaError_t launch_stage_variant(gw_ctx* c, const StageParams& p0) {
   }
   const int groups = g_stage_warps[c->device & 63].load(std::memory_order_relaxed);
   const bool dense = groups > gw::kRoomyWarpsPerSm * c->sms;
-  // Few FRUs: fewer of them per warp, as long as that makes at most four warps
-  // per SM (one per sub-partition), because the FRUs of a warp execute each
-  // other's branches.  Five stages at the peak of release with 8, 4, 2 and 1
-  // per warp: FP64 250 FRUs 2.97 / 2.85 / 2.82 / 2.81 ms, 1,250 FRUs 3.72 /
-  // 3.62 / 3.60 / 3.72, 2,500 FRUs 3.69 / 3.60 / 3.87 / 4.67; mixed 250 FRUs
-  // 0.651 / 0.630 / 0.614 / 0.609 ms.
-  int fpw = 8;
-  if ((p.flags & gw::kFlagAdvance) && !c->d.trace_ns)
-    fpw = 4 * groups <= 4 * c->sms ? 2 : 2 * groups <= 4 * c->sms ? 4 : 8;
+  // Few FRUs, counted over all cells in flight.  FP64: two per warp on sixteen
+  // lanes each while all those warps are resident (about 3,000 FRUs; figures
+  // at the kernel).  Mixed: fewer of them per warp, as long as that makes at
+  // most four warps per SM (one per sub-partition), because the FRUs of a warp
+  // execute each other's branches: five stages at the peak of release with 8,
+  // 4, 2 and 1 per warp, 250 FRUs 0.651 / 0.630 / 0.614 / 0.609 ms, 1,250 FRUs
+  // 0.792 / 0.762 / 0.759 / 0.778, 2,500 FRUs 0.791 / 0.765 / 0.807 / 0.960.
+  const bool few = (p.flags & gw::kFlagAdvance) && !c->d.trace_ns;
+  const bool wide = few && 4 * groups <= gw::kWideWarpsPerSm * c->sms;
+  const int fpw = !few ? 8 : 4 * groups <= 4 * c->sms ? 2 : 2 * groups <= 4 * c->sms ? 4 : 8;
   if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, fpw, dense, c->stream);
-  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, fpw, dense, c->stream)
+  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, wide, dense, c->stream)
                            : gw::launch_stage(c->d, p, c->stream);
 }
 

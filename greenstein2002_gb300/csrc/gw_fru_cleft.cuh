@@ -186,7 +186,20 @@ __device__ __forceinline__ R pick_basis(int i, R al, R be, R ga, R ap, R bp) {
 struct Group {
   int c;           // cleft of this lane (0..3)
   int base;        // lane index of cleft 0 of this FRU within the warp
-  unsigned mask;   // the four lanes of this FRU
+  unsigned mask;   // the lanes of this FRU
+  int q = 0;       // sixteen lanes per FRU: this lane's copy of the cleft (0..3)
+};
+// Sixteen lanes per FRU (FP64 launches of few FRUs, whose other lanes would
+// idle): four copies of each cleft's lane run the substep alike and share the
+// FP64 work of the local ODE; copy 0 stores.
+struct WideGroup : Group {};
+template <typename G>
+struct is_wide {
+  static constexpr bool value = false;
+};
+template <>
+struct is_wide<WideGroup> {
+  static constexpr bool value = true;
 };
 
 // group-local shuffles (the four lanes of one FRU may run while other
@@ -1102,6 +1115,55 @@ __device__ __forceinline__ void fcn_fru4(const Group& g, double cajsr, double ca
   dJSR = bJSR * (Jtr - (VSS / VJSR) * JRyRtot);
 }
 
+// The same on sixteen lanes: the copies of a cleft's lane take a quotient each
+// (a1 and a2 of the subspace, a1 of the JSR), then a difference times a
+// constant (JRyR, Jss, Jtr, Jxfer), then one sum (dCaSS on copy 0, dCaJSR on
+// copy 2), every lane with operands of its own in one stream: 18 FP64
+// instructions instead of 44.  x * 1 + y, x * y + 0 and x * (-1) + y round
+// as the sum, the product and the difference alone.
+__device__ __forceinline__ void fcn_fru4(const WideGroup& g, double cajsr, double cass, const double dep[3], double e2,
+                                         double a2j, bool small, bool lopen, double jcoef, double pca2, double& dJSR,
+                                         double& dSS) {
+  constexpr double JDHconstant = 1.0 / (2.0 * VSS * Faraday * 1000.0);
+  const int q = g.q;
+  auto copy = [&](double v, int k, int c) { return __shfl_sync(g.mask, v, g.base + 4 * k + c); };
+  double b;  // bSS, on copy 2 bJSR
+  {
+    const double x = (q == 2 ? cajsr : cass) + (q == 0 ? KBSR : q == 2 ? KmCSQN : KBSL);
+    const double den = x * x, num = q == 0 ? BSRtot * KBSR : q == 2 ? CSQNtot * KmCSQN : BSLtot * KBSL;
+    const bool ok = conc_ok(cass) && conc_ok(cajsr);  // alike on the copies of a cleft
+    const double a = ok ? fast_div(num, den) : num / den;
+    const double a1 = copy(a, 0, g.c), a2 = copy(a, 1, g.c), aj = copy(a, 2, g.c);
+    const double t = (1.0 + (q == 2 ? aj : a1)) + (q == 2 ? 0.0 : a2);
+    b = ok ? fast_rcp(t) : 1.0 / t;
+  }
+  const double cnext = from(g, cass, (g.c + 1) & 3);
+  double lin;  // JRyR, Jss, Jtr, Jxfer
+  {
+    const double x = (q == 0 ? cajsr : q == 2 ? dep[2] : cass) - (q == 0 ? cass : q == 1 ? cnext : q == 2 ? cajsr : dep[1]);
+    const double hi = q == 0 ? jcoef : q == 1 ? kDivTauss2ss.rhi : q == 2 ? kDivTautr.rhi : kDivTauxfer.rhi;
+    const double lo = q == 0 ? 0.0 : q == 1 ? kDivTauss2ss.rlo : q == 2 ? kDivTautr.rlo : kDivTauxfer.rlo;
+    lin = fma(x, hi, x * lo);
+  }
+  const double j0 = copy(lin, 0, 0), j1 = copy(lin, 0, 1), j2 = copy(lin, 0, 2), j3 = copy(lin, 0, 3);
+  const double JRyR = copy(lin, 0, g.c), Jss = copy(lin, 1, g.c), Jss_prev = copy(lin, 1, (g.c + 3) & 3);
+  const double Jxfer = copy(lin, 3, g.c);
+  double JDH = 0.0;
+  if (lopen) {
+    if (small) JDH = pca2 * (cass - Cao * 0.341) * JDHconstant;
+    else JDH = -(cass * e2 - Cao * 0.341) * a2j;
+  }
+  const bool jsr = q == 2;
+  double s = (jsr ? j0 : JDH) + (jsr ? j1 : JRyR);
+  s = s + (jsr ? j2 : -Jxfer);
+  s = s + (jsr ? j3 : -Jss);
+  s = fma(s, jsr ? VSS / VJSR : 1.0, jsr ? 0.0 : Jss_prev);
+  s = fma(s, jsr ? -1.0 : 1.0, jsr ? lin : 0.0);  // copy 2: Jtr less it
+  const double d = b * s;
+  dSS = copy(d, 0, g.c);
+  dJSR = copy(d, 2, 0);
+}
+
 // The rates of a substep decide two things: its size dt = min(0.1 / the
 // largest rate, a cap), and, against the draws, which channels change state.
 // Both are settled by FP32 estimates of the rates (relative error below
@@ -1155,8 +1217,9 @@ __device__ __forceinline__ void substep_a(Fru4<double>& F, Sub4<double>& S, cons
 
 // Second half: the remaining words, the RyR pseudo-states, the substep size,
 // the Heun step of the local Ca ODE and the transitions (:135-277).
-__device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const Group& g,
-                                          StageCtx& sc) {
+template <typename G>
+__device__ __forceinline__ void substep_b64(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const G& g,
+                                            StageCtx& sc) {
   uint32_t w = F.w;
   const double cajsr = S.cajsr, cass = S.cass, V = F.dep[0];
   const int regime = S.regime;
@@ -1330,22 +1393,32 @@ __device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, cons
   F.nsub++;
 }
 
+__device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L, const Group& g,
+                                          StageCtx& sc) {
+  substep_b64(F, S, L, g, sc);
+}
+__device__ __forceinline__ void substep_b(Fru4<double>& F, Sub4<double>& S, const LaneStage<double>& L,
+                                          const WideGroup& g, StageCtx& sc) {
+  substep_b64(F, S, L, g, sc);
+}
+
 // Regenerate, with the whole warp, the MT rows whose draws in this substep
 // run past word 624 (`go`: this lane's FRU takes a substep now).
 template <typename R>
 __device__ __forceinline__ void regen_step(const StageCtx& sc, int lane, const Group& g, bool go, const Fru4<R>& F,
                                            const Sub4<R>& S) {
   const bool cross = go && (F.mti + S.etot + 32 > kMtN);
-  const unsigned cross_mask = __ballot_sync(0xffffffffu, cross && g.c == 0);
-  const unsigned copy_mask = __ballot_sync(0xffffffffu, cross && g.c == 0 && *sc.my_hold_epoch != sc.p->epoch);
+  const bool lead = cross && g.c == 0 && g.q == 0;
+  const unsigned cross_mask = __ballot_sync(0xffffffffu, lead);
+  const unsigned copy_mask = __ballot_sync(0xffffffffu, lead && *sc.my_hold_epoch != sc.p->epoch);
   if (cross_mask) regen_crossing(sc, lane, cross_mask, copy_mask);
 }
 
 // One FRU over [t0, tf] by its four lanes (simfru_local.c:83-277).  cajsr and
 // cass are the FRU's FP64 state; arithmetic runs in R.  Every lane of the
 // warp calls it together (live = false for a group without an FRU).
-template <typename R>
-__device__ __forceinline__ void advance4(StageCtx& sc, const Group& g, bool live, double& cajsr64, double& cass64,
+template <typename R, typename G>
+__device__ __forceinline__ void advance4(StageCtx& sc, const G& g, bool live, double& cajsr64, double& cass64,
                                          uint32_t& w, int& mti, uint32_t& nsub, bool& overflow) {
   LaneStage<R> L;
   lane_stage(*sc.p, g, L);
@@ -1414,8 +1487,9 @@ __device__ __forceinline__ void put_seq(const StageParams& p, double* out, int l
   }
 }
 
-template <typename R>
+template <typename R, typename G = Group>
 __device__ __forceinline__ void stage_body(const DevState& s, const StageParams& p, int bidx, double* out, int fpw = 8) {
+  constexpr bool wide = is_wide<G>::value;  // sixteen lanes per FRU, at most two FRUs per warp
   const int lane = threadIdx.x & 31;
   const int first = (bidx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * fpw;  // the warp's first FRU
   const int grp = first >> 3;  // their 8-FRU group
@@ -1431,11 +1505,12 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
   }
   if (first >= s.nfru) return;  // whole warps past the cell's last FRU
   if (s.trace_ns && lane == 0) s.trace_ns[2 * grp] = global_ns();
-  Group g;
+  G g;
   g.c = lane & 3;
-  g.base = lane & ~3;
-  g.mask = 0xfu << g.base;
-  const int slot = lane >> 2;
+  g.q = wide ? (lane >> 2) & 3 : 0;
+  g.base = wide ? lane & ~15 : lane & ~3;
+  g.mask = (wide ? 0xffffu : 0xfu) << g.base;
+  const int slot = wide ? lane >> 4 : lane >> 2;
   bool active = slot < fpw && first + slot < s.nfru;  // uniform over each 4-lane group
   const int f = active ? first + slot : first;
   uint32_t nsub = 0;
@@ -1466,7 +1541,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
       w = s.chan[g.c * nf + f];
       mti = s.mti[f];
     }
-    if (p.flags & kFlagSave) {
+    if ((p.flags & kFlagSave) && g.q == 0) {
       if (g.c == 0) {
         s.frus_s[f] = cajsr;
         s.mti_s[f] = mti;
@@ -1484,7 +1559,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
   } else if (active && restore) {
     copy_row16(gm, hold, g);
   }
-  if (active) {
+  if (active && g.q == 0) {
     if (s.trace_sub && g.c == 0) s.trace_sub[f] = nsub;
     if (g.c == 0) {
       s.frus[f] = cajsr;
@@ -1497,7 +1572,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
   if (s.trace_ns && lane == 0) s.trace_ns[2 * grp + 1] = global_ns();
   if (overflow) out[kOutError] = 1.0;
   if (s.substeps) {
-    unsigned c = __reduce_add_sync(0xffffffffu, (g.c == 0) ? nsub : 0u);
+    unsigned c = __reduce_add_sync(0xffffffffu, (g.c == 0 && g.q == 0) ? nsub : 0u);
     if (lane == 0 && c) atomicAdd(s.substeps, (unsigned long long)c);
   }
   if (fpw < 8) {
@@ -1512,11 +1587,12 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();
-    active = slot < (int)size;
+    const int ff = grp * 8 + (lane >> 2);
+    active = ff < s.nfru;
     if (active) {
-      cajsr = __ldcg(&s.frus[grp * 8 + slot]);
-      cass = __ldcg(&s.frus[(g.c + 1) * nf + grp * 8 + slot]);
-      w = __ldcg(&s.chan[g.c * nf + grp * 8 + slot]);
+      cajsr = __ldcg(&s.frus[ff]);
+      cass = __ldcg(&s.frus[(g.c + 1) * nf + ff]);
+      w = __ldcg(&s.chan[g.c * nf + ff]);
     }
   }
   if (p.flags & kFlagAvg) {

@@ -11,21 +11,33 @@ namespace gw {
 // eleven single-warp blocks per SM) for launches that fit the GPU so, and
 // capped at 128 (sixteen) for more.  Five stages at the peak of release, 128
 // and 180 registers: 12,500 FRUs 6.82 and 6.07 ms, 250 FRUs alike.
-__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage4_kernel(DevState s, StageParams p, int fpw) {
-  cleft::stage_body<double>(s, p, blockIdx.x, s.res, fpw);
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage4_kernel(DevState s, StageParams p) {
+  cleft::stage_body<double>(s, p, blockIdx.x, s.res);
 }
-__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage4_dense_kernel(DevState s, StageParams p, int fpw) {
-  cleft::stage_body<double>(s, p, blockIdx.x, s.res, fpw);
+// Two FRUs per warp, sixteen lanes each: the FP64 chain of a substep is shorter
+// by the local ODE's (104 to about 55 instructions for an FRU alone in its
+// warp), for four times the warps.  Five stages at the peak of release, this
+// and the fixed layout (8 FRUs per warp; 4 below 2,500): 250 FRUs 2.36 and 2.79
+// ms, 1,250 2.98 and 3.71, 2,500 3.08 and 3.73, 3,000 3.83 and 4.13, 4,000 4.17
+// and 4.08.
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage4_wide_kernel(DevState s, StageParams p) {
+  cleft::stage_body<double, cleft::WideGroup>(s, p, blockIdx.x, s.res, 2);
+}
+__global__ void __launch_bounds__(kMaxStageWarps * 32, 2) fru_stage4_dense_kernel(DevState s, StageParams p) {
+  cleft::stage_body<double>(s, p, blockIdx.x, s.res);
 }
 
-cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, int fpw, bool dense, cudaStream_t st) {
-  const int blocks = stage_blocks(s.nfru, warps, fpw);
+cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, bool wide, bool dense, cudaStream_t st) {
+  const int blocks = stage_blocks(s.nfru, warps, wide ? 2 : 8);
   static const cudaError_t attr = stage_cache_attributes(fru_stage4_kernel);
   static const cudaError_t attr_dense = stage_cache_attributes(fru_stage4_dense_kernel);
   if (attr != cudaSuccess) return attr;
   if (attr_dense != cudaSuccess) return attr_dense;
-  if (dense) fru_stage4_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p, fpw);
-  else fru_stage4_kernel<<<blocks, 32 * warps, 0, st>>>(s, p, fpw);
+  static const cudaError_t attr_wide = stage_cache_attributes(fru_stage4_wide_kernel);
+  if (attr_wide != cudaSuccess) return attr_wide;
+  if (wide) fru_stage4_wide_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  else if (dense) fru_stage4_dense_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
+  else fru_stage4_kernel<<<blocks, 32 * warps, 0, st>>>(s, p);
   return cudaGetLastError();
 }
 

@@ -57,11 +57,12 @@ def test_substep_matches_oracle(gw, n, v, dv, ca, ms, packed):
     np.testing.assert_allclose(got["frus"], s["frus"], rtol=1e-12, atol=0)
 
 
-@pytest.mark.parametrize("n", [3, 9, 1216, 1217, 2427, 2433])
+@pytest.mark.parametrize("n", [3, 9, 1216, 2433, 3039, 3041])
 def test_few_frus_per_warp_match_oracle(gw, n):
-    """Launches with 2, 4 and 8 FRUs per warp (by FRU count), whose groups are
-    summed by the warp that completes them; the sums over n FRUs of values
-    equal to 1e-12 are equal to 1e-12."""
+    """FP64 launches of two FRUs per warp on sixteen lanes each, and of 8 per
+    warp above 3,040 FRUs; in the former the group of 8 is summed by the warp
+    that completes it.  The sums over n FRUs of values equal to 1e-12 are
+    equal to 1e-12."""
     s = random_set(n, 11 + n, (-4.0, -1.5))
     cell = gw.Cell(n)
     cell.upload(s)
@@ -74,3 +75,22 @@ def test_few_frus_per_warp_match_oracle(gw, n):
     for k in ("ltype", "ryr", "ito2", "mti", "mt"):
         np.testing.assert_array_equal(got[k], s[k], err_msg=k)
     np.testing.assert_allclose(got["frus"], s["frus"], rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("n", [5, 1217, 2433])
+def test_mixed_few_frus_per_warp_same_bits(gw, n):
+    """Mixed launches with 2, 4 and 8 FRUs per warp (by FRU count) against
+    packed ones, whose sums come from the fixed layout: the same bits."""
+    s = random_set(n, 23 + n, (-4.0, -1.5))
+    d0, df = np.array([5.0, 3e-4, 0.5]), np.array([5.4, 3e-4, 0.49])
+    res = []
+    for packed in (0, 7):
+        cell = gw.Cell(n, precision="mixed")
+        if packed:
+            cell.set_stage_packing(packed)
+        cell.upload(s)
+        nums = [cell.stage(t, t + 0.02, d0, df)[1] for t in (0.0, 0.02, 0.04)]
+        res.append((nums, cell.download()))
+    np.testing.assert_array_equal(res[0][0], res[1][0])
+    for k in ("frus", "ltype", "ryr", "ito2", "mti", "mt"):
+        np.testing.assert_array_equal(res[0][1][k], res[1][1][k], err_msg=k)
