@@ -112,17 +112,14 @@ __device__ __forceinline__ bool u_reaches(uint32_t y, double P) {
   thresh(P, fl, ex);
   return (uint64_t)y > fl || (ex && (uint64_t)y == fl);
 }
-// 2^32 - y rounded to FP32, from a 32-bit conversion (0 - y wraps to it for
-// y > 0): the same value as converting the 33-bit integer, without a 64-bit
-// integer conversion, which runs on the FP64 pipe.
-__device__ __forceinline__ float comp_u32(uint32_t y) { return y ? (float)(0u - y) : 4294967296.0f; }
-// FP32: complement form, 1 - u = (2^32 - y)/2^32 against dt*R
-__device__ __forceinline__ bool leave_gt(uint32_t y, float dt, float R) {
-  return comp_u32(y) < dt * R * 4294967296.0f;
-}
-__device__ __forceinline__ bool leave_ge(uint32_t y, float dt, float R) {
-  return comp_u32(y) <= dt * R * 4294967296.0f;
-}
+// 2^32 - y rounded to FP32, from a 32-bit conversion: the same value as
+// converting the 33-bit integer, without a 64-bit integer conversion, which
+// runs on the FP64 pipe.  (0 - y is 2^32 - y for y > 0; for y = 0, y = 1 rounds
+// to 2^32 too.)
+__device__ __forceinline__ float comp_u32(uint32_t y) { return (float)(0u - max(y, 1u)); }
+// FP32: complement form, 1 - u = (2^32 - y)/2^32 against dt*R, dts = dt 2^32
+__device__ __forceinline__ bool leave_gt(uint32_t y, float dts, float R) { return comp_u32(y) < dts * R; }
+__device__ __forceinline__ bool leave_ge(uint32_t y, float dts, float R) { return comp_u32(y) <= dts * R; }
 
 // Destination of a channel that leaves its state (simfru_local.c:215-253) in
 // FP32: walks the remaining exit mass against 1 - u = (2^32 - y)/2^32, which
@@ -806,11 +803,12 @@ __device__ __forceinline__ void substep_b(Fru4<R>& F, Sub4<R>& S, const LaneStag
   if (ilt(R(1.5e-3), cmax)) dtr = imin(dtr, R(5.001e-3));
   const R dt = F.clk.advance(dtr, L);
   // which channels leave (:215-276), beside the Heun step
-  const bool lcc_leaves = leave_gt(bw[0], dt, R0[0]), vdi_leaves = leave_ge(bw[1], dt, R0[1]),
-             cl_leaves = leave_ge(bw[7], dt, R0[7]);
+  const R dts = dt * R(4294967296.0);
+  const bool lcc_leaves = leave_gt(bw[0], dts, R0[0]), vdi_leaves = leave_ge(bw[1], dts, R0[1]),
+             cl_leaves = leave_ge(bw[7], dts, R0[7]);
   unsigned pend = 0u;
   #pragma unroll
-  for (int i = 0; i < kRyR; i++) pend |= leave_gt(bw[2 + i], dt, R0[2 + i]) ? (1u << i) : 0u;
+  for (int i = 0; i < kRyR; i++) pend |= leave_gt(bw[2 + i], dts, R0[2 + i]) ? (1u << i) : 0u;
   // ---- Heun step (simfru_local.c:149-173) ----
   R dJ, dS;
   fcn_fru4(g, cajsr, cass, dep, e2, a2j, small, lopen, nopen, pca_scale, dJ, dS);
