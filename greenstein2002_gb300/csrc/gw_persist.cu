@@ -445,16 +445,23 @@ using gw::persist::PCell;
 
 namespace {
 
-// 8-FRU groups a warp takes at once: up to four (32 FRUs, the packed
-// launches' best shape for full GPUs), fewer when the cells have too few
-// groups to give every resident warp two batches.  GW_PERSIST_GROUPS
-// (1..8) overrides the choice.
-int persist_batch(long long total_groups, long long warps) {
+// 8-FRU groups a warp takes at once.  A long batch keeps the warp's lanes busy
+// (its FRUs are handed out as others finish) but ends an operation late: eight
+// when every resident warp has 14 groups or more, so that other cells fill the
+// wait, and the cells 256 on average, so that its last batches are few of
+// many; else up to four, fewer when there are not two batches per warp.
+// Four and eight groups, mixed: 16 cells of 12,500 FRUs (20.6 groups per warp)
+// 244 and 228 ms (FP64 294 and 263), 12 of them (15.4) 184 and 172, 40 uneven
+// ones (16.6) 99 and 96, 64 uneven ones (27.8) 340 and 318; 8 of 12,500 (10.3)
+// 72.5 and 85.5, 24 uneven ones (about 10) 115.5 and 136, 200 of 700 (14.5) 53
+// and 58.  GW_PERSIST_GROUPS (1..8) overrides the choice.
+int persist_batch(int ncells, long long total_groups, long long warps) {
   const char* env = getenv("GW_PERSIST_GROUPS");
   if (env) {
     const int v = atoi(env);
     if (v >= 1 && v <= gw::persist::kMaxBatchGroups) return v;
   }
+  if (warps > 0 && total_groups >= 14 * warps && total_groups >= 256LL * ncells) return gw::persist::kMaxBatchGroups;
   long long b = warps > 0 ? total_groups / (2 * warps) : 1;
   return (int)(b < 1 ? 1 : b > 4 ? 4 : b);
 }
@@ -579,7 +586,7 @@ int run_persistent(int n, gw_ctx** cells, const gw_settings* sets, double* t, do
   args.running = (unsigned*)dcnt;
   args.open_mask = dmask;
   args.nwords = nwords;
-  args.batch = persist_batch(total_groups, (long long)sms * per_sm);
+  args.batch = persist_batch(n, total_groups, (long long)sms * per_sm);
   args.status = dcnt + 3;
   args.release = hold ? dcnt + 4 : nullptr;
   args.progress = d64;
