@@ -200,6 +200,9 @@ extern "C" int gw_run_device(int n, gw_ctx** cells, const gw_settings* sets, dou
       e = cudaMemcpyAsync(dblock0, hblock0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dcount, cnt, sizeof cnt, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(drounds, 0, sizeof(unsigned long long), st);
+    // an earlier run may have ended at the substep limit
+    for (int i = 0; i < n && e == cudaSuccess; i++)
+      e = cudaMemsetAsync(cells[i]->d.out + gw::kOutError, 0, sizeof(double), st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   }
   // graph: WHILE (cells running) { one round }

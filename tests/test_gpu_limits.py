@@ -1,0 +1,39 @@
+"""The substep limit (2^22 substeps of an FRU in one stage) as an error that
+ends with the call: a stage over [0, 1e9) ms, whose substeps are at most 0.01
+ms, runs into it.  No fault is involved and the state stays finite.  The call
+reports it, cells beside it are not touched, and the next call on the same
+cell, from an uploaded state, gives the bits of a fresh cell."""
+import numpy as np
+import pytest
+
+from test_gpu_batch import _cells
+
+pytestmark = pytest.mark.gpu
+
+
+def _long(gw):
+    return gw.settings(time_step=1e9, step_max=1e9)
+
+
+def _alone(gw, run, size, first):
+    cells, sets, states = _cells(gw, [size], "mixed", first=first)
+    t, old = np.zeros(1), np.full(1, 0.1)
+    run(cells, sets, t, states, old, 2)
+    return states[0], cells[0].download()
+
+
+def _same(a, b):
+    np.testing.assert_array_equal(a[0], b[0])
+    for k in b[1]:
+        np.testing.assert_array_equal(a[1][k], b[1][k], err_msg=k)
+
+
+def test_device_runner_runs_again_after_the_limit(gw):
+    cells, sets, states = _cells(gw, [2], "mixed")
+    s0, st0 = cells[0].download(), states.copy()
+    with pytest.raises(gw.GWError, match="substep limit"):
+        gw.run_device(cells, [_long(gw)], np.zeros(1), states, np.full(1, 1e9), 1)
+    cells[0].upload(s0)
+    states[:] = st0
+    gw.run_device(cells, sets, np.zeros(1), states, np.full(1, 0.1), 2)
+    _same((states[0], cells[0].download()), _alone(gw, gw.run_device, 2, 0))
