@@ -149,10 +149,14 @@ static void finish_round(gw_batch* b) {
   cudaError_t e = launch_round(b);
   if (e != cudaSuccess) b->error = (int)e;
   // hand every member its outputs now: slots are renumbered when a member
-  // leaves, so a waiter must not look its outputs up by index later
-  for (size_t i = 0; i < b->members.size(); i++)
+  // leaves, so a waiter must not look its outputs up by index later.  The
+  // kernel sets the error flag and never clears it: the slot may be another
+  // cell's in the next round
+  for (size_t i = 0; i < b->members.size(); i++) {
     for (int k = 0; k < gw::kBatchOutStride; k++)
       b->members[i]->batch_out[k] = b->h_outs[gw::kBatchOutStride * i + k];
+    b->h_outs[gw::kBatchOutStride * i + gw::kOutError] = 0.0;
+  }
   b->round++;
   b->nposted = 0;
   for (auto& x : b->posted) x = 0;

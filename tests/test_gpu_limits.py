@@ -37,3 +37,22 @@ def test_device_runner_runs_again_after_the_limit(gw):
     states[:] = st0
     gw.run_device(cells, sets, np.zeros(1), states, np.full(1, 0.1), 2)
     _same((states[0], cells[0].download()), _alone(gw, gw.run_device, 2, 0))
+
+
+def test_lockstep_batch_keeps_the_limit_to_its_cell(gw):
+    sizes = [2, 40, 25]
+    b = gw.Batch("mixed")
+    cells, sets, states = _cells(gw, sizes, "mixed")
+    s0, st0 = cells[0].download(), states[0].copy()
+    t = np.zeros(3)
+    with pytest.raises(gw.GWError, match="cell 0.*substep limit"):
+        b.run(cells, [_long(gw)] + sets[1:], t, states, np.array([1e9, 0.1, 0.1]), 2)
+    assert t[1] == 2 and t[2] == 2
+    want = [_alone(gw, gw.Batch("mixed").run, n, i) for i, n in enumerate(sizes)]
+    for i in (1, 2):
+        _same((states[i], cells[i].download()), want[i])
+    cells[0].upload(s0)
+    states[0] = st0
+    t0, old = np.zeros(1), np.full(1, 0.1)
+    b.run(cells[:1], sets[:1], t0, states[:1], old, 2)
+    _same((states[0], cells[0].download()), want[0])
