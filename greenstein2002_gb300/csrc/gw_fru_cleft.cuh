@@ -1566,9 +1566,11 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
     s.frus[(g.c + 1) * nf + f] = cass;
     s.chan[g.c * nf + f] = w;
   }
+  // before the barrier, so that lane 0's fences carry it and the host, which
+  // waits for the sequence number only, finds it with this launch's totals
+  if (overflow) out[kOutError] = 1.0;
   __syncwarp();
   if (s.trace_ns && lane == 0) s.trace_ns[2 * grp + 1] = global_ns();
-  if (overflow) out[kOutError] = 1.0;
   if (s.substeps) {
     unsigned c = __reduce_add_sync(0xffffffffu, (g.c == 0 && g.q == 0) ? nsub : 0u);
     if (lane == 0 && c) atomicAdd(s.substeps, (unsigned long long)c);

@@ -56,3 +56,24 @@ def test_lockstep_batch_keeps_the_limit_to_its_cell(gw):
     t0, old = np.zeros(1), np.full(1, 0.1)
     b.run(cells[:1], sets[:1], t0, states[:1], old, 2)
     _same((states[0], cells[0].download()), want[0])
+
+
+@pytest.mark.parametrize("packed", [0, 1])
+def test_limit_is_reported_by_its_own_stage(gw, packed):
+    """The flag is stored before the launch's number, which ends the wait."""
+    dep = np.array([-80.0, 1e-4, 0.5])
+    cells, _, _ = _cells(gw, [2, 2], "mixed")
+    cells[1].upload(cells[0].download())
+    s0 = cells[0].download()
+    for c in cells:
+        c.set_stage_packing(packed)
+    with pytest.raises(gw.GWError, match="substep limit"):
+        cells[0].stage(0.0, 1e9, dep, dep)
+    cells[0].upload(s0)
+    for t in (0.0, 0.02):
+        a, b = (c.stage(t, t + 0.02, dep, dep) for c in cells)
+        np.testing.assert_array_equal(a[0], b[0])
+        np.testing.assert_array_equal(a[1], b[1])
+    a, b = (c.download() for c in cells)
+    for k in a:
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
