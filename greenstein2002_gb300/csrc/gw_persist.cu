@@ -618,10 +618,14 @@ int run_persistent(int n, gw_ctx** cells, const gw_settings* sets, double* t, do
   if (e != cudaSuccess) {
     rc = gw_internal_error(GW_ECUDA, (std::string(who) + ": " + cudaGetErrorString(e)).c_str());
   } else if (hc[3] != gw::persist::kStatusOk) {
-    // operations may be half summed: their tickets start afresh
-    for (int i = 0; i < n; i++) cudaMemset(cells[i]->d.ticket, 0, sizeof(unsigned));
-    rc = gw_internal_error(GW_ECUDA, "gw_run_persistent: no progress within the wait limit (watchdog); the cells' "
-                                     "state is that of an unfinished run");
+    // operations may be half summed: their tickets start afresh, on the streams
+    // that the cells' next stages run on
+    for (int i = 0; i < n && e == cudaSuccess; i++)
+      e = cudaMemsetAsync(cells[i]->d.ticket, 0, sizeof(unsigned), cells[i]->stream);
+    rc = gw_internal_error(GW_ECUDA, e != cudaSuccess
+                                         ? (std::string(who) + ": " + cudaGetErrorString(e)).c_str()
+                                         : "gw_run_persistent: no progress within the wait limit (watchdog); the "
+                                           "cells' state is that of an unfinished run");
   } else {
     for (int i = 0; i < n; i++) {
       const DpCell& d = hout[i];

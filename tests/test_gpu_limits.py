@@ -77,3 +77,18 @@ def test_limit_is_reported_by_its_own_stage(gw, packed):
     a, b = (c.download() for c in cells)
     for k in a:
         np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+def test_stages_after_a_stopped_persistent_run(gw):
+    """The tickets of a persistent run that the wait limit ended are reset on
+    the cell's own stream, so the next stages sum every group."""
+    dep = np.array([-80.0, 1e-4, 0.5])
+    cells, sets, _ = _cells(gw, [500, 500], "fp64")
+    s0 = cells[1].download()
+    assert gw.persist_watchdog(cells[0], sets[0], 0.1) == 3
+    for c in cells:
+        c.upload(s0)
+    for t in (0.0, 0.02):
+        a, b = (c.stage(t, t + 0.02, dep, dep) for c in cells)
+        np.testing.assert_array_equal(a[0], b[0])
+        np.testing.assert_array_equal(a[1], b[1])
