@@ -2,7 +2,6 @@
 // downloads in the reference's array layout, and the stage / flux / average
 // / save / resume operations that replace the MPI layer of mpi_master.c.
 #include <cuda_runtime.h>
-#include <sched.h>
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -18,6 +17,7 @@
 #include "gw_kernels.h"
 #include "gw_fru_model.cuh"
 #include "gw_ctx_impl.h"
+#include "gw_wait.h"
 
 using gw::DevState;
 using gw::StageParams;
@@ -377,17 +377,15 @@ extern "C" int gw_seed(gw_ctx* c, int scheme, uint32_t base) {
 // this wait; a thread alone waits as long either way.  The stream is asked
 // now and then, so that a failed launch ends the wait; the kernel may still be
 // retiring when this returns, so all that follows stays ordered by the stream.
-static cudaError_t wait_totals(gw_ctx* c, uint32_t seq) {
-  const unsigned long long* slot = reinterpret_cast<const unsigned long long*>(c->h_out + gw::kOutSeq);
-  for (;;) {
-    for (int i = 0; i < 256; i++) {
-      for (int k = 0; k < 64; k++)
-        if (__atomic_load_n(slot, __ATOMIC_ACQUIRE) == seq) return cudaSuccess;
-      sched_yield();
-    }
-    const cudaError_t e = cudaStreamQuery(c->stream);
-    if (e != cudaErrorNotReady) return e;
-  }
+// *arrived: false when the stream has run dry without the number (the sums of
+// an earlier launch are still in h_out).
+static cudaError_t wait_totals(gw_ctx* c, uint32_t seq, bool* arrived) {
+  cudaError_t e = cudaSuccess;
+  *arrived = gw::wait_number(reinterpret_cast<const unsigned long long*>(c->h_out + gw::kOutSeq), seq, [&] {
+    e = cudaStreamQuery(c->stream);
+    return e == cudaErrorNotReady;
+  });
+  return e == cudaErrorNotReady ? cudaSuccess : e;
 }
 
 static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], const double depf[3], int advance,
@@ -422,7 +420,9 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
     if (c->profiling) CK(cudaEventRecord(c->pev[1], c->stream));
     // the one-lane kernel and the sequential sums do not number their totals
     const bool numbered = c->fru_lanes == 4 && c->sum_order == GW_SUM_TREE && !c->profiling;
-    CK(numbered ? wait_totals(c, p.seq) : cudaStreamSynchronize(c->stream));
+    bool arrived = true;
+    CK(numbered ? wait_totals(c, p.seq, &arrived) : cudaStreamSynchronize(c->stream));
+    if (!arrived) return set_err(GW_ECUDA, "FRU stage [%g, %g]: the launch ended without its sums", t0, tf);
   }
   if (c->h_out[gw::kOutError] != 0.0) {
     c->h_out[gw::kOutError] = 0.0;
