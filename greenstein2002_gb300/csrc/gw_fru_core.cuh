@@ -212,45 +212,58 @@ static __device__ inline void currents_from_sums(int nfru, double scale, const d
   out[3] = scale * ito2;
 }
 
+// a / b for a divisor in the fast form's range; a zero, of a cell without
+// open channels, keeps the sign of the product (the fast form's last sum makes
+// it +0).  `plain` is set where a is out of range (infinite, NaN).
+__device__ __forceinline__ double current_div(double a, double b, bool& plain) {
+  const bool zero = (__double_as_longlong(a) << 1) == 0;
+  plain = plain || !(zero || fits(fabs(a)));
+  const double y = rcp_seed(b), q = a * y;
+  const double f = fma(fma(-b, q, a), y, q);
+  return zero ? q : f;
+}
+
 // The currents of a launch's totals, one per lane: on return lanes 0..3 hold
 // Jxfer, Jtr, ICa, Ito2 in cur.  num: the flux numerators, the same in every
 // lane.  One instruction stream for the four (36 FP64 instructions; on one
 // lane one after another about 120, 4 us of every launch): a product and a
 // difference, two quotients and the scale, the operands selected by lane.
+// Potentials at 0 or beyond 500 mV and numerators out of the quotients' range
+// take the plain expressions.
 // GW_CONTRACT (the mixed-precision unit): products feeding a difference are
 // fused, as the compiler fuses currents_from_sums there.
 __device__ __forceinline__ double lane_current(const DevState& s, const StageParams& p, const double num[5], int lane) {
   const double V = p.depf[0];
   const long long av = __double_as_longlong(V) & 0x7fffffffffffffffLL;
-  if (av < __double_as_longlong(1.e-6) || av >= __double_as_longlong(500.0)) {
-    double cur[4];
-    currents_from_sums(s.nfru, p.nfru_scale, p.depf, num, cur);
-    const double c = lane == 0 ? cur[0] : lane == 1 ? cur[1] : lane == 2 ? cur[2] * p.pca_scale : cur[3];
-    return c;
-  }
-  const double VFRT = const_div(V, kDivRTF), VFsqRT = (1000.0 * Faraday) * VFRT;
-  const double e1 = exp(VFRT), e2 = e1 * e1;
-  const double n = (double)s.nfru;
-  const double c = num[3] * Cao;
-  // x * y, subtracted from or less the other operand z (lane 2: z = (num3 Cao) 0.341)
-  const double x = lane == 0 ? n * (double)kClefts : lane == 1 ? n : lane == 2 ? num[2] : Clo;
-  const double y = lane == 0 ? p.depf[1] : lane == 1 ? p.depf[2] : lane == 2 ? e2 : e1;
-  const double z = lane == 0 ? num[0] : lane == 1 ? num[1] : lane == 2 ? c * 0.341 : Cli;
-  const bool minus = lane == 0 || lane == 3;  // z - x y, else x y - z
+  bool plain = av < __double_as_longlong(1.e-6) || av >= __double_as_longlong(500.0);
+  if (!plain) {
+    const double VFRT = const_div(V, kDivRTF), VFsqRT = (1000.0 * Faraday) * VFRT;
+    const double e1 = exp(VFRT), e2 = e1 * e1;
+    const double n = (double)s.nfru;
+    const double c = num[3] * Cao;
+    // x * y, subtracted from or less the other operand z (lane 2: z = (num3 Cao) 0.341)
+    const double x = lane == 0 ? n * (double)kClefts : lane == 1 ? n : lane == 2 ? num[2] : Clo;
+    const double y = lane == 0 ? p.depf[1] : lane == 1 ? p.depf[2] : lane == 2 ? e2 : e1;
+    const double z = lane == 0 ? num[0] : lane == 1 ? num[1] : lane == 2 ? c * 0.341 : Cli;
+    const bool minus = lane == 0 || lane == 3;  // z - x y, else x y - z
 #ifdef GW_CONTRACT
-  double b = fma(minus ? -x : x, y, minus ? z : -z);
+    double b = fma(minus ? -x : x, y, minus ? z : -z);
 #else
-  const double xy = x * y;
-  double b = (minus ? z : xy) - (minus ? xy : z);
+    const double xy = x * y;
+    double b = (minus ? z : xy) - (minus ? xy : z);
 #endif
-  const double a = (lane == 2 ? PCa * 4.0 : num[4] * PCl) * VFsqRT;
-  const double ab = a * b;
-  b = lane >= 2 ? ab : b;
-  const double em1 = (lane == 2 ? e2 : 1.0) - (lane == 2 ? 1.0 : e1);
-  const double q = fast_div(b, lane == 0 ? tauxfer : lane == 1 ? tautr : em1);
-  const double r = fast_div(q, Acap);
-  const double cur = p.nfru_scale * (lane >= 2 ? r : q);
-  return lane == 2 ? cur * p.pca_scale : cur;  // ICa is proportional to the LCC permeability
+    const double a = (lane == 2 ? PCa * 4.0 : num[4] * PCl) * VFsqRT;
+    const double ab = a * b;
+    b = lane >= 2 ? ab : b;
+    const double em1 = (lane == 2 ? e2 : 1.0) - (lane == 2 ? 1.0 : e1);
+    const double q = current_div(b, lane == 0 ? tauxfer : lane == 1 ? tautr : em1, plain);
+    const double r = current_div(q, Acap, plain);
+    const double cur = p.nfru_scale * (lane >= 2 ? r : q);
+    if (!plain) return lane == 2 ? cur * p.pca_scale : cur;  // ICa is proportional to the LCC permeability
+  }
+  double cur[4];
+  currents_from_sums(s.nfru, p.nfru_scale, p.depf, num, cur);
+  return lane == 0 ? cur[0] : lane == 1 ? cur[1] : lane == 2 ? cur[2] * p.pca_scale : cur[3];
 }
 
 // Categorical selection of simfru_local.c:217-226 for a channel that has left
