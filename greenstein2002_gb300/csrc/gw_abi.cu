@@ -112,6 +112,9 @@ extern "C" int gw_create(gw_ctx** out, int nfru) {
   if (!c) return set_err(GW_ENOMEM, "gw_create: host allocation failed");
   cudaGetDevice(&c->device);
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
+  unsigned flags = 0;
+  c->blocking = cudaGetDeviceFlags(&flags) == cudaSuccess &&
+                (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
   DevState& d = c->d;
   d.nfru = nfru;
   d.stride = (nfru + 31) & ~31;
@@ -418,8 +421,9 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
       c->launches++;
     }
     if (c->profiling) CK(cudaEventRecord(c->pev[1], c->stream));
-    // the one-lane kernel and the sequential sums do not number their totals
-    const bool numbered = c->fru_lanes == 4 && c->sum_order == GW_SUM_TREE && !c->profiling;
+    // the one-lane kernel and the sequential sums do not number their totals,
+    // and a program with blocking waits keeps its cores
+    const bool numbered = c->fru_lanes == 4 && c->sum_order == GW_SUM_TREE && !c->profiling && !c->blocking;
     bool arrived = true;
     CK(numbered ? wait_totals(c, p.seq, &arrived) : cudaStreamSynchronize(c->stream));
     if (!arrived) return set_err(GW_ECUDA, "FRU stage [%g, %g]: the launch ended without its sums", t0, tf);

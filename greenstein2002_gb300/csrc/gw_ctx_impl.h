@@ -18,6 +18,7 @@ struct gw_ctx {
   int pending = 0;          // kFlagSave / kFlagResume to fold into the next launch
   int device = 0;
   int sms = 0;              // its multiprocessors
+  bool blocking = false;    // the program waits with cudaDeviceScheduleBlockingSync
   cudaEvent_t ev[8] = {};
   cudaEvent_t pev[2] = {};  // bracket of the last stage launch while profiling
   bool profiling = false;

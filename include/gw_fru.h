@@ -45,7 +45,10 @@ const char *gw_last_error(void);
 typedef struct gw_ctx gw_ctx;
 
 /* Cell of nfru FRUs on the current CUDA device (replaces the per-rank FRU
- * blocks of initialize_mpi_state, mpi_master.c:199-361). */
+ * blocks of initialize_mpi_state, mpi_master.c:199-361).  Its stage and flux
+ * calls wait by polling the result in host memory, yielding the core between
+ * polls; if the device's scheduling flag is cudaDeviceScheduleBlockingSync
+ * when the cell is created, they block on its stream instead. */
 int gw_create(gw_ctx **ctx, int nfru);
 int gw_destroy(gw_ctx *ctx);
 int gw_nfru(const gw_ctx *ctx);
