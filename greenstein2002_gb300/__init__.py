@@ -205,7 +205,7 @@ class Cell:
         _check(self._L.gw_stage_trace(self._h, 1 if enable else 0), "gw_stage_trace", self._L)
 
     def stage_trace_read(self):
-        """(substeps per FRU, per-warp [begin, end] ns) of the last stage launch."""
+        """(substeps per FRU, [begin, end] ns per 8-FRU group) of the last stage launch."""
         sub = np.zeros(self.nfru, np.uint32)
         ns = np.zeros(((self.nfru + 7) // 8, 2), np.uint64)
         _check(self._L.gw_stage_trace_read(self._h, sub.ctypes.data_as(C.c_void_p), ns.ctypes.data_as(C.c_void_p)),

@@ -73,9 +73,15 @@ static cudaError_t launch_stage_variant(gw_ctx* c, const StageParams& p0) {
   // execute each other's branches: five stages at the peak of release with 8,
   // 4, 2 and 1 per warp, 250 FRUs 0.651 / 0.630 / 0.614 / 0.609 ms, 1,250 FRUs
   // 0.792 / 0.762 / 0.759 / 0.778, 2,500 FRUs 0.791 / 0.765 / 0.807 / 0.960.
-  const bool few = (p.flags & gw::kFlagAdvance) && !c->d.trace_ns;
+  const bool few = (p.flags & gw::kFlagAdvance) != 0;
   const bool wide = few && 4 * groups <= gw::kWideWarpsPerSm * c->sms;
   const int fpw = !few ? 8 : 4 * groups <= 4 * c->sms ? 2 : 2 * groups <= 4 * c->sms ? 4 : 8;
+  if (c->d.trace_ns && c->fru_lanes == 4 && (c->precision == 1 ? fpw < 8 : wide)) {
+    // warps that share a group take the least of their begin times
+    const cudaError_t e =
+        cudaMemsetAsync(c->d.trace_ns, 0xff, sizeof(unsigned long long) * 2 * ((c->d.nfru + 7) / 8), c->stream);
+    if (e != cudaSuccess) return e;
+  }
   if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, fpw, dense, c->stream);
   return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, wide, dense, c->stream)
                            : gw::launch_stage(c->d, p, c->stream);

@@ -1502,7 +1502,11 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
     s.qctl[1 + ((p.launch + 1u) & 1u)] = 0u;
   }
   if (first >= s.nfru) return;  // whole warps past the cell's last FRU
-  if (s.trace_ns && lane == 0) s.trace_ns[2 * grp] = global_ns();
+  // traced group: its first warp's begin and its last warp's end
+  if (s.trace_ns && lane == 0) {
+    if (fpw < 8) atomicMin(&s.trace_ns[2 * grp], global_ns());
+    else s.trace_ns[2 * grp] = global_ns();
+  }
   G g;
   g.c = lane & 3;
   g.q = wide ? (lane >> 2) & 3 : 0;
@@ -1570,7 +1574,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
   // waits for the sequence number only, finds it with this launch's totals
   if (overflow) out[kOutError] = 1.0;
   __syncwarp();
-  if (s.trace_ns && lane == 0) s.trace_ns[2 * grp + 1] = global_ns();
+  if (fpw == 8 && s.trace_ns && lane == 0) s.trace_ns[2 * grp + 1] = global_ns();
   if (s.substeps) {
     unsigned c = __reduce_add_sync(0xffffffffu, (g.c == 0 && g.q == 0) ? nsub : 0u);
     if (lane == 0 && c) atomicAdd(s.substeps, (unsigned long long)c);
@@ -1584,6 +1588,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
       __threadfence();
       last = (atomicAdd(&s.gcount[grp], mine) + mine == size) ? 1u : 0u;
       if (last) s.gcount[grp] = 0u;
+      if (last && s.trace_ns) s.trace_ns[2 * grp + 1] = global_ns();
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();

@@ -66,7 +66,7 @@ struct DevState {
   double* res;
   unsigned long long* substeps;
   // stage trace (null unless enabled): substeps of every FRU in the last
-  // 4-lane launch, and each 8-FRU warp's begin/end global time (ns)
+  // 4-lane launch, and each 8-FRU group's begin/end global time (ns)
   uint32_t* trace_sub;
   unsigned long long* trace_ns;
   // FRU queue of the packed stage kernel: qctl[0] queue head, [1..2] counts

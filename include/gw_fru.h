@@ -142,7 +142,8 @@ int gw_profile(gw_ctx *ctx, int enable);
 int gw_group_timer(int n, gw_ctx **cells, int phase, float *ms);
 /* Stage trace (diagnostics of the 4-lane kernels; no reference
  * counterpart): when enabled, every stage launch records each FRU's substep
- * count and each 8-FRU warp's begin and end global time in ns;
+ * count and each 8-FRU group's begin and end global time in ns (where several
+ * warps share a group, the first one's begin and the last one's end);
  * gw_stage_trace_read returns the last launch's: substeps[nfru],
  * warp_ns[ceil(nfru/8)][2] (either may be NULL).  Enable before the cell
  * joins a batch. */
