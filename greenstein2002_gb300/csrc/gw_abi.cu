@@ -17,6 +17,7 @@
 #include "gw_kernels.h"
 #include "gw_fru_model.cuh"
 #include "gw_ctx_impl.h"
+#include "gw_stage_shape.h"
 #include "gw_wait.h"
 
 using gw::DevState;
@@ -40,8 +41,8 @@ static int set_err(int code, const char* fmt, ...) {
   } while (0)
 
 // Warps (8-FRU groups) of the stages in flight on each device, over all cells
-// and threads: a launch takes the stage kernel's roomy build while they all
-// fit the device with it, else the dense one.  Both give the same results.
+// and threads, by which a launch takes its build of the stage kernel
+// (gw_stage_shape.h).  All give the same results.
 static std::atomic<int> g_stage_warps[64];
 struct StageInFlight {
   std::atomic<int>& n;
@@ -64,26 +65,16 @@ static cudaError_t launch_stage_variant(gw_ctx* c, const StageParams& p0) {
     c->pack_launch++;
     c->launches++;
   }
-  const int groups = g_stage_warps[c->device & 63].load(std::memory_order_relaxed);
-  const bool dense = groups > gw::kRoomyWarpsPerSm * c->sms;
-  // Few FRUs, counted over all cells in flight.  FP64: two per warp on sixteen
-  // lanes each while all those warps are resident (about 3,000 FRUs; figures
-  // at the kernel).  Mixed: fewer of them per warp, as long as that makes at
-  // most four warps per SM (one per sub-partition), because the FRUs of a warp
-  // execute each other's branches: five stages at the peak of release with 8,
-  // 4, 2 and 1 per warp, 250 FRUs 0.651 / 0.630 / 0.614 / 0.609 ms, 1,250 FRUs
-  // 0.792 / 0.762 / 0.759 / 0.778, 2,500 FRUs 0.791 / 0.765 / 0.807 / 0.960.
-  const bool few = (p.flags & gw::kFlagAdvance) != 0;
-  const bool wide = few && 4 * groups <= gw::kWideWarpsPerSm * c->sms;
-  const int fpw = !few ? 8 : 4 * groups <= 4 * c->sms ? 2 : 2 * groups <= 4 * c->sms ? 4 : 8;
-  if (c->d.trace_ns && c->fru_lanes == 4 && (c->precision == 1 ? fpw < 8 : wide)) {
+  const gw::StageShape sh = gw::stage_shape(g_stage_warps[c->device & 63].load(std::memory_order_relaxed), c->sms,
+                                            c->stage_warps, (p.flags & gw::kFlagAdvance) != 0);
+  if (c->d.trace_ns && c->fru_lanes == 4 && (c->precision == 1 ? sh.fpw < 8 : sh.wide)) {
     // warps that share a group take the least of their begin times
     const cudaError_t e =
         cudaMemsetAsync(c->d.trace_ns, 0xff, sizeof(unsigned long long) * 2 * ((c->d.nfru + 7) / 8), c->stream);
     if (e != cudaSuccess) return e;
   }
-  if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, fpw, dense, c->stream);
-  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, wide, dense, c->stream)
+  if (c->precision == 1) return gw::launch_stage_mixed(c->d, p, c->stage_warps, sh.fpw, sh.dense, c->stream);
+  return c->fru_lanes == 4 ? gw::launch_stage4(c->d, p, c->stage_warps, sh.wide, sh.dense, c->stream)
                            : gw::launch_stage(c->d, p, c->stream);
 }
 

@@ -10,10 +10,10 @@
 
 namespace gw {
 
-// Two builds, as in gw_fru_stage4.cu: 182 registers (eleven single-warp blocks
-// per SM) and 128 (sixteen).  Alone, five stages with 128 and 182: 1,251 FRUs
-// 0.532 and 0.505 ms, 12,500 FRUs 1.415 and 1.370 ms; 16 cells of 12,500 FRUs
-// at once for 10 ms: 580 and 891 ms.
+// Two builds, as in gw_fru_stage4.cu: 178 registers (eight warps per SM) and
+// 128 (sixteen).  Alone, five stages with 128 and 178: 1,251 FRUs 0.532 and
+// 0.505 ms, 12,500 FRUs 1.415 and 1.370 ms; 16 cells of 12,500 FRUs at once for
+// 10 ms: 580 and 891 ms.
 __global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage_mixed_kernel(DevState s, StageParams p, int fpw) {
   cleft::stage_body<float>(s, p, blockIdx.x, s.res, fpw);
 }

@@ -7,10 +7,11 @@
 
 namespace gw {
 
-// Two builds of the fixed-layout kernel: with the registers it asks for (180,
-// eleven single-warp blocks per SM) for launches that fit the GPU so, and
-// capped at 128 (sixteen) for more.  Five stages at the peak of release, 128
-// and 180 registers: 12,500 FRUs 6.82 and 6.07 ms, 250 FRUs alike.
+// Two builds of the fixed-layout kernel: with the registers it asks for (178:
+// two warps per sub-partition, eight per SM) for launches of about one wave,
+// and capped at 128 (sixteen per SM) for more (gw_stage_shape.h).  Five stages
+// at the peak of release, dense and roomy: 12,500 FRUs 6.82 and 6.07 ms, 250
+// FRUs alike.
 __global__ void __launch_bounds__(kMaxStageWarps * 32, 1) fru_stage4_kernel(DevState s, StageParams p) {
   cleft::stage_body<double>(s, p, blockIdx.x, s.res);
 }

@@ -108,9 +108,8 @@ cudaError_t launch_stage_mixed_batch(const BatchArgs& a, int nblocks, int warps,
 // cleft-parallel variants: 4 lanes per FRU, 8 FRUs per warp, `warps` warps
 // per block; FP64 (the plain method) and mixed precision (FP32 rates and
 // local ODE); in launches that advance, `wide`: two FRUs per warp on sixteen
-// lanes each, `fpw`: FRUs per warp (8, 4, 2 or 1); `dense`: the build with
-// fewer registers, for more warps than kRoomyWarpsPerSm per SM
-constexpr int kRoomyWarpsPerSm = 11, kWideWarpsPerSm = 10;  // resident single-warp blocks of those builds
+// lanes each, `fpw`: FRUs per warp (8, 4 or 2); `dense`: the build with fewer
+// registers (gw_stage_shape.h chooses)
 cudaError_t launch_stage4(const DevState& s, const StageParams& p, int warps, bool wide, bool dense, cudaStream_t st);
 cudaError_t launch_stage_mixed(const DevState& s, const StageParams& p, int warps, int fpw, bool dense, cudaStream_t st);
 // packed variants: `warps` single-warp blocks whose 4-lane groups take the
