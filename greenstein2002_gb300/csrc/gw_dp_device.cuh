@@ -133,7 +133,7 @@ __device__ __forceinline__ void fcn_warp(DpCell& c, double time, double* y, doub
   __syncwarp();
 }
 
-// stage 2 (node 1/5) from F1 with the step `step` (launch_stage2)
+// stage 2 (node 1/5, rk_pd54m.c:121-127) from F1 with the step `step`
 __device__ __forceinline__ void launch_stage2_warp(DpCell& c, double step, int lane) {
   for (int i = lane; i < GW_NSTATE; i += 32) {
     const double k1 = step * c.F1[i];

@@ -71,8 +71,9 @@ __device__ __forceinline__ double checked_div(double a, double b) {
 }
 
 // x / d for a constant d: rhi = 1/d rounded, rlo = 1/d - rhi rounded; the
-// two-instruction form returns the correctly rounded quotient for every x
-// for the constants below (N. Brisebarre, J.-M. Muller and S. K. Raina,
+// two-instruction form returns the correctly rounded quotient for every finite
+// x whose products do not underflow (|x| > 2^-900, far below any difference of
+// two concentrations, or 0) for the constants below (N. Brisebarre, J.-M. Muller and S. K. Raina,
 // "Accelerating correctly rounded floating-point division when the divisor
 // is known in advance", IEEE Trans. Comput. 53, 2004; the finitely many x
 // whose quotient lies close enough to a midpoint to matter are checked one

@@ -7,10 +7,12 @@
 // lasts as long as the FP64 instruction chain of its slowest FRU.  Spreading an
 // FRU over its clefts divides that chain by about four at the same total work.
 //
-// R = double: the plain FP64 method.  Every operation is the reference's,
-// rounded as the reference rounds it, arranged to issue few FP64
-// instructions (what bounds the kernels, see gw_fp64_math.cuh):
-//   - quotients, reciprocals and exponentials from gw_fp64_math.cuh;
+// R = double: the plain FP64 method.  Every operation is the reference's, in
+// its order, arranged to issue few FP64 instructions (what bounds the
+// kernels).  Sums and products are rounded as the reference rounds them;
+//   - quotients, reciprocals and exponentials are those of gw_fp64_math.cuh:
+//     quotients correctly rounded unless within 2^-37 of a last place of a
+//     midpoint, exponentials to 0.52 of a last place;
 //   - max/min/compares of non-negative doubles on their bit patterns;
 //   - rates are estimated in FP32 and formed in FP64 only where the estimate
 //     leaves a decision open: which rate is the largest (when 0.1 over it is
@@ -247,10 +249,6 @@ __device__ __forceinline__ void regen32(uint32_t* m, int lane) {
   regen_chunk<7>(m, 224, lane);
   regen_chunk<6>(m, 448, lane);
 }
-__device__ __forceinline__ void copy4(uint32_t* dst, const uint32_t* src, const Group& g) {
-  for (int k = g.c; k < kMtN; k += 4) dst[k] = src[k];
-  __syncwarp(g.mask);
-}
 // 624 words in 16-byte pieces by the group's 4 lanes (rows 16-byte aligned)
 __device__ __forceinline__ void copy_row16(uint32_t* dst, const uint32_t* src, const Group& g) {
   const uint4* s4 = reinterpret_cast<const uint4*>(src);
@@ -354,14 +352,15 @@ __device__ __forceinline__ void fetch_old(const StageCtx& sc, const Group& g, in
   }
 }
 
-// cross / copy: bit 4*i set when group i regenerates / first copies its
-// pre-regeneration words to its hold row in this epoch (lane 4*i's ballot).
+// cross / copy: the bit of a group's first lane (regen_step's ballots) is set
+// when the group regenerates its row / first copies its words of before to its
+// hold row in this epoch.
 __device__ __forceinline__ void regen_crossing(const StageCtx& sc, int lane, unsigned cross, unsigned copy) {
   while (cross) {
     const int l0 = __ffs(cross) - 1;
     cross &= cross - 1u;
     uint32_t* row = reinterpret_cast<uint32_t*>(__shfl_sync(0xffffffffu, (unsigned long long)sc.m, l0));
-    const int fg = __shfl_sync(0xffffffffu, sc.f, l0);  // the FRU of group l0/4
+    const int fg = __shfl_sync(0xffffffffu, sc.f, l0);  // the FRU of lane l0's group
     __syncwarp();  // the group has read its old words
     if (copy & (1u << l0)) {
       const uint4* s4 = reinterpret_cast<const uint4*>(row);
@@ -1164,13 +1163,20 @@ __device__ __forceinline__ void fcn_fru4(const WideGroup& g, double cajsr, doubl
 
 // The rates of a substep decide two things: its size dt = min(0.1 / the
 // largest rate, a cap), and, against the draws, which channels change state.
-// Both are settled by FP32 estimates of the rates (relative error below
-// 2^-17: two or three roundings, an exponential of an argument below 10 and
-// truncated inputs) wherever the comparison is clear by kRateTol; the rates
-// that could be the largest, and all of a cleft with a draw too close to its
-// threshold (about one substep in 10^4), are formed in FP64 as the reference
-// does.  Rates in FP64 throughout took about 60 of a substep's 190 FP64
-// instructions.
+// Both are settled by FP32 estimates of the rates wherever the comparison is
+// clear by kRateTol; the rates that could be the largest, and all of a cleft
+// with a draw too close to its threshold (about one substep in 10^4), are formed
+// in FP64 as the reference does.  Rates in FP64 throughout took about 60 of a
+// substep's 190 FP64 instructions.
+// The estimates' relative error is below 2^-15 (truncated inputs, a few
+// roundings, exponentials of arguments below 10; the most in RyR state 7's
+// total, where 1 - p7 cancels) but for the VDI gate: the exponentials of yinf
+// and tau have arguments up to 33, and 1 - yinf, the rate of an open gate,
+// cancels, to nothing at negative potentials.  Its error is small against the
+// thresholds instead: over |V| < 150 mV and the longest substep, with the error
+// bounds documented for the approximate functions, below 0.2 of the 2^32 values
+// of a draw, which the 2 in a threshold's tolerance covers; and at most 1/60 per
+// ms it is never the largest rate of a substep below the cap.
 constexpr float kRateTol = 0x1p-13f;
 
 // First half of one FP64 substep (simfru_local.c:83-146 up to the draws):
@@ -1321,8 +1327,9 @@ __device__ __forceinline__ void substep_b64(Fru4<double>& F, Sub4<double>& S, co
   F.ss.v = fma(k1S + dt * dS, 0.5, cass);
   // ---- transitions of this cleft's 8 channels (:215-276) ----
   // A channel leaves when c = 2^32 - y is below about dt*R*2^32; `open` is set
-  // where c is within the tolerance of a threshold (or of the 2 that
-  // roundings of the exact one can move it).  The RyRs that leave take one
+  // where c is within the tolerance of a threshold: kRateTol of it, and 2 for
+  // the roundings of the exact one (below 1) and the VDI gate's estimate (0.2).
+  // The RyRs that leave take one
   // pass each: the lanes of a warp share the pass.  Each RyR's row depends
   // only on its own state and its cleft's constants, so the order of the
   // passes does not matter.

@@ -41,8 +41,10 @@ cudaError_t launch_stage_mixed_batch(const BatchArgs& a, int nblocks, int warps,
   return cudaGetLastError();
 }
 
-// 16 cells of 12,500 FRUs for 10 ms, 32 FRUs per warp, with at least 12 / 14 /
-// 16 / 18 / 20 single-warp blocks per SM: 528 / 487 / 501 / 562 / 545 ms.
+// 124 registers, sixteen single-warp blocks per SM.  16 cells of 12,500 FRUs
+// for 10 ms, 32 FRUs per warp, with a bound of 12 / 14 / 16 / 18 / 20 blocks (151 /
+// 124 / 124 / 96 / 96 registers): 528 / 487 / 501 / 562 / 545 ms; equal builds
+// differ by 3%, the noise of these figures.
 __global__ void __launch_bounds__(32, 14) fru_stage_mixed_packed_kernel(DevState s, StageParams p) {
   cleft::stage_body_packed<float>(s, p, s.res);
 }

@@ -51,9 +51,11 @@ cudaError_t launch_stage4_batch(const BatchArgs& a, int nblocks, int warps, cuda
   return cudaGetLastError();
 }
 
-// At least thirteen single-warp blocks per SM (<= 152 registers).  16 cells
-// of 12,500 FRUs for 2 ms, 32 FRUs per warp, with 11 / 12 / 13 / 14 / 15 / 16
-// blocks: 617 / 604 / 584 / 592 / 591 / 595 ms.
+// A bound of thirteen blocks or more makes the compiler take 128 registers
+// (sixteen single-warp blocks per SM; 56 bytes spilled at 13, 28 at 14 and 15, 4
+// at 16), of eleven or twelve 168 (twelve blocks).  16 cells of 12,500 FRUs for 2 ms,
+// 32 FRUs per warp, at 11 / 12 / 13 / 14 / 15 / 16: 617 / 604 / 584 / 592 / 591 /
+// 595 ms; the last four differ by spills and noise.
 __global__ void __launch_bounds__(32, 13) fru_stage4_packed_kernel(DevState s, StageParams p) {
   cleft::stage_body_packed<double>(s, p, s.res);
 }

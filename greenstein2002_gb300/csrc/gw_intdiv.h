@@ -3,10 +3,11 @@
  *
  * GB300 issues one FP64 warp instruction per 64 cycles per SM sub-partition,
  * and a hardware-sequence double division takes about six of those slots,
- * while integer instructions issue every cycle.  The FRU stage kernels divide
- * about fifteen times per lane and substep, so moving division off the FP64
- * pipe frees it for the rest of the substep.  The quotient is the IEEE-754
- * round-to-nearest-even one, bit for bit, so results do not change.
+ * while integer instructions issue every cycle.  The quotient is the IEEE-754
+ * round-to-nearest-even one, bit for bit.  In the FRU stage kernels, which
+ * divide about fifteen times per lane and substep, this form ran 22-27% slower
+ * than the FP64 pipe's, and they use the three-instruction quotient of
+ * gw_fp64_math.cuh; kept for the comparison (gw_probe_div).
  *
  * Method (for normal operands whose quotient is normal; anything else --
  * zeros, subnormals, infinities, NaNs, underflow, overflow -- takes the

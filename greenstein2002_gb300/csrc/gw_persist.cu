@@ -176,7 +176,7 @@ __device__ __forceinline__ void finish_op(const Args& a, int ci, const Sums<ND, 
 
 // One 8-FRU group's partial sums, by the whole warp in the lanes of the
 // fixed-layout kernel (FRU grp*8 + lane/4, cleft lane%4), from the FRUs as
-// stored: stage_body_fin's epilogue.
+// stored: the sums at the end of stage_body.
 __device__ __forceinline__ void terms(int c, double jsr, double ss, uint32_t w, FluxSums& v) {
   flux_terms(c, jsr, ss, w, v);
 }
@@ -314,7 +314,7 @@ __device__ __forceinline__ void run_batch(const Args& a, int ci, int grp0, int n
       __syncwarp();
     }
   } else {
-    // no advance: apply a pending save / resume (stage_body_fin without the
+    // no advance: apply a pending save / resume (stage_body without the
     // substeps), in the fixed layout
     for (int grp = grp0; grp < grp0 + ng; grp++) {
       const int ff = grp * 8 + (lane >> 2);

@@ -248,7 +248,7 @@ cudaError_t probe_fp64_issue(double* cycles) {
   return e;
 }
 
-// gw_div_rn (the integer-pipe division of the FRU kernels) against the
+// gw_div_rn (division on the integer pipe, which no kernel uses) against the
 // hardware division on the device: every thread draws operand pairs from a
 // splitmix64 stream -- arbitrary bit patterns, then normal operands of
 // magnitude 1e-8 .. 1e4 (the FRU substep's range) -- and counts quotients

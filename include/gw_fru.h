@@ -261,8 +261,9 @@ int gw_run_device(int n, gw_ctx **cells, const gw_settings *sets, double *t, dou
  * the stage dispatch of distrib_simFRU, mpi_master.c:369-469, for many cells
  * at once): n cells advance n_steps output steps each inside one resident
  * launch, captured with its copy-back as one CUDA graph.  Warps take batches
- * of 8-FRU groups (1 to 4 groups, fewer for small runs; the environment
- * variable GW_PERSIST_GROUPS = 1..8 overrides) from whichever cell has an
+ * of 8-FRU groups (1 to 4 groups by the size of the run, 8 in runs that fill the
+ * GPU many times; the environment variable GW_PERSIST_GROUPS = 1..8
+ * overrides) from whichever cell has an
  * open stage or flux evaluation, advance and sum them, and the warp that
  * finishes a cell's operation runs its integrator step; so no cell waits for
  * another's slowest FRU and no host thread or round trip sits inside a step.
