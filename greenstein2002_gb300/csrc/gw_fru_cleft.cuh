@@ -493,8 +493,11 @@ __device__ __forceinline__ void lane_stage(const StageParams& p, const Group& g,
 
 // FP64: exp(2VF/RT) and the GHK factor a2 of fcn_fru.c:78-101 for voltage V
 // (any V and scale: beyond +-500 mV or a scale near the ends of the exponent
-// range the hardware's division).
-__device__ __forceinline__ void ghk_terms(double V, double pca4, double& e2, double& a2j, bool& small) {
+// range the hardware's division).  The reference's LCC flux is a product with
+// the open flag, NaN for closed channels too where a factor is not finite; the
+// local ODE selects by the flag, so there Cai, which every cleft's flux takes,
+// becomes NaN instead (the product or a test in the ODE cost 1% of a stage).
+__device__ __forceinline__ void ghk_terms(double V, double pca4, double& e2, double& a2j, bool& small, double& cai) {
   constexpr double JDHconstant = 1.0 / (2.0 * VSS * Faraday * 1000.0);
   // 2VF/RT is V over half the divisor and 1000 F VF/RT half of 1000 F times
   // it: exact scalings by two of the reference's products
@@ -505,7 +508,12 @@ __device__ __forceinline__ void ghk_terms(double V, double pca4, double& e2, dou
   a2j = 0.0;
   if (!small) {
     const double num = pca4 * VFsqRT, em1 = e2 - 1.0;
-    a2j = (abs_lt(V, 500.0) && fits(pca4) ? fast_div(num, em1) : num / em1) * JDHconstant;
+    if (abs_lt(V, 500.0) && fits(pca4)) {
+      a2j = fast_div(num, em1) * JDHconstant;
+    } else {
+      a2j = num / em1 * JDHconstant;
+      if (!isfinite(e2) || !isfinite(a2j)) cai = __longlong_as_double(0x7ff8000000000000ll);
+    }
   }
 }
 
@@ -531,7 +539,7 @@ __device__ __forceinline__ void lane_stage(const StageParams& p, const Group& g,
   L.interval = p.tf - p.t0;
   L.rhi = 1.0 / L.interval;
   L.rlo = fma(-L.interval, L.rhi, 1.0) * L.rhi;
-  ghk_terms(L.dep0[0], L.pca4, L.e2, L.a2j, L.small);
+  ghk_terms(L.dep0[0], L.pca4, L.e2, L.a2j, L.small, L.dep0[1]);
   L.isdiv = g.c >= 2;
   L.cA = L.isdiv ? (g.c == 2 ? 12.5f : 30.0f) : -35.0f;
   L.cR = L.isdiv ? (g.c == 2 ? 1.0f / 5.0f : 1.0f / 12.0f) : (g.c == 0 ? 0.012f : -0.05f);
@@ -1321,7 +1329,7 @@ __device__ __forceinline__ void substep_b64(Fru4<double>& F, Sub4<double>& S, co
     F.dep[1] = from(g, mine, 1);
     F.dep[2] = from(g, mine, 2);
   }
-  ghk_terms(F.dep[0], L.pca4, F.e2, F.a2j, F.small);
+  ghk_terms(F.dep[0], L.pca4, F.e2, F.a2j, F.small, F.dep[1]);
   fcn_fru4(g, y1J, y1S, F.dep, F.e2, F.a2j, F.small, F.lopen, F.jcoef, L.pca2, dJ, dS);
   F.jsr.v = fma(k1J + dt * dJ, 0.5, cajsr);
   F.ss.v = fma(k1S + dt * dS, 0.5, cass);
