@@ -402,7 +402,7 @@ static int run_stage(gw_ctx* c, double t0, double tf, const double dep0[3], cons
   p.pca_scale = c->pca_scale;
   p.epoch = c->epoch;
   p.flags = c->pending | (advance ? gw::kFlagAdvance : 0);
-  p.seq = ++c->seq;
+  p.seq = c->seq = gw::next_number(c->seq);
   c->pending = 0;
   if (c->batch) {
     int rc = gw_batch_post(c, p, c->h_out);

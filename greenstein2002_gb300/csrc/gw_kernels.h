@@ -86,7 +86,7 @@ struct StageParams {
   uint32_t epoch;
   int flags;
   uint32_t launch;  // packed launches of the cell so far
-  uint32_t seq;     // number of the launch, for the host that waits for its totals
+  uint32_t seq;     // number of the launch, for the host that waits for its totals (0: none waits)
 };
 
 // Many cells in one launch (cleft-parallel kernels): cell i owns blocks

@@ -6,6 +6,10 @@
 
 namespace gw {
 
+/* The number of the next launch to wait for: never 0, which launches that
+ * nobody waits for carry and leave in the slot. */
+static inline uint32_t next_number(uint32_t n) { return n + 1u ? n + 1u : 1u; }
+
 /* True once *slot holds seq.  busy(), asked now and then, says whether the
  * work that writes it is still under way; false: that work has ended (or
  * failed) and the number is not there. */

@@ -18,5 +18,6 @@ int main() {
   printf("with the end %d\n", r);
   r = gw::wait_number(&slot, 9, [&] { return false; });
   printf("never %d\n", r);
+  printf("next %u %u %u\n", gw::next_number(0), gw::next_number(7), gw::next_number(0xffffffffu));
   return 0;
 }

@@ -12,4 +12,5 @@ def test_wait_ends_with_the_number_or_the_work():
     subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-I" + os.path.join(ROOT, "greenstein2002_gb300", "csrc"),
                            "-o", exe, os.path.join(ROOT, "tests", "native", "wait_check.cpp")])
     out = subprocess.run([exe], capture_output=True, text=True, timeout=60, check=True).stdout
-    assert out.splitlines() == ["there 1 0", "while running 1 3", "with the end 1", "never 0"]
+    assert out.splitlines() == ["there 1 0", "while running 1 3", "with the end 1", "never 0",
+                                "next 1 8 1"]
