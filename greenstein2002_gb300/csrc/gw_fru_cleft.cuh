@@ -1606,6 +1606,7 @@ __device__ __forceinline__ void stage_body(const DevState& s, const StageParams&
       if (last && s.trace_ns) s.trace_ns[2 * grp + 1] = global_ns();
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __syncwarp();  // lane 0's count before every lane's reads (a shuffle orders no memory)
     __threadfence();
     const int ff = grp * 8 + (lane >> 2);
     active = ff < s.nfru;

@@ -169,6 +169,7 @@ __device__ __forceinline__ bool finish_groups(const DevState& s, Sums<ND, NI>& v
     last = (atomicAdd(s.ticket, count) + count == (unsigned)ngroups) ? 1u : 0u;
   }
   if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+  __syncwarp();  // lane 0's count before every lane's reads (a shuffle orders no memory)
   __threadfence();
   v = {};
 #pragma unroll 8
